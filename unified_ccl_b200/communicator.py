@@ -16,6 +16,11 @@ import torch
 
 from . import _C
 
+# The handle of the stream that is current on a device.  torch.cuda.current_stream() builds a Stream object
+# around the same number, which took 3 of the 7 us of a small call; this takes 0.07.  None in a CPU-only
+# torch, where nobody asks.
+current_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
 _DTYPES = {
     torch.float16: 0,
     torch.bfloat16: 1,
@@ -90,6 +95,7 @@ class Communicator:
             unique_id = _derive_unique_id(rank, world_size)
         self._comm = _C.comm_init_rank(world_size, unique_id, rank)
         self._info = _C.comm_info(self._comm)
+        self._device = self._info["cuda_device"]  # -1 on the CPU backend
 
     # ------------------------------------------------------------------ properties
     @property
@@ -106,7 +112,7 @@ class Communicator:
 
     @property
     def on_gpu(self) -> bool:
-        return self._info["cuda_device"] >= 0
+        return self._device >= 0
 
     @property
     def handle(self) -> int:
@@ -122,19 +128,18 @@ class Communicator:
             raise TypeError(f"unsupported dtype {t.dtype}")
         if reducible and t.dtype not in _REDUCIBLE:
             raise TypeError(f"dtype {t.dtype} cannot be reduced; use float16, bfloat16 or float32")
-        if self.on_gpu and not t.is_cuda:
-            raise ValueError("this communicator runs on GPUs: tensors must be CUDA tensors")
-        if not self.on_gpu and t.is_cuda:
-            raise ValueError("this communicator runs on the CPU backend: tensors must be CPU tensors")
-        if t.is_cuda and t.device.index != self._info["cuda_device"]:
-            raise ValueError(f"tensor is on cuda:{t.device.index}, communicator on cuda:{self._info['cuda_device']}")
+        index = t.get_device()  # -1 for a CPU tensor
+        if index != self._device:
+            if index < 0:
+                raise ValueError("this communicator runs on GPUs: tensors must be CUDA tensors")
+            if self._device < 0:
+                raise ValueError("this communicator runs on the CPU backend: tensors must be CPU tensors")
+            raise ValueError(f"tensor is on cuda:{index}, communicator on cuda:{self._device}")
         if not t.is_contiguous():
             raise ValueError("tensor must be contiguous")
 
     def _stream(self) -> int:
-        if not self.on_gpu:
-            return 0
-        return torch.cuda.current_stream(self._info["cuda_device"]).cuda_stream
+        return current_raw_stream(self._device) if self._device >= 0 else 0
 
     # ------------------------------------------------------------------ collectives
     def allreduce(self, tensor: torch.Tensor, op: str = "sum", out: torch.Tensor = None) -> torch.Tensor:

@@ -2,6 +2,7 @@
 import torch
 
 from .. import _C
+from ..communicator import current_raw_stream
 
 
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, swiglu: bool = False) -> torch.Tensor:
@@ -25,7 +26,15 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, swiglu
         out = torch.empty(M, n_out, device=a.device, dtype=torch.bfloat16)
     elif out.shape != (M, n_out) or out.dtype != torch.bfloat16 or out.stride(1) != 1:
         raise ValueError("bad out tensor")
-    with torch.cuda.device(a.device):
-        _C.gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-                     1 if swiglu else 0, torch.cuda.current_stream().cuda_stream)
+    device = a.get_device()
+    if device == torch._C._cuda_getDevice():
+        _launch(a, b, out, M, N, K, swiglu, device)
+    else:
+        with torch.cuda.device(device):
+            _launch(a, b, out, M, N, K, swiglu, device)
     return out
+
+
+def _launch(a, b, out, M, N, K, swiglu, device):
+    _C.gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+                 1 if swiglu else 0, current_raw_stream(device))
