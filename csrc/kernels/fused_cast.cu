@@ -15,10 +15,10 @@
 // Work is cut in units of 128 elements so that an fp8 scale block never straddles two CTAs, and
 // the 128 elements of a block sit in consecutive lanes of one warp (16 lanes for 16-bit input,
 // 32 for fp32 input), which makes the block's amax a shuffle reduction.
-#include <cuda_fp8.h>
-
 #include "coll_device.cuh"
 #include "collectives.cuh"
+#include "fp8_cast.cuh"
+#include "gemm_sm100.h"
 
 namespace uccl {
 namespace dev {
@@ -43,17 +43,13 @@ __device__ __forceinline__ void store_cast(char* out, size_t elem, const float (
   }
 }
 
-// quantise with the block's scale (a true division, as in the MoE dispatch, so that the result is
-// bit-identical to an fp32 restatement of the cast)
+// quantise with the block's scale: bit-identical to an fp32 restatement of the cast, as in the MoE dispatch
 template <int NE>
 __device__ __forceinline__ void store_fp8(char* out, size_t elem, const float (&v)[8], float blockScale) {
+  const float inv = __frcp_rn(blockScale);
   uint32_t w[2] = {0, 0};
 #pragma unroll
-  for (int j = 0; j < NE / 4; ++j) {
-    const __nv_fp8x2_storage_t a0 = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(v[4 * j], blockScale), __fdiv_rn(v[4 * j + 1], blockScale)), __NV_SATFINITE, __NV_E4M3);
-    const __nv_fp8x2_storage_t a1 = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(v[4 * j + 2], blockScale), __fdiv_rn(v[4 * j + 3], blockScale)), __NV_SATFINITE, __NV_E4M3);
-    w[j] = static_cast<uint32_t>(a0) | (static_cast<uint32_t>(a1) << 16);
-  }
+  for (int j = 0; j < NE / 4; ++j) w[j] = fp8::quantise4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3], blockScale, inv);
   char* p = out + elem;
   if (NE == 8) *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
   else *reinterpret_cast<uint32_t*>(p) = w[0];
@@ -81,7 +77,7 @@ __global__ void __launch_bounds__(kThreads, 1) reduce_cast_kernel(const __grid_c
                    min(len, userBytes - begin));
     }
   }
-  if (n > 1 && !rank_barrier(dc)) return;  // a single rank has no arena to meet in
+  if (!rank_barrier(dc)) return;
   const size_t mine = static_cast<size_t>(dc.rank) * a.chunkStride;
   // whole warps run every iteration: lanes beyond the slice's last vector still take part in the shuffles
   const size_t vEnd = v1 > v0 ? v0 + ((v1 - v0 + 31) / 32) * 32 : v0;
@@ -114,7 +110,7 @@ __global__ void __launch_bounds__(kThreads, 1) reduce_cast_kernel(const __grid_c
       for (int e = 0; e < NE; ++e) amax = fmaxf(amax, fabsf(acc[e]));
 #pragma unroll
       for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      const float blockScale = fmaxf(amax, 1e-10f) / 448.f;
+      const float blockScale = fp8::block_scale(amax);
       if (live) {
         store_fp8<NE>(a.out, elem, acc, blockScale);
         if ((v % LANES) == 0) a.outScales[v / LANES] = blockScale;
@@ -123,10 +119,133 @@ __global__ void __launch_bounds__(kThreads, 1) reduce_cast_kernel(const __grid_c
       store_cast<OUT, NE>(a.out, elem, acc);
     }
   }
-  if (n > 1) rank_barrier(dc);
+  rank_barrier(dc);
+}
+
+// One rank: nothing to add and nobody to meet, so the work is a stream from memory to memory.  Every
+// thread takes U pieces of 32 input bytes (16 elements of a 16-bit type, 8 of fp32) that lie one CTA
+// width apart, with all their loads in flight before the first use: four pieces at four 256-thread
+// CTAs per SM are 128 KiB in flight, where the shared kernel above, with one 16-byte load per thread
+// on at most kMaxBlocks CTAs, reached a fifth of the memory bandwidth.  A 128-element scale block is
+// 8 (or 16) consecutive lanes.
+struct CastLocalArgs {
+  const char* in;
+  char* out;
+  float* outScales;
+  size_t elems;  // a multiple of 16 input bytes, and of 128 for fp8 output
+  float scale;
+  int wide;      // both buffers are 32-byte aligned
+};
+
+constexpr int kCastThreads = 256;
+
+template <int DT, int OUT, int U>
+__global__ void __launch_bounds__(kCastThreads, 4) cast_local_kernel(const __grid_constant__ CastLocalArgs a) {
+  using V = Vec<DT>;
+  constexpr int E = 32 / V::ES;     // elements per piece
+  constexpr int LANES = 128 / E;    // lanes that share one scale block
+  const size_t pieces = (a.elems + E - 1) / E;
+  const size_t c0 = static_cast<size_t>(blockIdx.x) * (kCastThreads * U) + threadIdx.x;
+  uint32_t raw[U][8];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const size_t c = c0 + u * kCastThreads;
+    const char* p = a.in + c * 32;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) raw[u][j] = 0;
+    if (c < pieces) {
+      if (a.wide && (c + 1) * E <= a.elems) {
+        ptx::ld_stream_v8(p, raw[u]);
+      } else {
+        const uint4 lo = ptx::ld_stream_v4(p);
+        raw[u][0] = lo.x, raw[u][1] = lo.y, raw[u][2] = lo.z, raw[u][3] = lo.w;
+        if ((c + 1) * E <= a.elems) {  // the last piece may be half a one
+          const uint4 hi = ptx::ld_stream_v4(p + 16);
+          raw[u][4] = hi.x, raw[u][5] = hi.y, raw[u][6] = hi.z, raw[u][7] = hi.w;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const size_t c = c0 + u * kCastThreads;
+    const bool live = c < pieces, whole = (c + 1) * E <= a.elems;
+    float v[E];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      V::add(acc, make_uint4(raw[u][4 * h], raw[u][4 * h + 1], raw[u][4 * h + 2], raw[u][4 * h + 3]));
+#pragma unroll
+      for (int e = 0; e < E / 2; ++e) v[h * (E / 2) + e] = acc[e] * a.scale;
+    }
+    char* out = a.out + c * E * (OUT == OUT_FP8 ? 1 : OUT == OUT_F32 ? 4 : 2);
+    if (OUT == OUT_FP8) {
+      float amax = 0.f;
+#pragma unroll
+      for (int e = 0; e < E; ++e) amax = fmaxf(amax, fabsf(v[e]));
+#pragma unroll
+      for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+      const float blockScale = fp8::block_scale(amax), inv = __frcp_rn(blockScale);
+      uint32_t w[E / 4];
+#pragma unroll
+      for (int j = 0; j < E / 4; ++j) w[j] = fp8::quantise4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3], blockScale, inv);
+      if (live) {
+        if constexpr (E == 16) ptx::st_global_v4(out, make_uint4(w[0], w[1], w[2], w[3]));
+        else *reinterpret_cast<uint2*>(out) = make_uint2(w[0], w[1]);
+        if (c % LANES == 0) a.outScales[c / LANES] = blockScale;
+      }
+    } else {
+      constexpr int W = OUT == OUT_F32 ? E : E / 2;  // output words of a piece: 16, 8 or 4
+      uint32_t w[W];
+#pragma unroll
+      for (int j = 0; j < W; ++j)
+        w[j] = OUT == OUT_F32 ? __float_as_uint(v[j]) : OUT == OUT_BF16 ? ptx::pack_bf16x2(v[2 * j], v[2 * j + 1]) : ptx::pack_f16x2(v[2 * j], v[2 * j + 1]);
+      if (W == 4) {  // fp32 -> 16 bits: a piece is 16 output bytes, and a half piece is 8
+        if (live && whole) ptx::st_global_v4(out, make_uint4(w[0], w[1], w[2], w[3]));
+        else if (live) *reinterpret_cast<uint2*>(out) = make_uint2(w[0], w[1]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < W; j += 8) {
+          if (!live || (j * 2 >= W && !whole)) continue;
+          const uint32_t(&o)[8] = *reinterpret_cast<const uint32_t(*)[8]>(&w[j]);
+          if (a.wide && (W == 16 || whole)) {
+            ptx::st_global_v8(out + j * 4, o);
+          } else {
+            ptx::st_global_v4(out + j * 4, make_uint4(o[0], o[1], o[2], o[3]));
+            if (W == 16 || whole) ptx::st_global_v4(out + j * 4 + 16, make_uint4(o[4], o[5], o[6], o[7]));
+          }
+        }
+      }
+    }
+  }
 }
 
 }  // namespace dev
+
+template <int DT, int OUT>
+static cudaError_t launchLocal(const dev::CastLocalArgs& a, cudaStream_t s) {
+  const size_t pieces = (a.elems + 32 / dev::Vec<DT>::ES - 1) / (32 / dev::Vec<DT>::ES);
+  // four pieces per thread once that still gives every SM its four CTAs; below that one piece per
+  // thread spreads the work over more SMs
+  constexpr int T = dev::kCastThreads;
+  if (pieces >= static_cast<size_t>(deviceSmCount()) * 4 * T * 4) {
+    dev::cast_local_kernel<DT, OUT, 4><<<static_cast<unsigned>((pieces + 4 * T - 1) / (4 * T)), T, 0, s>>>(a);
+  } else {
+    dev::cast_local_kernel<DT, OUT, 1><<<static_cast<unsigned>((pieces + T - 1) / T), T, 0, s>>>(a);
+  }
+  return cudaGetLastError();
+}
+
+template <int DT>
+static cudaError_t launchLocalOut(const dev::CastLocalArgs& a, int outType, cudaStream_t s) {
+  switch (outType) {
+    case ucclFloat16: return launchLocal<DT, dev::OUT_F16>(a, s);
+    case ucclBfloat16: return launchLocal<DT, dev::OUT_BF16>(a, s);
+    case ucclFloat32: return launchLocal<DT, dev::OUT_F32>(a, s);
+    case ucclFloat8e4m3: return launchLocal<DT, dev::OUT_FP8>(a, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
 
 template <int DT, bool NVLS>
 static cudaError_t launchOut(const CastArgs& a, int blocks, cudaStream_t s) {
@@ -142,6 +261,21 @@ static cudaError_t launchOut(const CastArgs& a, int blocks, cudaStream_t s) {
 
 cudaError_t launchReduceCastKernel(const CastArgs& a, int blocks, cudaStream_t s) {
   if (blocks < 1 || blocks > kMaxBlocks) return cudaErrorInvalidValue;
+  if (a.dc.nranks == 1) {
+    dev::CastLocalArgs l;
+    l.in = a.in[0];
+    l.out = a.out;
+    l.outScales = a.outScales;
+    l.elems = a.chunkElems;
+    l.scale = a.scale;
+    l.wide = ((reinterpret_cast<uintptr_t>(l.in) | reinterpret_cast<uintptr_t>(l.out)) & 31) == 0;
+    switch (a.inType) {
+      case ucclFloat16: return launchLocalOut<dev::DT_F16>(l, a.outType, s);
+      case ucclBfloat16: return launchLocalOut<dev::DT_BF16>(l, a.outType, s);
+      case ucclFloat32: return launchLocalOut<dev::DT_F32>(l, a.outType, s);
+      default: return cudaErrorInvalidValue;
+    }
+  }
   const bool nvls = a.inMc != nullptr;
   switch (a.inType) {
     case ucclFloat16: return nvls ? launchOut<dev::DT_F16, true>(a, blocks, s) : launchOut<dev::DT_F16, false>(a, blocks, s);

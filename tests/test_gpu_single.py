@@ -33,6 +33,41 @@ def test_moe_single_rank():
 
 
 @gpu
+@pytest.mark.parametrize("din", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("dout", [torch.bfloat16, torch.float16, torch.float32, torch.float8_e4m3fn])
+def test_cast_single_rank(din, dout):
+    """One rank: scaled and rounded once, so every bit is known.  Pieces of 32 input bytes (the last one halved), one and
+    four pieces per thread, buffers on 32-byte and only on 16-byte boundaries; powers of two put many quotients on ties."""
+    import os
+
+    from unified_ccl_b200 import Communicator
+
+    os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    comm = Communicator(0, 1)
+    fp8 = dout == torch.float8_e4m3fn
+    step = 16 // torch.empty((), dtype=din).element_size()
+    for count in (128, 128 * 77, 1 << 24) if fp8 else (step, 3 * step, 257 * 16, 1027 * step, 1 << 24):
+        for off in (0, step):  # elements in front: the input starts on a 16-byte boundary only
+            g = torch.Generator(device="cuda").manual_seed(count + off)
+            x = torch.randn(count + off, device="cuda", generator=g)
+            x[: count // 2] = torch.exp2((x[: count // 2] * 3).round()) * x[: count // 2].sign()
+            x = x.to(din)[off:]
+            out = torch.empty(count, device="cuda", dtype=dout)
+            out, scales = comm.reduce_scatter_cast(x, out, 0.37)
+            ref = (x.float() + 0.0) * torch.tensor(0.37, device="cuda")
+            if fp8:
+                # division by a tensor: torch turns one by a number into a product on the GPU
+                blocks = ref.view(-1, 128)
+                sc = blocks.abs().amax(-1, keepdim=True).clamp_min(1e-10)
+                sc = sc / torch.full_like(sc, 448.0)
+                assert torch.equal(scales, sc.view(-1)), (count, off)
+                assert torch.equal(out.view(torch.uint8), (blocks / sc).to(dout).view(torch.uint8).view(-1)), (count, off)
+            else:
+                assert torch.equal(out, ref.to(dout)), (count, off)
+    comm.destroy()
+
+
+@gpu
 def test_canaries_around_symmetric_buffers():
     assert_all_ok(run_ranks("canary", 1, env={"UCCL_CANARY": "1"}))
 
