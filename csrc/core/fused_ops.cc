@@ -147,8 +147,7 @@ extern "C" ucclResult_t ucclAllReduceResidualRMSNorm(const void* x, const void* 
     a.dc.nranks = 1;
     a.inUser = static_cast<const char*>(x);
     a.resOutUser = static_cast<char*>(residualOut);
-    const int blocks = std::min(deviceSmCount(), std::max(1, tokens));
-    if (launchArNormKernel(a, blocks, s) != cudaSuccess) {
+    if (launchArNormKernel(a, 1, s) != cudaSuccess) {
       commSetError(c, "norm kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
       return ucclSystemError;
     }

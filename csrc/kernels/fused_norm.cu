@@ -14,8 +14,11 @@
 // Only one tensor travels the all-gather direction; the normalised output never crosses NVLink.
 // CTA b handles rows b, b+B, ... of every shard in both phases, so the CTA-level rank barrier
 // covers exactly the rows it later reads.
+#include <algorithm>
+
 #include "coll_device.cuh"
 #include "collectives.cuh"
+#include "gemm_sm100.h"
 
 #ifdef UCCL_EXPERIMENTS
 #define UCCL_NORM_DBG(a, bit) (((a).debug & (bit)) != 0)  // leave a phase out to time the rest (benchmarks/fused_layers.py)
@@ -254,67 +257,154 @@ __global__ void __launch_bounds__(kThreads, 1) ar_norm_kernel(const __grid_const
   }
 }
 
-// single-rank / reference path: out = rmsnorm(x + residual) * gamma without any communication
-__global__ void __launch_bounds__(kThreads, 1) add_norm_kernel(const __grid_constant__ ArNormArgs a) {
-  const int vecPerRow = a.hidden >> 3;
-  const size_t rowBytes = static_cast<size_t>(a.hidden) * 2;
-  const int perRow = (vecPerRow + kThreads - 1) / kThreads;
-  NormPass np;
-  np.nvecThread = perRow;
-  np.R = min(kNormMaxRows, kNormSlots / perRow);
-  const size_t tokens = static_cast<size_t>(a.tokens);
-  const int B = gridDim.x;
-  for (size_t r0 = blockIdx.x; r0 < tokens; r0 += static_cast<size_t>(B) * np.R) {
-    size_t rowIdx[kNormMaxRows];
-    int rowsHere = 0;
+// ------------------------------------------------------------------ one rank
+// out = rmsnorm(x + residual) * gamma without any communication: 2 reads and 2 writes per element.
+struct NormLocalArgs {
+  const char* x;
+  const char* residual;
+  const char* gamma;
+  char* out;
+  char* resOut;  // may be `residual`
+  int tokens, hidden;
+  float eps;
+};
+
+// h = bf16(x + residual), and the sum of its squares is added to `ss`
+__device__ __forceinline__ uint4 add_square(uint4 x, uint4 res, float& ss) {
+  const uint4 h = add_bf16x8(x, res);
+  const uint32_t w[4] = {h.x, h.y, h.z, h.w};
 #pragma unroll
-    for (int j = 0; j < kNormMaxRows; ++j) {
-      const size_t r = r0 + static_cast<size_t>(j) * B;
-      rowIdx[j] = r < tokens ? r : r0;
-      if (j < np.R && r < tokens) rowsHere = j + 1;
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = ptx::unpack_bf16x2(w[e]);
+    ss += f.x * f.x + f.y * f.y;
+  }
+  return h;
+}
+__device__ __forceinline__ uint4 scale_gamma(uint4 h, uint4 g, float rstd) {
+  const uint32_t w[4] = {h.x, h.y, h.z, h.w}, gw[4] = {g.x, g.y, g.z, g.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = ptx::unpack_bf16x2(w[e]), gg = ptx::unpack_bf16x2(gw[e]);
+    o[e] = ptx::pack_bf16x2(f.x * rstd * gg.x, f.y * rstd * gg.y);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// W bytes (16 or 32) of a row per piece, NV pieces per thread, `lanes` threads per row and blockDim / lanes
+// rows per CTA.  Bound by memory: all loads of a thread are out before the first use, and nothing is
+// persistent, so that on every SM some CTAs load while others reduce and store.  8192 x 8192: 82 us =
+// 6.5 TB/s, what a copy reaches; one persistent CTA per SM took 109 us (loads into registers, four rows
+// per pass) and 100 us (a ring of bulk loads, 190 KiB of them in flight: groups of warps then wait for
+// each other's reductions).
+template <int NV, int W>
+__global__ void __launch_bounds__(NV * W > 32 ? 512 : 1024) add_norm_kernel(const __grid_constant__ NormLocalArgs a, int lanes) {
+  __shared__ float part[32];
+  constexpr int Q = W / 16;
+  const int t = threadIdx.x % lanes, sub = threadIdx.x / lanes;
+  const long row = static_cast<long>(blockIdx.x) * (blockDim.x / lanes) + sub;
+  const bool live = row < a.tokens;
+  const int pieces = live ? (a.hidden * 2) / W : 0;
+  const size_t base = static_cast<size_t>(row) * a.hidden * 2;
+  uint4 x[NV][Q], r[NV][Q];
+  auto load = [](const char* p, uint4 (&v)[Q]) {
+    if constexpr (Q == 2) {
+      uint32_t w[8];
+      ptx::ld_stream_v8(p, w);
+      v[0] = make_uint4(w[0], w[1], w[2], w[3]);
+      v[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    } else {
+      v[0] = ptx::ld_stream_v4(p);
     }
-    uint4 h[kNormSlots], res[kNormSlots];
-#pragma unroll
-    for (int s = 0; s < kNormSlots; ++s) {
-      int j, v;
-      if (np.slot(s, rowsHere, &j, &v) && v < vecPerRow) {
-        size_t row = rowIdx[0];
-#pragma unroll
-        for (int jj = 1; jj < kNormMaxRows; ++jj)
-          if (jj == j) row = rowIdx[jj];
-        const size_t off = row * rowBytes + (static_cast<size_t>(v) << 4);
-        h[s] = ptx::ld_global_v4(a.inUser + off);
-        res[s] = ptx::ld_global_v4(reinterpret_cast<const char*>(a.residual) + off);
-      } else {
-        h[s] = make_uint4(0, 0, 0, 0);
-        res[s] = make_uint4(0, 0, 0, 0);
-      }
+  };
+  auto store = [](char* p, const uint4 (&v)[Q]) {
+    if constexpr (Q == 2) {
+      const uint32_t w[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
+      ptx::st_global_v8(p, w);
+    } else {
+      ptx::st_global_v4(p, v[0]);
     }
+  };
 #pragma unroll
-    for (int s = 0; s < kNormSlots; ++s) {
-      int j, v;
-      if (np.slot(s, rowsHere, &j, &v) && v < vecPerRow) {
-        size_t row = rowIdx[0];
+  for (int j = 0; j < NV; ++j) {
+    const int v = t + j * lanes;
 #pragma unroll
-        for (int jj = 1; jj < kNormMaxRows; ++jj)
-          if (jj == j) row = rowIdx[jj];
-        h[s] = add_bf16x8(h[s], res[s]);
-        ptx::st_global_v4(a.resOutUser + row * rowBytes + (static_cast<size_t>(v) << 4), h[s]);
-      }
+    for (int q = 0; q < Q; ++q) x[j][q] = r[j][q] = make_uint4(0, 0, 0, 0);
+    if (v < pieces) {
+      load(a.x + base + static_cast<size_t>(v) * W, x[j]);
+      load(a.residual + base + static_cast<size_t>(v) * W, r[j]);
     }
-    normalise_rows(np, h, rowsHere, rowIdx, a.gamma, a.outLocal, rowBytes, a.eps, a.hidden);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int v = t + j * lanes;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) x[j][q] = add_square(x[j][q], r[j][q], ss);
+    if (v < pieces) store(a.resOut + base + static_cast<size_t>(v) * W, x[j]);
+  }
+  ss = warp_sum(ss);
+  if (lanes > 32) {
+    const int warps = lanes >> 5, l = threadIdx.x & 31;
+    if (l == 0) part[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    ss = warp_sum(l < warps ? part[sub * warps + l] : 0.f);
+  }
+  const float rstd = rsqrtf(ss / static_cast<float>(a.hidden) + a.eps);
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int v = t + j * lanes;
+    if (v < pieces) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        x[j][q] = scale_gamma(x[j][q], ptx::ld_global_v4(a.gamma + static_cast<size_t>(v) * W + q * 16), rstd);
+      store(a.out + base + static_cast<size_t>(v) * W, x[j]);
+    }
   }
 }
 
 }  // namespace dev
 
+template <int W>
+static cudaError_t launchNormLocal(const dev::NormLocalArgs& l, cudaStream_t s) {
+  const int pieces = l.hidden * 2 / W;
+  // two CTAs of rows per SM or fewer (decode): a thread per piece, for the shortest chain.  More rows: up to
+  // 64 bytes of either input per thread, so that a barrier and its shuffles pay for more data.
+  const int most = l.tokens <= 2 * deviceSmCount() ? (pieces + 1023) / 1024 : (pieces > 32 ? 64 / W : 1);
+  const int nv = most <= 1 ? 1 : most <= 2 ? 2 : 4;
+  const int lanes = ((pieces + nv - 1) / nv + 31) / 32 * 32;
+  const int rows = lanes >= 256 ? 1 : 256 / lanes;
+  const unsigned grid = static_cast<unsigned>((static_cast<long>(l.tokens) + rows - 1) / rows);
+  if (nv == 1) dev::add_norm_kernel<1, W><<<grid, lanes * rows, 0, s>>>(l, lanes);
+  else if (nv == 2) dev::add_norm_kernel<2, W><<<grid, lanes * rows, 0, s>>>(l, lanes);
+  else dev::add_norm_kernel<4, W><<<grid, lanes * rows, 0, s>>>(l, lanes);
+  return cudaGetLastError();
+}
+
 cudaError_t launchArNormKernel(const ArNormArgs& a, int blocks, cudaStream_t stream) {
-  // the multi-rank kernel has one cross-rank barrier slot per CTA
-  if (a.hidden % 8 != 0 || a.hidden > dev::kNormMaxVec * dev::kThreads * 8 || blocks < 1 ||
-      blocks > (a.dc.nranks <= 1 ? 1024 : kMaxBlocks))
-    return cudaErrorInvalidValue;
-  if (a.dc.nranks <= 1) dev::add_norm_kernel<<<blocks, dev::kThreads, 0, stream>>>(a);
-  else dev::ar_norm_kernel<<<blocks, dev::kThreads, 0, stream>>>(a);
+  if (a.hidden % 8 != 0 || a.hidden > dev::kNormMaxVec * dev::kThreads * 8) return cudaErrorInvalidValue;
+  if (a.dc.nranks <= 1) {
+    dev::NormLocalArgs l;
+    l.x = a.inUser;
+    l.residual = reinterpret_cast<const char*>(a.residual);
+    l.gamma = reinterpret_cast<const char*>(a.gamma);
+    l.out = a.outLocal;
+    l.resOut = a.resOutUser;
+    l.tokens = a.tokens;
+    l.hidden = a.hidden;
+    l.eps = a.eps;
+    const uintptr_t all = reinterpret_cast<uintptr_t>(l.x) | reinterpret_cast<uintptr_t>(l.residual) |
+                          reinterpret_cast<uintptr_t>(l.out) | reinterpret_cast<uintptr_t>(l.resOut) | (a.hidden * 2);
+    return (all & 31) == 0 ? launchNormLocal<32>(l, stream) : launchNormLocal<16>(l, stream);
+  }
+  // one cross-rank barrier slot per CTA
+  if (blocks < 1 || blocks > kMaxBlocks) return cudaErrorInvalidValue;
+  dev::ar_norm_kernel<<<blocks, dev::kThreads, 0, stream>>>(a);
   return cudaGetLastError();
 }
 

@@ -68,6 +68,29 @@ def test_cast_single_rank(din, dout):
 
 
 @gpu
+@pytest.mark.parametrize("tokens,hidden", [(1, 8), (700, 24), (297, 512), (700, 1032), (300, 8192), (5, 8200), (300, 16376), (300, 16384)])
+def test_norm_single_rank_shapes(tokens, hidden):
+    """Pieces of 16 and 32 bytes, one to four per thread, several rows per CTA and one; residual in place."""
+    import os
+
+    from unified_ccl_b200 import Communicator
+    from unified_ccl_b200.parallel import allreduce_residual_rmsnorm
+
+    os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    comm = Communicator(0, 1)
+    g = torch.Generator(device="cuda").manual_seed(tokens + hidden)
+    x, res = (torch.randn(tokens, hidden, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    gamma = (1 + 0.02 * torch.randn(hidden, device="cuda", generator=g)).to(torch.bfloat16)
+    h = (x.float() + res.float()).to(torch.bfloat16)
+    ref = h.float() * torch.rsqrt(h.float().square().mean(-1, keepdim=True) + 1e-6) * gamma.float()
+    out, res_out = allreduce_residual_rmsnorm(comm, x, res, gamma, 1e-6)
+    assert res_out is res and torch.equal(res, h)
+    # one rounding to bf16 of a value whose fp32 error is far below it
+    assert ((out.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-6).all()
+    comm.destroy()
+
+
+@gpu
 def test_canaries_around_symmetric_buffers():
     assert_all_ok(run_ranks("canary", 1, env={"UCCL_CANARY": "1"}))
 
