@@ -15,20 +15,48 @@ __device__ __forceinline__ uint32_t pack4(float a, float b, float c, float d) {
   return static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
 }
 
-// Four elements -> four e4m3 bytes, bit for bit those of the true quotient x / scale, without a
-// division per element.  With inv = 1 / scale rounded, r = x * inv lies within 2^-22.9 (two
-// roundings) of the exact quotient, whose own rounding adds 2^-24: the rounded quotient is inside
-// [r (1 - 2^-21), r (1 + 2^-21)].  Rounding to e4m3 is monotonic, so where both ends give the same
-// byte it is the quotient's byte as well.  The ends differ only next to a point halfway between two
-// e4m3 values (about one element in 2^18 of ordinary data); those four elements take the division.
-__device__ __forceinline__ uint32_t quantise4(float x0, float x1, float x2, float x3, float scale, float inv) {
-  constexpr float kUp = 1.0f + 0x1p-21f, kDown = 1.0f - 0x1p-21f;
-  const float r0 = x0 * inv, r1 = x1 * inv, r2 = x2 * inv, r3 = x3 * inv;
-  const uint32_t up = pack4(r0 * kUp, r1 * kUp, r2 * kUp, r3 * kUp);
-  const uint32_t down = pack4(r0 * kDown, r1 * kDown, r2 * kDown, r3 * kDown);
-  if (up == down) return up;
-  return pack4(__fdiv_rn(x0, scale), __fdiv_rn(x1, scale), __fdiv_rn(x2, scale), __fdiv_rn(x3, scale));
+// Two elements per instruction.
+__device__ __forceinline__ float2 mul2(float2 x, float2 y) {
+  float2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<const unsigned long long&>(x)), "l"(reinterpret_cast<const unsigned long long&>(y)));
+  return r;
 }
+__device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {
+  float2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<const unsigned long long&>(x)), "l"(reinterpret_cast<const unsigned long long&>(y)),
+        "l"(reinterpret_cast<const unsigned long long&>(z)));
+  return r;
+}
+
+// Correctly rounded quotients by one divisor, for the many elements that share a scale.  Markstein's
+// theorem ("Computation of elementary functions on the IBM RISC System/6000 processor", 1990): with y =
+// RN(1 / b) and q within one unit in the last place of a / b, RN(q + RN(a - b q) y) is RN(a / b).
+// RN(a y) may be one and a half units off, so a first step makes q faithful and a second one exact.
+// It takes and carries -a and -y, which keeps the sign of a zero.  No residual that decides a byte
+// can underflow (b >= 1e-10 / 448, and quotients below 2^-10 are zero in e4m3).  An infinite b (an
+// infinity in the block) becomes 0 with y = 0: finite elements give zero, infinite ones NaN, as a / b does.
+struct Divisor {
+  float2 b, ny;
+  __device__ __forceinline__ explicit Divisor(float scale) {
+    const float d = isinf(scale) ? 0.f : scale, n = -__frcp_rn(scale);
+    b = make_float2(d, d);
+    ny = make_float2(n, n);
+  }
+  __device__ __forceinline__ float2 quotient_of_negated(float2 na) const {
+    float2 q = mul2(na, ny);
+    q = fma2(fma2(q, b, na), ny, q);
+    return fma2(fma2(q, b, na), ny, q);
+  }
+  // e4m3 bytes of four quotients, the elements given with their signs changed
+  __device__ __forceinline__ uint32_t quantise4(float2 na, float2 nb) const {
+    const float2 p = quotient_of_negated(na), q = quotient_of_negated(nb);
+    return pack4(p.x, p.y, q.x, q.y);
+  }
+};
 
 }  // namespace fp8
 }  // namespace uccl

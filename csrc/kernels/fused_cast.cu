@@ -15,6 +15,8 @@
 // Work is cut in units of 128 elements so that an fp8 scale block never straddles two CTAs, and
 // the 128 elements of a block sit in consecutive lanes of one warp (16 lanes for 16-bit input,
 // 32 for fp32 input), which makes the block's amax a shuffle reduction.
+#include <type_traits>
+
 #include "coll_device.cuh"
 #include "collectives.cuh"
 #include "fp8_cast.cuh"
@@ -46,10 +48,11 @@ __device__ __forceinline__ void store_cast(char* out, size_t elem, const float (
 // quantise with the block's scale: bit-identical to an fp32 restatement of the cast, as in the MoE dispatch
 template <int NE>
 __device__ __forceinline__ void store_fp8(char* out, size_t elem, const float (&v)[8], float blockScale) {
-  const float inv = __frcp_rn(blockScale);
+  const fp8::Divisor div(blockScale);
   uint32_t w[2] = {0, 0};
 #pragma unroll
-  for (int j = 0; j < NE / 4; ++j) w[j] = fp8::quantise4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3], blockScale, inv);
+  for (int j = 0; j < NE / 4; ++j)
+    w[j] = div.quantise4(make_float2(-v[4 * j], -v[4 * j + 1]), make_float2(-v[4 * j + 2], -v[4 * j + 3]));
   char* p = out + elem;
   if (NE == 8) *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
   else *reinterpret_cast<uint32_t*>(p) = w[0];
@@ -139,6 +142,31 @@ struct CastLocalArgs {
 
 constexpr int kCastThreads = 256;
 
+// Largest magnitude among the input elements of a scale block, which LANES consecutive lanes hold.
+// Scaling is monotonic, so it may be applied to the maximum; 16-bit elements are compared two at a time.
+template <int DT, int LANES>
+__device__ __forceinline__ float piece_amax(const uint32_t (&raw)[8]) {
+  if constexpr (DT == DT_F32) {
+    float m = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m = fmaxf(m, fabsf(__uint_as_float(raw[j])));
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    return m;
+  } else {
+    using T2 = typename std::conditional<DT == DT_BF16, __nv_bfloat162, __half2>::type;
+    auto as2 = [](uint32_t w) { return *reinterpret_cast<T2*>(&w); };
+    T2 m = __habs2(as2(raw[0]));
+#pragma unroll
+    for (int j = 1; j < 8; ++j) m = __hmax2(m, __habs2(as2(raw[j])));
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) m = __hmax2(m, as2(__shfl_xor_sync(0xffffffffu, *reinterpret_cast<uint32_t*>(&m), o)));
+    const uint32_t w = *reinterpret_cast<uint32_t*>(&m);
+    const float2 f = DT == DT_BF16 ? ptx::unpack_bf16x2(w) : ptx::unpack_f16x2(w);
+    return fmaxf(0.f, fmaxf(f.x, f.y));
+  }
+}
+
 template <int DT, int OUT, int U>
 __global__ void __launch_bounds__(kCastThreads, 4) cast_local_kernel(const __grid_constant__ CastLocalArgs a) {
   using V = Vec<DT>;
@@ -170,25 +198,25 @@ __global__ void __launch_bounds__(kCastThreads, 4) cast_local_kernel(const __gri
   for (int u = 0; u < U; ++u) {
     const size_t c = c0 + u * kCastThreads;
     const bool live = c < pieces, whole = (c + 1) * E <= a.elems;
-    float v[E];
+    // 0 + x, as a sum starts: a zero comes out positive
+    float2 v[E / 2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       V::add(acc, make_uint4(raw[u][4 * h], raw[u][4 * h + 1], raw[u][4 * h + 2], raw[u][4 * h + 3]));
 #pragma unroll
-      for (int e = 0; e < E / 2; ++e) v[h * (E / 2) + e] = acc[e] * a.scale;
+      for (int e = 0; e < E / 4; ++e) v[h * (E / 4) + e] = make_float2(acc[2 * e], acc[2 * e + 1]);
     }
+    const float factor = OUT == OUT_FP8 ? -a.scale : a.scale;  // the divisor takes its elements negated
+#pragma unroll
+    for (int e = 0; e < E / 2; ++e) v[e] = fp8::mul2(v[e], make_float2(factor, factor));
     char* out = a.out + c * E * (OUT == OUT_FP8 ? 1 : OUT == OUT_F32 ? 4 : 2);
     if (OUT == OUT_FP8) {
-      float amax = 0.f;
-#pragma unroll
-      for (int e = 0; e < E; ++e) amax = fmaxf(amax, fabsf(v[e]));
-#pragma unroll
-      for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      const float blockScale = fp8::block_scale(amax), inv = __frcp_rn(blockScale);
+      const float blockScale = fp8::block_scale(fabsf(piece_amax<DT, LANES>(raw[u]) * a.scale));
+      const fp8::Divisor div(blockScale);
       uint32_t w[E / 4];
 #pragma unroll
-      for (int j = 0; j < E / 4; ++j) w[j] = fp8::quantise4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3], blockScale, inv);
+      for (int j = 0; j < E / 4; ++j) w[j] = div.quantise4(v[2 * j], v[2 * j + 1]);
       if (live) {
         if constexpr (E == 16) ptx::st_global_v4(out, make_uint4(w[0], w[1], w[2], w[3]));
         else *reinterpret_cast<uint2*>(out) = make_uint2(w[0], w[1]);
@@ -199,7 +227,7 @@ __global__ void __launch_bounds__(kCastThreads, 4) cast_local_kernel(const __gri
       uint32_t w[W];
 #pragma unroll
       for (int j = 0; j < W; ++j)
-        w[j] = OUT == OUT_F32 ? __float_as_uint(v[j]) : OUT == OUT_BF16 ? ptx::pack_bf16x2(v[2 * j], v[2 * j + 1]) : ptx::pack_f16x2(v[2 * j], v[2 * j + 1]);
+        w[j] = OUT == OUT_F32 ? __float_as_uint((j & 1) ? v[j / 2].y : v[j / 2].x) : OUT == OUT_BF16 ? ptx::pack_bf16x2(v[j].x, v[j].y) : ptx::pack_f16x2(v[j].x, v[j].y);
       if (W == 4) {  // fp32 -> 16 bits: a piece is 16 output bytes, and a half piece is 8
         if (live && whole) ptx::st_global_v4(out, make_uint4(w[0], w[1], w[2], w[3]));
         else if (live) *reinterpret_cast<uint2*>(out) = make_uint2(w[0], w[1]);
