@@ -91,6 +91,54 @@ def test_norm_single_rank_shapes(tokens, hidden):
 
 
 @gpu
+@pytest.mark.parametrize("tokens,hidden,experts,topk,off", [
+    (1, 128, 1, 1, 0), (3, 1152, 4, 3, 8), (700, 1152, 16, 16, 0), (2000, 384, 8, 2, 0), (1300, 7168, 256, 8, 8), (65, 8192, 32, 5, 0)])
+def test_moe_single_rank_shapes(tokens, hidden, experts, topk, off):
+    """Rows of part of a warp up to 512 threads, scales that bulk copies cannot move, several tokens per CTA, unused
+    slots, an input on a 16-byte boundary only (`off` elements in front), every top-k class of the combine."""
+    import os
+
+    from unified_ccl_b200 import Communicator
+    from unified_ccl_b200.parallel import MoeDispatcher
+
+    os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    comm = Communicator(0, 1)
+    disp = MoeDispatcher(comm, tokens, hidden, experts, topk)
+    g = torch.Generator(device="cuda").manual_seed(tokens + hidden)
+    x = torch.randn(tokens * hidden + off, device="cuda", generator=g).to(torch.bfloat16)[off:].view(tokens, hidden)
+    w, idx = torch.softmax(torch.randn(tokens, experts, device="cuda", generator=g), -1).topk(min(topk, experts), dim=-1)
+    if topk > 2:
+        idx[tokens // 2, 1] = -1
+    idx, w = idx.to(torch.int32).contiguous(), w.contiguous()
+    for _ in range(2):  # the second call finds the counters the first one left
+        recv_x, recv_scale, recv_meta, counts = disp.dispatch(x, idx)
+        rows = int(counts[0])
+        assert rows == int((idx >= 0).sum())
+        meta = recv_meta[0, :rows].long()
+        key, order = (meta[:, 0] * topk + meta[:, 2]).sort()
+        assert torch.equal(key, (idx.view(-1) >= 0).nonzero().view(-1))
+        assert torch.equal(meta[order, 1], idx.view(-1)[key].long()) and (meta[:, 3] == 1).all()
+        blocks = x[meta[order, 0]].float().view(rows, hidden // 128, 128)
+        scale = blocks.abs().amax(-1, keepdim=True).clamp_min(1e-10)
+        scale = scale / torch.full_like(scale, 448.0)
+        q = (blocks / scale).to(torch.float8_e4m3fn).view(rows, hidden)
+        assert torch.equal(recv_scale[0, order], scale.view(rows, -1))
+        assert torch.equal(recv_x[0, order].view(torch.uint8), q.view(torch.uint8))
+    disp.expert_out.normal_(generator=g)
+    out = disp.combine(w)
+    ref = torch.zeros(tokens, hidden, device="cuda")
+    mag = torch.zeros_like(ref)
+    part = disp.expert_out[0, order].float() * w.view(-1)[key].unsqueeze(-1)
+    ref.index_add_(0, key // topk, part)
+    mag.index_add_(0, key // topk, part.abs())
+    # topk fp32 additions in another order, then one rounding to bf16
+    assert ((out.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + mag * topk * 2.0 ** -23).all()
+    assert disp.overflow() == 0
+    disp.close()
+    comm.destroy()
+
+
+@gpu
 def test_canaries_around_symmetric_buffers():
     assert_all_ok(run_ranks("canary", 1, env={"UCCL_CANARY": "1"}))
 
