@@ -3,7 +3,7 @@
 // tensor-parallel collective next to it.
 //
 //   warp 0      TMA producer : streams A and B tiles through a shared-memory ring, 128-byte swizzle
-//   warp 1      MMA issuer   : one elected lane issues tcgen05.mma, accumulators double-buffered in
+//   warp 1      MMA issuer   : one elected lane of the converged warp issues tcgen05.mma, accumulators double-buffered in
 //                              TMEM (2 x 256 columns) so the epilogue of tile i overlaps the main
 //                              loop of tile i+1
 //   warps 2..5  epilogue     : tcgen05.ld TMEM -> registers -> bf16 -> global (or -> shared -> TMA
@@ -181,7 +181,7 @@ __device__ __forceinline__ bool wait_flag_geq(const uint32_t* flag, uint32_t tar
   }
 }
 
-// The launch's rank barrier, run by lanes 1 .. nranks of one otherwise idle warp of GEMM CTA 0
+// The launch's rank barrier, run by lanes 1 .. nranks of the producer warp (lane 0 alone loads) of GEMM CTA 0
 // (lane p + 1 deals with rank p) while the GEMM roles already work on tiles that need no peer:
 // same words and epochs as the collectives' CTA barrier (coll_device.cuh rank_barrier), on a slot
 // of its own.  Raises `go` for everybody who is about to touch a peer.
@@ -849,6 +849,11 @@ __device__ __forceinline__ void publish_tile(const Args& a, int mb, int lane, ui
   }
 }
 
+// Bounded wait of a whole warp: every lane gets the same answer, so that the warp stays together.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* bail) {
+  return __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar, parity, bail));
+}
+
 // ------------------------------------------------------------------ single-CTA kernel
 template <int EPI, int COMM>
 __global__ void __launch_bounds__(COMM == kCommAllGather ? NUM_THREADS_FWD : NUM_THREADS, 1)
@@ -952,25 +957,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           ptx::tma_load_2d(sB + B_STAGE_BYTES / 2, &tmB, &full_bar[s], kb * BK, brow1);
         }
       }
+    } else if (COMM != kCommNone && a.comm.go && cta_id == 0) {
+      prologue_barrier(a.comm, lane, a.err);  // the warp's idle lanes run the launch's rank barrier
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = ptx::umma_idesc_f16(1u, BM, BN);
-      uint32_t it = 0, tcount = 0;
-      for (int tile = cta_id; tile < num_tiles && !*bail; tile += gemm_ctas, ++tcount) {
-        const uint32_t acc = tcount & 1, acc_ph = (tcount >> 1) & 1;
-        if (!ptx::mbar_wait_bounded(&tempty_bar[acc], acc_ph ^ 1, bail)) break;
+    // ------------------------------------------------------------ MMA issuer (see the pair kernel on its form)
+    constexpr uint32_t idesc = ptx::umma_idesc_f16(1u, BM, BN);
+    const bool issue = ptx::elect_one();
+    uint32_t it = 0, tcount = 0;
+    for (int tile = cta_id; tile < num_tiles; tile += gemm_ctas, ++tcount) {
+      const uint32_t acc = tcount & 1, acc_ph = (tcount >> 1) & 1;
+      if (!warp_wait(&tempty_bar[acc], acc_ph ^ 1, bail)) break;
+      ptx::tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      bool ok = true;
+      for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        const int s = it % STAGES;
+        const uint32_t ph = (it / STAGES) & 1;
+        if (!(ok = warp_wait(&full_bar[s], ph, bail))) break;
         ptx::tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!ptx::mbar_wait_bounded(&full_bar[s], ph, bail)) break;
-          ptx::tc_fence_after();
-          const uint32_t sA = ptx::smem_u32(smem + s * STAGE_BYTES);
-          const uint64_t da = ptx::umma_smem_desc_sw128(sA);
-          const uint64_t db = ptx::umma_smem_desc_sw128(sA + A_STAGE_BYTES);
+        const uint32_t sA = ptx::smem_u32(smem + s * STAGE_BYTES);
+        const uint64_t da = ptx::umma_smem_desc_sw128(sA);
+        const uint64_t db = ptx::umma_smem_desc_sw128(sA + A_STAGE_BYTES);
+        if (issue) {
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t koff = static_cast<uint64_t>((k * UMMA_K * 2) >> 4);
@@ -978,10 +987,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
           ptx::umma_commit(&empty_bar[s]);
         }
-        ptx::umma_commit(&tfull_bar[acc]);
+        __syncwarp();
       }
-    } else if (COMM != kCommNone && a.comm.go && cta_id == 0) {
-      prologue_barrier(a.comm, lane, a.err);  // the warp's idle lanes run the launch's rank barrier
+      if (!ok) break;
+      if (issue) ptx::umma_commit(&tfull_bar[acc]);
+      __syncwarp();
     }
   } else if (warp == 6) {
     // ------------------------------------------------------------ forwarder (all-gather, spread mode)
@@ -1121,8 +1131,6 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const uint32_t tmem_base = *tmem_holder;
   const uint32_t full0 = ptx::mapa(ptx::smem_u32(&full_bar[0]), 0);
   const uint32_t tempty0 = ptx::mapa(ptx::smem_u32(&tempty_bar[0]), 0);
-  const uint32_t empty_peer = ptx::mapa(ptx::smem_u32(&empty_bar[0]), 1);
-  const uint32_t tfull_peer = ptx::mapa(ptx::smem_u32(&tfull_bar[0]), 1);
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -1161,39 +1169,48 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           ptx::tma_load_2d_pair(sB, &tmB, fb, kb * BK, brow);
         }
       }
+    } else if (COMM != kCommNone && a.comm.go && cta_id == 0) {
+      prologue_barrier(a.comm, lane, a.err);  // the warp's idle lanes run the launch's rank barrier
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader only)
-    if (leader && lane == 0) {
+    // The whole warp walks the loop and one elected lane issues.  The tensor core holds few
+    // instructions ahead, so the issuer's own path between two stages shows: with a single lane in a
+    // divergent branch and one commit per CTA a stage of 512 tensor cycles took 670 (no loads at all
+    // made no difference), in this form 525.  16384 x 4096 x 14336: 1571 -> 1397 us (1.38 PFLOP/s,
+    // against the power cap), zeros 1153 -> 997 us; 2048 x 4096 x 4096: 58 -> 51 us.
+    if (leader) {
       constexpr uint32_t idesc = ptx::umma_idesc_f16(1u, 2 * BM, BN);
+      const bool issue = ptx::elect_one();
       uint32_t it = 0, tcount = 0;
-      for (int tile = pair_id; tile < num_tiles && !*bail; tile += pairs, ++tcount) {
+      for (int tile = pair_id; tile < num_tiles; tile += pairs, ++tcount) {
         const uint32_t acc = tcount & 1, acc_ph = (tcount >> 1) & 1;
-        if (!ptx::mbar_wait_bounded(&tempty_bar[acc], acc_ph ^ 1, bail)) break;
+        if (!warp_wait(&tempty_bar[acc], acc_ph ^ 1, bail)) break;
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
+        bool ok = true;
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % ST;
           const uint32_t ph = (it / ST) & 1;
-          if (!ptx::mbar_wait_bounded(&full_bar[s], ph, bail)) break;
+          if (!(ok = warp_wait(&full_bar[s], ph, bail))) break;
           ptx::tc_fence_after();
           const uint32_t sA = ptx::smem_u32(smem + s * pair::STAGE_BYTES);
           const uint64_t da = ptx::umma_smem_desc_sw128(sA);
           const uint64_t db = ptx::umma_smem_desc_sw128(sA + pair::A_BYTES);
+          if (issue) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t koff = static_cast<uint64_t>((k * UMMA_K * 2) >> 4);
-            ptx::umma_f16_pair(d_tmem, da + koff, db + koff, idesc, (kb | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              const uint64_t koff = static_cast<uint64_t>((k * UMMA_K * 2) >> 4);
+              ptx::umma_f16_pair(d_tmem, da + koff, db + koff, idesc, (kb | k) != 0 ? 1u : 0u);
+            }
+            ptx::umma_commit_both(&empty_bar[s]);  // the stage is free in both CTAs once these MMAs have read it
           }
-          // the stage is free in both CTAs once these MMAs have read it
-          ptx::umma_commit_pair(ptx::smem_u32(&empty_bar[s]));
-          ptx::umma_commit_pair(empty_peer + static_cast<uint32_t>(s) * 8);
+          __syncwarp();
         }
-        ptx::umma_commit_pair(ptx::smem_u32(&tfull_bar[acc]));
-        ptx::umma_commit_pair(tfull_peer + acc * 8);
+        if (!ok) break;
+        if (issue) ptx::umma_commit_both(&tfull_bar[acc]);
+        __syncwarp();
       }
-    } else if (COMM != kCommNone && a.comm.go && cta_id == 0) {
-      prologue_barrier(a.comm, lane, a.err);  // the warp's idle lanes run the launch's rank barrier
     }
   } else if (warp == 6) {
     // ------------------------------------------------------------ forwarder (all-gather, spread mode)
