@@ -1,0 +1,366 @@
+// The GEMM without a collective: C[M,N] = A[M,K] * B[N,K]^T, or silu(A Bg^T) * (A Bu^T), bf16 in and out, fp32
+// sums.  Same roles as the fused kernels of gemm_sm100.cuh (producer warp, issuer warp, four epilogue warps,
+// accumulators double-buffered in TMEM); what is free here is the cut of the work, chosen per shape by the
+// launcher (choosePlain in gemm_sm100.cu):
+//
+//   CG      CTAs that share a tile: 2 (256 rows, tcgen05 cta_group::2) or 1 (128 rows)
+//   bn      columns of B rows per tile, 16 to 256: a narrower tile than 256 where it fills the last wave
+//   split   parts that K is cut in, one group of CG CTAs each, all in one cluster.  They add their sums up
+//           through distributed shared memory, so that few tiles over a long K (a handful of tokens, a small
+//           weight) still use most SMs and no workspace or second launch is needed.
+//
+// A tile's stage of the ring holds 64 columns of K: the A rows and bn / CG rows of B.  With fewer than 128
+// rows in all the A part holds just these (a_rows); the tensor core then reads rows of B where the rest of A
+// would be, which only reaches accumulator rows that nobody looks at.
+#pragma once
+#include "gemm_sm100.cuh"
+
+namespace uccl {
+namespace gemm {
+namespace plain {
+
+constexpr int MAX_STAGES = 24;
+constexpr int MAX_CLUSTER = 8;
+constexpr int SMEM = PIPE_BYTES + EPI_STAGE_BYTES + 1024 /*align slack*/ + 512 /*barriers*/;
+
+struct Args {
+  __nv_bfloat16* C;
+  int ldc;
+  int M, out_n;          // rows and columns of C
+  int num_kb;            // stages of 64 columns of K
+  int tiles_m, num_tiles;
+  int tiles_n;
+  int bn, out_bn;        // accumulator columns and output columns of a tile
+  int tma_bn;            // out_bn, or 0 if no tensor map describes C
+  int b_half_rows;       // SwiGLU: row offset of the "up" half inside B
+  int a_rows;            // rows of A in a stage (128, or fewer when M is)
+  int stages, stage_bytes;
+  int split, workers;    // clusters in the grid; one tile each if split > 1
+  uint32_t* err;
+};
+
+// GROUP consecutive row tiles share a sweep over the column tiles
+template <int GROUP>
+__device__ __forceinline__ void coords(const Args& a, int tile, int& mt, int& nt) {
+  const int per_group = GROUP * a.tiles_n;
+  const int g = tile / per_group, first = g * GROUP;
+  const int gsz = min(GROUP, a.tiles_m - first);
+  const int r = tile - g * per_group;
+  nt = r / gsz;
+  mt = first + (r - nt * gsz);
+}
+
+// 16 output columns of one row as bf16 pairs
+template <int EPI>
+__device__ __forceinline__ void pack16(const uint32_t (&x)[16], const uint32_t (&y)[16], uint32_t (&o)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float p = __uint_as_float(x[2 * j]), q = __uint_as_float(x[2 * j + 1]);
+    if (EPI == kEpiSwiGLU) o[j] = ptx::pack_bf16x2(silu_f(p) * __uint_as_float(y[2 * j]), silu_f(q) * __uint_as_float(y[2 * j + 1]));
+    else o[j] = ptx::pack_bf16x2(p, q);
+  }
+}
+__device__ __forceinline__ void store16(const Args& a, int row, int col, const uint32_t (&o)[8]) {
+  if (row >= a.M) return;
+  __nv_bfloat16* p = a.C + static_cast<size_t>(row) * a.ldc + col;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (col + h * 8 + 8 <= a.out_n) {
+      *reinterpret_cast<uint4*>(p + h * 8) = make_uint4(o[4 * h], o[4 * h + 1], o[4 * h + 2], o[4 * h + 3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (col + h * 8 + j < a.out_n) reinterpret_cast<uint16_t*>(p)[h * 8 + j] = static_cast<uint16_t>(o[4 * h + j / 2] >> (16 * (j & 1)));
+    }
+  }
+}
+
+// The whole tile of one warp (32 rows from row0): 64 output columns at a time through shared memory and TMA
+// stores, which clip what lies outside C; the columns that are left in units of 16 straight from registers.
+template <int EPI>
+__device__ __forceinline__ void store_tile(const Args& a, const CUtensorMap* tmC, uint32_t taddr, int row0, int col0, int lane,
+                                           uint8_t* stage, uint32_t& stage_it) {
+  if (row0 >= a.M) return;
+  int c = 0;
+#pragma unroll 1
+  for (; c + 64 <= a.tma_bn && col0 + c < a.out_n; c += 64) {
+    uint4 v[8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t x[32], y[32];
+      ptx::tmem_ld_32x32b_x32(taddr + c + h * 32, x);
+      if (EPI == kEpiSwiGLU) ptx::tmem_ld_32x32b_x32(taddr + a.out_bn + c + h * 32, y);
+      ptx::tmem_ld_wait();
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        uint32_t o[8];
+        pack16<EPI>(*reinterpret_cast<const uint32_t(*)[16]>(&x[g * 16]), *reinterpret_cast<const uint32_t(*)[16]>(&y[g * 16]), o);
+        v[h * 4 + g * 2] = make_uint4(o[0], o[1], o[2], o[3]);
+        v[h * 4 + g * 2 + 1] = make_uint4(o[4], o[5], o[6], o[7]);
+      }
+    }
+    stage_and_store<2>(tmC, v, col0 + c, row0, true, lane, stage, stage_it);
+  }
+#pragma unroll 1
+  for (; c < a.out_bn && col0 + c < a.out_n; c += 16) {
+    uint32_t x[16], y[16], o[8];
+    ptx::tmem_ld_32x32b_x16(taddr + c, x);
+    if (EPI == kEpiSwiGLU) ptx::tmem_ld_32x32b_x16(taddr + a.out_bn + c, y);
+    ptx::tmem_ld_wait();
+    pack16<EPI>(x, y, o);
+    store16(a, row0 + lane, col0 + c, o);
+    __syncwarp();
+  }
+}
+
+// split > 1, after a cluster barrier that follows everybody's last MMA: part s of the cluster owns output columns
+// [s, s + 1) * out_bn / split.  Every warp hands the other parts their columns of its 32 rows (into the ring, which
+// is idle now: slot of the source, then 16-byte pieces of four columns, 128 rows of each), and after a second
+// barrier adds up what it got in the order of K.
+__device__ __forceinline__ uint32_t part_addr(const Args& a, uint32_t ring, int dst, int src, int halves, int piece, int r) {
+  const int slot = src < dst ? src : src - 1;
+  const int pieces = halves * (a.out_bn / a.split) / 4;
+  return ring + static_cast<uint32_t>(((slot * pieces + piece) * BM + r) * 16);
+}
+template <int EPI>
+__device__ __forceinline__ void send_parts(const Args& a, uint32_t ring, uint32_t taddr, int part, int rank0, int cg, int r) {
+  constexpr int H = EPI == kEpiSwiGLU ? 2 : 1;
+  const int w = a.out_bn / a.split;
+#pragma unroll 1
+  for (int i = 1; i < a.split; ++i) {
+    const int dst = part + i < a.split ? part + i : part + i - a.split;
+    const uint32_t remote = ptx::mapa(ring, static_cast<uint32_t>(dst * cg + rank0));
+#pragma unroll 1
+    for (int c = 0; c < w; c += 16) {
+      uint32_t x[H][16];
+#pragma unroll
+      for (int h = 0; h < H; ++h) ptx::tmem_ld_32x32b_x16(taddr + h * a.out_bn + dst * w + c, x[h]);
+      ptx::tmem_ld_wait();
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          ptx::st_cluster_v4(part_addr(a, remote, dst, part, H, (h * w + c) / 4 + j, r),
+                             make_uint4(x[h][4 * j], x[h][4 * j + 1], x[h][4 * j + 2], x[h][4 * j + 3]));
+    }
+  }
+}
+template <int EPI>
+__device__ __forceinline__ void sum_parts(const Args& a, const uint8_t* ring, uint32_t taddr, int part, int row, int col0, int r) {
+  constexpr int H = EPI == kEpiSwiGLU ? 2 : 1;
+  const int w = a.out_bn / a.split;
+#pragma unroll 1
+  for (int c = 0; c < w && col0 + part * w + c < a.out_n; c += 16) {
+    uint32_t own[H][16];
+    float sum[H][16];
+#pragma unroll
+    for (int h = 0; h < H; ++h) ptx::tmem_ld_32x32b_x16(taddr + h * a.out_bn + part * w + c, own[h]);
+    ptx::tmem_ld_wait();
+#pragma unroll 1
+    for (int s = 0; s < a.split; ++s) {
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float4 v;
+          if (s == part) v = make_float4(__uint_as_float(own[h][4 * j]), __uint_as_float(own[h][4 * j + 1]), __uint_as_float(own[h][4 * j + 2]), __uint_as_float(own[h][4 * j + 3]));
+          else v = *reinterpret_cast<const float4*>(ring + part_addr(a, 0, part, s, H, (h * w + c) / 4 + j, r));
+          sum[h][4 * j] = s == 0 ? v.x : sum[h][4 * j] + v.x;
+          sum[h][4 * j + 1] = s == 0 ? v.y : sum[h][4 * j + 1] + v.y;
+          sum[h][4 * j + 2] = s == 0 ? v.z : sum[h][4 * j + 2] + v.z;
+          sum[h][4 * j + 3] = s == 0 ? v.w : sum[h][4 * j + 3] + v.w;
+        }
+      }
+    }
+    uint32_t x[16], y[16], o[8];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      x[j] = __float_as_uint(sum[0][j]);
+      y[j] = __float_as_uint(sum[H - 1][j]);
+    }
+    pack16<EPI>(x, y, o);
+    store16(a, row, col0 + part * w + c, o);
+    __syncwarp();
+  }
+}
+
+template <int EPI, int CG>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ Args a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + PIPE_BYTES + EPI_STAGE_BYTES);  // CG 2: used in the leader
+  uint64_t* empty_bar = full_bar + MAX_STAGES;
+  uint64_t* tfull_bar = empty_bar + MAX_STAGES;
+  uint64_t* tempty_bar = tfull_bar + 2;  // CG 2: used in the leader
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty_bar + 2);
+  volatile uint32_t* bail = tmem_holder + 1;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int csize = CG * a.split;
+  const int crank = csize > 1 ? static_cast<int>(ptx::cluster_ctarank()) : 0;
+  const int part = crank / CG, half = crank % CG;  // part of K, CTA of the pair
+  const bool leader = half == 0;
+  const int worker = static_cast<int>(blockIdx.x) / csize;
+  const int kb0 = a.split > 1 ? a.num_kb * part / a.split : 0;
+  const int kb1 = a.split > 1 ? a.num_kb * (part + 1) / a.split : a.num_kb;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < a.stages; ++s) {
+      ptx::mbar_init(&full_bar[s], 1);
+      ptx::mbar_init(&empty_bar[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      ptx::mbar_init(&tfull_bar[i], 1);
+      ptx::mbar_init(&tempty_bar[i], 4 * CG);
+    }
+    *bail = 0;
+    ptx::mbar_fence_init();
+    ptx::prefetch_tmap(&tmA);
+    ptx::prefetch_tmap(&tmB);
+    if (a.tma_bn) ptx::prefetch_tmap(&tmC);
+  }
+  if (warp == 1) {
+    if (CG == 2) {
+      ptx::tmem_alloc_pair(tmem_holder, TMEM_COLS);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(tmem_holder, TMEM_COLS);
+      ptx::tmem_relinquish();
+    }
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (CG == 2) ptx::cluster_sync();  // both CTAs' barriers and TMEM exist before anybody signals the other
+  ptx::tc_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      const uint32_t lead_full = CG == 2 ? ptx::mapa(ptx::smem_u32(full_bar), static_cast<uint32_t>(crank - half)) : 0;
+      const uint32_t bytes = static_cast<uint32_t>(CG * a.stage_bytes);
+      int s = 0;
+      uint32_t ph = 1;
+      for (int tile = worker; tile < a.num_tiles && !*bail; tile += a.workers) {
+        int mt, nt;
+        coords<CG == 2 ? 8 : 16>(a, tile, mt, nt);
+        const int m0 = (mt * CG + half) * BM;
+        const int b0 = nt * (EPI == kEpiSwiGLU ? a.out_bn : a.bn);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!ptx::mbar_wait_bounded(&empty_bar[s], ph, bail)) break;
+          uint8_t* sA = smem + s * a.stage_bytes;
+          uint8_t* sB = sA + a.a_rows * (BK * 2);
+          if (CG == 2) {
+            if (leader) ptx::mbar_expect_tx(&full_bar[s], bytes);
+            const uint32_t fb = lead_full + static_cast<uint32_t>(s) * 8;
+            ptx::tma_load_2d_pair(sA, &tmA, fb, kb * BK, m0);
+            ptx::tma_load_2d_pair(sB, &tmB, fb, kb * BK, leader ? b0 : b0 + (EPI == kEpiSwiGLU ? a.b_half_rows : a.bn / 2));
+          } else {
+            ptx::mbar_expect_tx(&full_bar[s], bytes);
+            ptx::tma_load_2d(sA, &tmA, &full_bar[s], kb * BK, m0);
+            ptx::tma_load_2d(sB, &tmB, &full_bar[s], kb * BK, b0);
+            if (EPI == kEpiSwiGLU) ptx::tma_load_2d(sB + a.out_bn * (BK * 2), &tmB, &full_bar[s], kb * BK, b0 + a.b_half_rows);
+          }
+          if (++s == a.stages) s = 0, ph ^= 1;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer: the warp stays converged (see the
+    // pair kernel of gemm_sm100.cuh), one elected lane issues
+    if (leader) {
+      const uint32_t idesc = ptx::umma_idesc_f16(1u, CG * BM, static_cast<uint32_t>(a.bn));
+      const bool issue = ptx::elect_one();
+      int s = 0;
+      uint32_t ph = 0, tcount = 0;
+      for (int tile = worker; tile < a.num_tiles; tile += a.workers, ++tcount) {
+        const uint32_t acc = tcount & 1, acc_ph = (tcount >> 1) & 1;
+        if (!warp_wait(&tempty_bar[acc], acc_ph ^ 1, bail)) break;
+        ptx::tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * BN;
+        bool ok = true;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!(ok = warp_wait(&full_bar[s], ph, bail))) break;
+          ptx::tc_fence_after();
+          const uint32_t sA = ptx::smem_u32(smem) + static_cast<uint32_t>(s * a.stage_bytes);
+          const uint64_t da = ptx::umma_smem_desc_sw128(sA);
+          const uint64_t db = ptx::umma_smem_desc_sw128(sA + static_cast<uint32_t>(a.a_rows * (BK * 2)));
+          if (issue) {
+#pragma unroll
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              const uint64_t koff = static_cast<uint64_t>((k * UMMA_K * 2) >> 4);
+              const uint32_t accumulate = (kb != kb0 || k != 0) ? 1u : 0u;
+              if (CG == 2) ptx::umma_f16_pair(d_tmem, da + koff, db + koff, idesc, accumulate);
+              else ptx::umma_f16(d_tmem, da + koff, db + koff, idesc, accumulate);
+            }
+            if (CG == 2) ptx::umma_commit_both(&empty_bar[s], crank);
+            else ptx::umma_commit(&empty_bar[s]);
+          }
+          __syncwarp();
+          if (++s == a.stages) s = 0, ph ^= 1;
+        }
+        if (!ok) break;
+        if (issue) {
+          if (CG == 2) ptx::umma_commit_both(&tfull_bar[acc], crank);
+          else ptx::umma_commit(&tfull_bar[acc]);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue warps
+    const int q = warp & 3;  // TMEM lane quarter this warp may access
+    uint8_t* stage = smem + PIPE_BYTES + q * 2 * EPI_BUF_BYTES;
+    const uint32_t lead_tempty = CG == 2 ? ptx::mapa(ptx::smem_u32(tempty_bar), static_cast<uint32_t>(crank - half)) : 0;
+    uint32_t tcount = 0, stage_it = 0;
+    for (int tile = worker; tile < a.num_tiles; tile += a.workers, ++tcount) {
+      const uint32_t acc = tcount & 1, acc_ph = (tcount >> 1) & 1;
+      if (!warp_wait(&tfull_bar[acc], acc_ph, bail)) break;
+      if (a.split > 1) break;  // one tile, finished below
+      int mt, nt;
+      coords<CG == 2 ? 8 : 16>(a, tile, mt, nt);
+      ptx::tc_fence_after();
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
+      store_tile<EPI>(a, &tmC, taddr, (mt * CG + half) * BM + q * 32, nt * a.out_bn, lane, stage, stage_it);
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 2) ptx::mbar_arrive_cluster(lead_tempty + acc * 8);
+        else ptx::mbar_arrive(&tempty_bar[acc]);
+      }
+    }
+    if (lane == 0) ptx::tma_store_wait<0>();  // staging buffers stay valid until read
+    __syncwarp();
+  }
+
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (a.split > 1) {
+    int mt, nt;
+    coords<CG == 2 ? 8 : 16>(a, worker, mt, nt);
+    const int q = warp & 3, r = q * 32 + lane, row = (mt * CG + half) * BM + r;
+    const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    const bool busy = warp >= 2 && row - lane < a.M;
+    ptx::cluster_sync();  // every part has used up its ring
+    ptx::tc_fence_after();
+    if (busy) send_parts<EPI>(a, ptx::smem_u32(smem), taddr, part, half, CG, r);
+    __syncwarp();
+    ptx::cluster_sync();
+    if (busy) sum_parts<EPI>(a, smem, taddr, part, row, nt * a.out_bn, r);
+    ptx::tc_fence_before();
+    __syncthreads();
+  }
+  if (CG == 2) ptx::cluster_sync();  // nobody leaves while the other CTA may still signal it or read its memory
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    if (CG == 2) ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else ptx::tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+  if (threadIdx.x == 0 && *bail && a.err) atomicCAS(a.err, 0u, 0x47454d31u);
+}
+
+}  // namespace plain
+}  // namespace gemm
+}  // namespace uccl

@@ -11,6 +11,7 @@
 #include "../core/cuda_driver.h"
 #include "../core/log.h"
 #include "device_comm.h"
+#include "gemm_plain.cuh"
 #include "gemm_sm100.cuh"
 
 namespace uccl {
@@ -52,11 +53,11 @@ bool makeTensorMap(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t co
 // Raises the dynamic shared-memory limit of one kernel once per (thread, device). The caller owns
 // the two state words, one pair per kernel: kernels of equal signature share a function type.
 template <typename Kern>
-cudaError_t ensureSmem(Kern kern, int* last_dev, cudaError_t* err) {
+cudaError_t ensureSmem(Kern kern, int* last_dev, cudaError_t* err, int bytes = gemm::SMEM_BYTES) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev != *last_dev) {
-    *err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm::SMEM_BYTES);
+    *err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     *last_dev = dev;
   }
   return *err;
@@ -88,42 +89,181 @@ cudaError_t launchPairT(const CUtensorMap& tmA, const CUtensorMap& tmB, const ge
   return cudaGetLastError();
 }
 
-// Clusters of two CTAs that fit on the device at once (one CTA per SM; GPCs with an odd number of
-// usable SMs leave one SM unpaired).
-int maxResidentPairs() {
-  static int cached[64];
+// Clusters of `csize` CTAs that fit on the device at once (one CTA per SM; what a GPC's SMs do not divide into
+// stays unused).
+template <int CG>
+int residentClusters(int csize) {
+  static int cached[64][gemm::plain::MAX_CLUSTER + 1];
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return deviceSmCount() / 2;
-  if (cached[dev] == 0) {
-    auto kern = gemm::gemm2_bf16_kernel<gemm::kEpiStore, gemm::kCommNone>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm::SMEM_BYTES);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * deviceSmCount(), 1, 1);
-    cfg.blockDim = dim3(gemm::NUM_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = gemm::SMEM_BYTES;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
-      (void)cudaGetLastError();
-      n = deviceSmCount() / 2 - 4;
-    }
-    cached[dev] = n;
-    UCCL_LOG(INFO, "gemm: %d CTA pairs can be resident on device %d", n, dev);
+  const bool keep = dev >= 0 && dev < 64;
+  if (keep && cached[dev][csize] != 0) return cached[dev][csize];
+  auto kern = gemm::plain::gemm_plain_kernel<gemm::kEpiStore, CG>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm::plain::SMEM);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(csize * deviceSmCount(), 1, 1);
+  cfg.blockDim = dim3(gemm::NUM_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = gemm::plain::SMEM;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = csize;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+    (void)cudaGetLastError();
+    n = std::max(1, deviceSmCount() / csize - 4);
   }
-  return cached[dev];
+  if (keep) cached[dev][csize] = n;
+  UCCL_LOG(INFO, "gemm: %d clusters of %d CTAs can be resident on device %d", n, csize, dev);
+  return n;
 }
+int maxResidentPairs() { return residentClusters<2>(2); }
 
 // UCCL_GEMM_PAIR=0 selects the single-CTA kernel, 1 the CTA-pair kernel (default).
 bool usePairKernel() {
   const char* s = getenv("UCCL_GEMM_PAIR");
   return (s && *s) ? atoi(s) != 0 : true;
+}
+
+struct PlainPlan {
+  int cg, bn, split;
+};
+
+// How to cut a GEMM without a collective.  Cycles of a candidate: waves of tiles x stages per tile x the longer of
+// the tensor cores' time for a stage (two cycles per accumulator column, at least a round trip of the ring) and its
+// loads (78 bytes per cycle and SM), at least the time of memory, plus a tile's epilogue or the exchange of the
+// parts.  The constants are a fit to 102 shapes with every candidate measured (1 to 6000 rows, B of 0.1 to 240 MB):
+// the choice is within 2% of the best candidate on average.
+PlainPlan choosePlain(int M, int N, int K, bool swiglu, int max_ctas) {
+  PlainPlan best = {1, 256, 1};
+#ifdef UCCL_EXPERIMENTS
+  if (const char* e = getenv("UCCL_GEMM_PLAN")) {
+    if (sscanf(e, "%d,%d,%d", &best.cg, &best.bn, &best.split) == 3) return best;
+  }
+#endif
+  const bool pairs = usePairKernel();
+  const int num_kb = (K + gemm::BK - 1) / gemm::BK;
+  const int out_n = swiglu ? N / 2 : N;
+  const double bytes = 2.0 * (static_cast<double>(M) * K + static_cast<double>(N) * K + static_cast<double>(M) * out_n);
+  double best_t = 1e300;
+  for (int cg = 1; cg <= (pairs ? 2 : 1); ++cg) {
+    const int tiles_m = (M + cg * gemm::BM - 1) / (cg * gemm::BM);
+    const int a_rows = cg == 1 && M < gemm::BM ? (M + 7) / 8 * 8 : gemm::BM;
+    const int step = cg == 2 || swiglu ? 32 : 16;
+    for (int split = 1; split * cg <= gemm::plain::MAX_CLUSTER && split <= num_kb; split *= 2) {
+      int resident = cg == 2 ? residentClusters<2>(2 * split) : residentClusters<1>(split);
+      if (max_ctas > 0) resident = std::max(1, std::min(resident, max_ctas / (cg * split)));
+      const int kbs = (num_kb + split - 1) / split;
+      for (int bn = step; bn <= gemm::BN; bn += step) {
+        const int out_bn = swiglu ? bn / 2 : bn;
+        if (split > 1 && out_bn % (16 * split) != 0) continue;
+        const int tiles = tiles_m * ((out_n + out_bn - 1) / out_bn);
+        if (split > 1 && tiles > resident) continue;
+        const int waves = (tiles + resident - 1) / resident;
+        const double stage = std::max(std::max(2.0 * bn, 329.0) + 54.0, (a_rows + bn / cg) * 128.0 / 78.0);
+        const double memory = bytes / std::min(3500.0, std::min(tiles, resident) * cg * split * 83.0);
+        double t = std::max(memory, waves * kbs * stage) + waves * 34.0;
+        if (split == 1) t += 8.0 * bn;
+        else t += 3100.0 + 280.0 * split + 30.0 * bn * std::min(M, cg * gemm::BM) / (cg * gemm::BM);
+        if (t < best_t) {
+          best_t = t;
+          best = {cg, bn, split};
+        }
+      }
+    }
+  }
+  return best;
+}
+
+// The choice is a function of the shape alone: each thread keeps a few.
+PlainPlan planFor(int M, int N, int K, bool swiglu, int max_ctas) {
+#ifdef UCCL_EXPERIMENTS
+  return choosePlain(M, N, K, swiglu, max_ctas);
+#endif
+  struct Entry {
+    int M, N, K, flags, dev;
+    PlainPlan plan;
+  };
+  static thread_local Entry table[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int flags = (swiglu ? 1 : 0) | (usePairKernel() ? 2 : 0) | (max_ctas << 2);
+  const uint32_t h = static_cast<uint32_t>(M) * 2654435761u ^ static_cast<uint32_t>(N) * 2246822519u ^ static_cast<uint32_t>(K) * 3266489917u;
+  Entry& e = table[(h >> 20) & 63];
+  if (e.M != M || e.N != N || e.K != K || e.flags != flags || e.dev != dev) {
+    e.plan = choosePlain(M, N, K, swiglu, max_ctas);
+    e.M = M, e.N = N, e.K = K, e.flags = flags, e.dev = dev;
+  }
+  return e.plan;
+}
+
+template <int EPI, int CG>
+cudaError_t launchPlainT(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const gemm::plain::Args& args,
+                         cudaStream_t stream) {
+  auto kern = gemm::plain::gemm_plain_kernel<EPI, CG>;
+  static thread_local int last_dev = -1;
+  static thread_local cudaError_t attr_err = cudaSuccess;
+  cudaError_t e = ensureSmem(kern, &last_dev, &attr_err, gemm::plain::SMEM);
+  if (e != cudaSuccess) return e;
+  const int csize = CG * args.split;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(args.workers * csize, 1, 1);
+  cfg.blockDim = dim3(gemm::NUM_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = gemm::plain::SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = csize;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = csize > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, args);
+}
+
+ucclResult_t launchPlain(const GemmLaunch& g, cudaStream_t stream) {
+  const bool swiglu = g.epilogue == gemm::kEpiSwiGLU;
+  const int out_n = swiglu ? g.N / 2 : g.N;
+  const PlainPlan p = planFor(g.M, g.N, g.K, swiglu, g.max_ctas);
+  gemm::plain::Args a = {};
+  a.C = static_cast<__nv_bfloat16*>(g.C);
+  a.ldc = g.ldc;
+  a.M = g.M;
+  a.out_n = out_n;
+  a.num_kb = (g.K + gemm::BK - 1) / gemm::BK;
+  a.bn = p.bn;
+  a.out_bn = swiglu ? p.bn / 2 : p.bn;
+  a.b_half_rows = swiglu ? g.N / 2 : 0;
+  a.a_rows = p.cg == 1 && g.M < gemm::BM ? (g.M + 7) / 8 * 8 : gemm::BM;
+  a.tiles_m = (g.M + p.cg * gemm::BM - 1) / (p.cg * gemm::BM);
+  a.tiles_n = (out_n + a.out_bn - 1) / a.out_bn;
+  a.num_tiles = a.tiles_m * a.tiles_n;
+  a.stage_bytes = (a.a_rows + p.bn / p.cg) * gemm::BK * 2;
+  a.stages = std::min(gemm::plain::MAX_STAGES, gemm::PIPE_BYTES / a.stage_bytes);
+  a.split = p.split;
+  a.err = g.err;
+  // the stride of a single row means nothing; rows that overlap have no tensor map
+  const int ldc = g.M == 1 ? (out_n + 7) / 8 * 8 : g.ldc;
+  const bool mapped = ldc >= out_n;
+  a.tma_bn = mapped ? a.out_bn : 0;
+  int resident = p.cg == 2 ? maxResidentPairs() : deviceSmCount();
+  if (g.max_ctas > 0) resident = std::max(1, std::min(resident, g.max_ctas / p.cg));
+  a.workers = p.split > 1 ? a.num_tiles : std::min(a.num_tiles, resident);
+  CUtensorMap tmA, tmB, tmC = {};
+  if (!makeTensorMap(&tmA, g.A, g.M, g.K, g.lda, gemm::BK, a.a_rows) || !makeTensorMap(&tmB, g.B, g.N, g.K, g.ldb, gemm::BK, swiglu || p.cg == 2 ? p.bn / 2 : p.bn) ||
+      (mapped && !makeTensorMap(&tmC, g.C, g.M, out_n, ldc, 64, 32)))
+    return ucclSystemError;
+  cudaError_t e;
+  if (swiglu) e = p.cg == 2 ? launchPlainT<gemm::kEpiSwiGLU, 2>(tmA, tmB, tmC, a, stream) : launchPlainT<gemm::kEpiSwiGLU, 1>(tmA, tmB, tmC, a, stream);
+  else e = p.cg == 2 ? launchPlainT<gemm::kEpiStore, 2>(tmA, tmB, tmC, a, stream) : launchPlainT<gemm::kEpiStore, 1>(tmA, tmB, tmC, a, stream);
+  if (e != cudaSuccess) {
+    UCCL_LOG(ERROR, "gemm launch failed: %s", cudaGetErrorString(e));
+    return ucclSystemError;
+  }
+  return ucclSuccess;
 }
 
 }  // namespace
@@ -137,6 +277,7 @@ ucclResult_t launchGemmBf16(const GemmLaunch& g, const GemmFusion* f, cudaStream
   const int role = f ? f->role : 0;
   if (role == gemm::kCommReduceScatter && g.epilogue != gemm::kEpiStore)
     return ucclInvalidArgument;
+  if (role == 0) return launchPlain(g, stream);
 
   CUtensorMap tmA, tmB;
   if (!makeTensorMap(&tmA, g.A, g.M, g.K, g.lda, gemm::BK, gemm::BM)) return ucclSystemError;
@@ -177,7 +318,7 @@ ucclResult_t launchGemmBf16(const GemmLaunch& g, const GemmFusion* f, cudaStream
   const int sms = g.max_ctas > 0 ? g.max_ctas : deviceSmCount();
   gemm::PeerMaps pm = {};
   int comm_ctas = 0;
-  if (role != 0) {
+  {
     if (f->nranks > gemm::kMaxPeers || f->rows_per_rank % gemm::BM != 0) return ucclInvalidArgument;
     gemm::CommArgs& c = a.comm;
     c.rank = f->rank;
@@ -253,9 +394,9 @@ ucclResult_t launchGemmBf16(const GemmLaunch& g, const GemmFusion* f, cudaStream
     }
   }
 
-  const bool fusedOk = role == 0 || (f->rows_per_rank % (2 * gemm::BM) == 0);
+  const bool pairsFit = f->rows_per_rank % (2 * gemm::BM) == 0;
   cudaError_t e;
-  if (usePairKernel() && fusedOk) {
+  if (usePairKernel() && pairsFit) {
     // CTA pairs: 256-row tiles; both parts of the grid are even, and every cluster of the grid
     // must be resident at once because the GEMM CTAs of a fused launch wait for the
     // communication CTAs of the same launch
@@ -273,28 +414,18 @@ ucclResult_t launchGemmBf16(const GemmLaunch& g, const GemmFusion* f, cudaStream
     int pairs = std::max(1, std::min(maxPairs - comm_ctas / 2 - reducers / 2, tiles2));
     a.gemm_ctas = 2 * pairs;
     const int grid = a.gemm_ctas + comm_ctas + reducers;
-    if (g.epilogue == gemm::kEpiSwiGLU) {
-      if (role == gemm::kCommAllGather) e = launchPairT<gemm::kEpiSwiGLU, gemm::kCommAllGather>(tmA, tmB, pm, a, grid, stream);
-      else e = launchPairT<gemm::kEpiSwiGLU, gemm::kCommNone>(tmA, tmB, pm, a, grid, stream);
-    } else {
-      if (role == gemm::kCommAllGather) e = launchPairT<gemm::kEpiStore, gemm::kCommAllGather>(tmA, tmB, pm, a, grid, stream);
-      else if (role == gemm::kCommReduceScatter) e = launchPairT<gemm::kEpiStore, gemm::kCommReduceScatter>(tmA, tmB, pm, a, grid, stream);
-      else e = launchPairT<gemm::kEpiStore, gemm::kCommNone>(tmA, tmB, pm, a, grid, stream);
-    }
+    if (role == gemm::kCommReduceScatter) e = launchPairT<gemm::kEpiStore, gemm::kCommReduceScatter>(tmA, tmB, pm, a, grid, stream);
+    else if (g.epilogue == gemm::kEpiSwiGLU) e = launchPairT<gemm::kEpiSwiGLU, gemm::kCommAllGather>(tmA, tmB, pm, a, grid, stream);
+    else e = launchPairT<gemm::kEpiStore, gemm::kCommAllGather>(tmA, tmB, pm, a, grid, stream);
   } else {
     const int tiles = a.tiles_m * a.tiles_n;
     int reducers = 0;
     if (role == gemm::kCommReduceScatter && f->tail_next && f->rs_reducers > 0) reducers = std::min(f->rs_reducers, sms / 2);
     a.gemm_ctas = std::max(1, std::min(sms - comm_ctas - reducers, tiles));
     const int grid = a.gemm_ctas + comm_ctas + reducers;
-    if (g.epilogue == gemm::kEpiSwiGLU) {
-      if (role == gemm::kCommAllGather) e = launchT<gemm::kEpiSwiGLU, gemm::kCommAllGather>(tmA, tmB, pm, a, grid, stream);
-      else e = launchT<gemm::kEpiSwiGLU, gemm::kCommNone>(tmA, tmB, pm, a, grid, stream);
-    } else {
-      if (role == gemm::kCommAllGather) e = launchT<gemm::kEpiStore, gemm::kCommAllGather>(tmA, tmB, pm, a, grid, stream);
-      else if (role == gemm::kCommReduceScatter) e = launchT<gemm::kEpiStore, gemm::kCommReduceScatter>(tmA, tmB, pm, a, grid, stream);
-      else e = launchT<gemm::kEpiStore, gemm::kCommNone>(tmA, tmB, pm, a, grid, stream);
-    }
+    if (role == gemm::kCommReduceScatter) e = launchT<gemm::kEpiStore, gemm::kCommReduceScatter>(tmA, tmB, pm, a, grid, stream);
+    else if (g.epilogue == gemm::kEpiSwiGLU) e = launchT<gemm::kEpiSwiGLU, gemm::kCommAllGather>(tmA, tmB, pm, a, grid, stream);
+    else e = launchT<gemm::kEpiStore, gemm::kCommAllGather>(tmA, tmB, pm, a, grid, stream);
   }
   if (e != cudaSuccess) {
     UCCL_LOG(ERROR, "gemm launch failed: %s", cudaGetErrorString(e));

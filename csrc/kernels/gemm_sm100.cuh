@@ -1,6 +1,6 @@
 // Persistent warp-specialised bf16 GEMM for sm_100a: C[M,N] = A[M,K] * B[N,K]^T (both K-major,
-// i.e. the torch.nn.Linear layout), fp32 accumulation in TMEM, optionally fused with the
-// tensor-parallel collective next to it.
+// i.e. the torch.nn.Linear layout), fp32 accumulation in TMEM, fused with the tensor-parallel
+// collective next to it.  The GEMM without a collective is in gemm_plain.cuh.
 //
 //   warp 0      TMA producer : streams A and B tiles through a shared-memory ring, 128-byte swizzle
 //   warp 1      MMA issuer   : one elected lane of the converged warp issues tcgen05.mma, accumulators double-buffered in
@@ -85,7 +85,6 @@ enum Epilogue : int {
   kEpiSwiGLU = 1,  // B rows of a tile are [128 gate rows | 128 up rows]; C[M,N/2] = silu(g)*u
 };
 enum CommRole : int {
-  kCommNone = 0,
   kCommAllGather = 1,
   kCommReduceScatter = 2,    // epilogue TMA-stores tiles into the owners' staging slots
 };
@@ -154,7 +153,12 @@ struct Args {
   CommArgs comm;
 };
 
-__device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
+// x / (1 + exp(-x)).  A zero skips the division, whose result it is: the division has a slow path for zero
+// numerators, and the accumulator rows beyond a small M hold nothing else.
+__device__ __forceinline__ float silu_f(float x) {
+  const float q = (x == 0.f ? 1.f : x) / (1.0f + __expf(-x));
+  return x == 0.f ? x : q;
+}
 
 // Bounded wait until *flag >= target. Returns false on timeout / abort.
 // Relaxed polls with a growing pause, one system-scope fence on success.
@@ -957,7 +961,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           ptx::tma_load_2d(sB + B_STAGE_BYTES / 2, &tmB, &full_bar[s], kb * BK, brow1);
         }
       }
-    } else if (COMM != kCommNone && a.comm.go && cta_id == 0) {
+    } else if (a.comm.go && cta_id == 0) {
       prologue_barrier(a.comm, lane, a.err);  // the warp's idle lanes run the launch's rank barrier
     }
   } else if (warp == 1) {
@@ -1169,7 +1173,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           ptx::tma_load_2d_pair(sB, &tmB, fb, kb * BK, brow);
         }
       }
-    } else if (COMM != kCommNone && a.comm.go && cta_id == 0) {
+    } else if (a.comm.go && cta_id == 0) {
       prologue_barrier(a.comm, lane, a.err);  // the warp's idle lanes run the launch's rank barrier
     }
   } else if (warp == 1) {

@@ -45,3 +45,37 @@ def test_gemm_swiglu(M, N, K):
     err = (out - ref).abs().max().item()
     scale = ref.abs().max().item()
     assert err <= 2e-2 * scale + 1e-2, (err, scale)
+
+
+@gpu
+@pytest.mark.parametrize("M,N,K,epilogue", [
+    (1, 8, 12288, 0),       # one tile, K in eight parts
+    (9, 30, 4104, 0),       # columns that end inside 16, K that ends inside a stage
+    (64, 4096, 14336, 0),   # A rows of half a tile, four parts
+    (127, 6160, 264, 0),    # one stage less than a ring
+    (129, 512, 12288, 0),   # pairs in parts, second CTA with one row
+    (40, 62, 512, 1), (64, 7168, 4096, 1), (250, 1024, 8192, 1),  # the same with gate and up
+    (1000, 3592, 4104, 0), (4096, 7168, 1024, 1),  # tiles narrower than 256, more than one wave
+])
+def test_gemm_cuts(M, N, K, epilogue):
+    """Every cut of the work, in an output with a border that has to stay as it is, the same bits twice."""
+    from unified_ccl_b200.ops import gemm_bf16
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    b = (torch.randn(N, K, device="cuda", generator=g) * 0.02).to(torch.bfloat16)
+    n_out = N // 2 if epilogue else N
+    border = torch.full((M + 1, (n_out + 7) // 8 * 8 + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    out = border[:M, :n_out]
+    gemm_bf16(a, b, out=out, swiglu=bool(epilogue))
+    first = out.clone()
+    gemm_bf16(a, b, out=out, swiglu=bool(epilogue))
+    assert torch.equal(out, first)
+    assert (border[M] == 7).all() and (border[:M, n_out:] == 7).all()
+    ref = a.double() @ b.double().t()
+    if epilogue:
+        ref = torch.nn.functional.silu(ref[:, :n_out]) * ref[:, n_out:]
+    # one rounding to bf16 (2^-9 of the value), fp32 sums of K products of N(0, 1) x N(0, 0.02) numbers whose error
+    # is below K * 2^-24 of their sum of magnitudes (K * 0.013), in the SwiGLU carried by factors of a few
+    bound = ref.abs() * 2.0 ** -8 + K * 2.0 ** -24 * K * 0.013 * (8 if epilogue else 1) + 1e-6
+    assert ((out.double() - ref).abs() <= bound).all()
