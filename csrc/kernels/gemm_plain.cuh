@@ -235,6 +235,10 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   if (CG == 2) ptx::cluster_sync();  // both CTAs' barriers and TMEM exist before anybody signals the other
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  // Everything up to here may run while the launch before is still at work; no operand is read and C not
+  // touched before that one has ended.
+  ptx::launch_dependents();
+  ptx::wait_dependencies();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer

@@ -214,13 +214,15 @@ cudaError_t launchPlainT(const CUtensorMap& tmA, const CUtensorMap& tmB, const C
   cfg.blockDim = dim3(gemm::NUM_THREADS, 1, 1);
   cfg.dynamicSmemBytes = gemm::plain::SMEM;
   cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = csize;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = csize > 1 ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = csize;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = csize > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, args);
 }
 

@@ -188,6 +188,12 @@ __device__ __forceinline__ void multimem_red_add_u32(uint32_t* mc, uint32_t v) {
   asm volatile("multimem.red.release.sys.global.add.u32 [%0], %1;" ::"l"(mc), "r"(v) : "memory");
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// Lets the next launch of the stream (if it asks for it) come up once every CTA of this one is running.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Waits until the launch before has ended and its writes are visible.
+__device__ __forceinline__ void wait_dependencies() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

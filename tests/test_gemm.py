@@ -79,3 +79,49 @@ def test_gemm_cuts(M, N, K, epilogue):
     # is below K * 2^-24 of their sum of magnitudes (K * 0.013), in the SwiGLU carried by factors of a few
     bound = ref.abs() * 2.0 ** -8 + K * 2.0 ** -24 * K * 0.013 * (8 if epilogue else 1) + 1e-6
     assert ((out.double() - ref).abs() <= bound).all()
+
+
+@gpu
+@pytest.mark.parametrize("tokens", [5, 300])
+def test_gemm_chain_captured(tokens):
+    """Launches that come up early wait for the ones before: each operand and each output of a GEMM is written or read
+    by its neighbour in the stream, eagerly and in a graph."""
+    from unified_ccl_b200.ops import gemm_bf16
+
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn(tokens, 512, device="cuda", generator=g).to(torch.bfloat16)
+    w1 = (torch.randn(2048, 512, device="cuda", generator=g) * 0.04).to(torch.bfloat16)
+    w2 = (torch.randn(512, 1024, device="cuda", generator=g) * 0.04).to(torch.bfloat16)
+    h, y = torch.empty(tokens, 1024, device="cuda", dtype=torch.bfloat16), torch.empty(tokens, 512, device="cuda", dtype=torch.bfloat16)
+    w = torch.empty(64, 512, device="cuda", dtype=torch.bfloat16)
+    z = torch.empty(64, tokens + 7 & ~7, device="cuda", dtype=torch.bfloat16)[:, :tokens]
+
+    def chain(a):
+        for _ in range(8):
+            gemm_bf16(a, w1, out=h, swiglu=True)
+            gemm_bf16(h, w2, out=y)          # A is the last output
+            torch.mul(w1[:64], 0.5, out=w)
+            gemm_bf16(w, y, out=z)           # A comes from another kernel, B from the GEMM before that
+            a = y                            # and y is overwritten next while z has just read it
+        return y, z
+
+    def steps(a):
+        for _ in range(8):
+            for t, f in ((h, lambda: gemm_bf16(a, w1, out=h, swiglu=True)), (y, lambda: gemm_bf16(h, w2, out=y)),
+                         (w, lambda: torch.mul(w1[:64], 0.5, out=w)), (z, lambda: gemm_bf16(w, y, out=z))):
+                f()
+                torch.cuda.synchronize()
+            a = y
+        return y.clone(), z.clone()
+
+    want = steps(x)
+    assert all(torch.equal(a, b) for a, b in zip(want, chain(x)))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain(x)
+    for _ in range(3):
+        y.zero_(), z.zero_(), h.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(want[0], y) and torch.equal(want[1], z)
+    del graph
