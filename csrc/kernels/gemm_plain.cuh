@@ -12,6 +12,10 @@
 // A tile's stage of the ring holds 64 columns of K: the A rows and bn / CG rows of B.  With fewer than 128
 // rows in all the A part holds just these (a_rows); the tensor core then reads rows of B where the rest of A
 // would be, which only reaches accumulator rows that nobody looks at.
+//
+// Bound by memory when rows are few, by the tensor cores (and then the power cap) when they are many.  Against pair
+// tiles of 256 x 256 alone: 64 x 4096 x 14336 71 -> 25.8 us (4.6 TB/s), SwiGLU 64 x 28672 x 4096 81 -> 50 us (4.7
+// TB/s), 512 x 4096 x 4096 29 -> 19.5 us, 1000 x 3592 x 4104 33 -> 30 us, SwiGLU 4096 x 7168 x 4096 167 -> 162 us.
 #pragma once
 #include "gemm_sm100.cuh"
 

@@ -136,7 +136,9 @@ struct PlainPlan {
 // the tensor cores' time for a stage (two cycles per accumulator column, at least a round trip of the ring) and its
 // loads (78 bytes per cycle and SM), at least the time of memory, plus a tile's epilogue or the exchange of the
 // parts.  The constants are a fit to 102 shapes with every candidate measured (1 to 6000 rows, B of 0.1 to 240 MB):
-// the choice is within 2% of the best candidate on average.
+// the choice is within 2% of the best candidate on average.  Both sides of some of its lines, in us: 64 x 4096 x 14336
+// 25.7 in four parts of 128 columns, 62 uncut; 2048 x 4096 x 4096 48 in pair tiles of 256, 54 of 160 or of single CTAs;
+// 2048 x 7168 x 4096 (SwiGLU) 86 in pair tiles of 224, 92 of 256; 512 x 4096 x 4096 20 in tiles of 128, 25 of 256.
 PlainPlan choosePlain(int M, int N, int K, bool swiglu, int max_ctas) {
   PlainPlan best = {1, 256, 1};
 #ifdef UCCL_EXPERIMENTS
