@@ -225,7 +225,9 @@ cudaError_t launchPlainT(const CUtensorMap& tmA, const CUtensorMap& tmB, const C
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = csize > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, args);
+  e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, args);
+  (void)cudaGetLastError();  // a launch that was refused is reported here, not by the thread's next launch
+  return e;
 }
 
 ucclResult_t launchPlain(const GemmLaunch& g, cudaStream_t stream) {

@@ -125,3 +125,35 @@ def test_gemm_chain_captured(tokens):
         torch.cuda.synchronize()
         assert torch.equal(want[0], y) and torch.equal(want[1], z)
     del graph
+
+
+@gpu
+def test_gemm_refused_launch_is_reported_once():
+    """A launch that the driver refuses (its stream is in a capture that has been invalidated, an error of the host alone)
+    fails the GEMM, and nothing that the thread launches afterwards."""
+    import ctypes
+    import os
+
+    from unified_ccl_b200 import Communicator
+    from unified_ccl_b200.ops import gemm_bf16
+
+    os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    cu = ctypes.CDLL("libcuda.so.1")
+    comm = Communicator(0, 1)
+    a = torch.ones(64, 256, device="cuda", dtype=torch.bfloat16)
+    out = torch.empty(64, 64, device="cuda", dtype=torch.bfloat16)
+    v, w = torch.ones(1024, device="cuda"), torch.empty(1024, device="cuda")
+    gemm_bf16(a, a, out=out)
+    comm.reduce_scatter_cast(v, w, 2.0)  # both kernels are loaded now
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    stream, graph = ctypes.c_void_p(side.cuda_stream), ctypes.c_void_p()
+    assert cu.cuStreamBeginCapture_v2(stream, 2) == 0  # CU_STREAM_CAPTURE_MODE_RELAXED
+    assert cu.cuStreamQuery(stream) == 900             # CUDA_ERROR_STREAM_CAPTURE_UNSUPPORTED: ends the capture's validity
+    with torch.cuda.stream(side), pytest.raises(RuntimeError):
+        gemm_bf16(a, a, out=out)
+    assert cu.cuStreamEndCapture(stream, ctypes.byref(graph)) == 901  # CUDA_ERROR_STREAM_CAPTURE_INVALIDATED
+    comm.reduce_scatter_cast(v, w, 3.0)
+    torch.cuda.synchronize()
+    assert (w == 3.0).all()
+    comm.destroy()
