@@ -76,9 +76,7 @@ extern "C" ucclResult_t ucclReduceScatterEx(const void* sendbuff, void* recvbuff
   const size_t chunkBytes = recvcount * es;
   const size_t outEs = dataTypeSize(outType);
   commCount(c, ucclCollReduceScatter, chunkBytes * n, ucclAlgoTwoShot);
-  int blocks = c->cfg.maxCtas > 0 ? std::min(c->cfg.maxCtas, kMaxBlocks) : kMaxBlocks;
-  if (c->forcedBlocks > 0) blocks = std::min(c->forcedBlocks, kMaxBlocks);
-  blocks = static_cast<int>(std::max<size_t>(1, std::min<size_t>(blocks, (recvcount + 4095) / 4096)));
+  const int limit = c->forcedBlocks > 0 ? c->forcedBlocks : std::max(c->cfg.maxCtas, 0);  // 0: none asked for
 
   CastArgs a;
   memset(&a, 0, sizeof(a));
@@ -94,9 +92,11 @@ extern "C" ucclResult_t ucclReduceScatterEx(const void* sendbuff, void* recvbuff
     a.chunkElems = recvcount;
     a.out = static_cast<char*>(recvbuff);
     a.outScales = blockScales;
-    if (launchReduceCastKernel(a, blocks, s) != cudaSuccess) return ucclSystemError;
+    if (launchCastKernel(a, limit, s) != cudaSuccess) return ucclSystemError;
     return ucclSuccess;
   }
+  int blocks = limit > 0 ? std::min(limit, kMaxBlocks) : kMaxBlocks;
+  blocks = static_cast<int>(std::max<size_t>(1, std::min<size_t>(blocks, (recvcount + 4095) / 4096)));
   SymSegment* seg = c->heap.find(sendbuff, chunkBytes * n);
   if (seg) {
     const size_t off = static_cast<size_t>(static_cast<const char*>(sendbuff) - seg->local);

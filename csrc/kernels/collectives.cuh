@@ -66,6 +66,9 @@ struct CastArgs {
   float* outScales;                      // fp8 output: one scale per 128 elements
 };
 cudaError_t launchReduceCastKernel(const CastArgs& a, int blocks, cudaStream_t stream);
+// One rank (in[0], out, outScales, chunkElems, types and scale are read): as many CTAs as the data has, at most
+// `limit` unless it is 0.
+cudaError_t launchCastKernel(const CastArgs& a, int limit, cudaStream_t stream);
 
 // Ring all-reduce / all-gather / reduce-scatter over peer-memory step FIFOs (Simple protocol)
 // and the LL128 line protocol; see ring.cu.

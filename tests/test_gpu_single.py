@@ -68,6 +68,47 @@ def test_cast_single_rank(din, dout):
 
 
 @gpu
+@pytest.mark.parametrize("din,dout", [(torch.bfloat16, torch.float8_e4m3fn), (torch.float32, torch.bfloat16)])
+def test_cast_single_rank_keeps_to_its_ctas(din, dout):
+    """A limit on the CTAs of a communicator's kernels holds for one rank too, with one and with four pieces per thread, a
+    last round that is nearly empty, and the same bits as without a limit."""
+    import os
+
+    from torch.profiler import ProfilerActivity, profile
+
+    from unified_ccl_b200 import Communicator
+
+    os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    comm = Communicator(0, 1)
+    per_cta = 256 * 32 // torch.empty((), dtype=din).element_size()  # elements of a CTA's round, one piece per thread
+    for blocks in (1, 3):
+        for count in (128, per_cta * blocks + 128, 4 * per_cta * blocks, 4 * per_cta * blocks * 5 + 128):
+            x = torch.randn(count, device="cuda").to(din)
+            out, ref = (torch.zeros(count, device="cuda", dtype=dout) for _ in range(2))
+            comm.set_blocks(0)
+            ref_scales = comm.reduce_scatter_cast(x, ref, 0.37)[1]
+            comm.set_blocks(blocks)
+            torch.cuda.synchronize()
+            with profile(activities=[ProfilerActivity.CUDA]) as prof:
+                scales = comm.reduce_scatter_cast(x, out, 0.37)[1]
+                torch.cuda.synchronize()
+            grids = [e["args"]["grid"] for e in _kernel_events(prof) if "cast" in e["name"]]
+            assert len(grids) == 1 and grids[0][0] <= blocks and grids[0][1:] == [1, 1], (count, grids)
+            assert torch.equal(out.view(torch.uint8), ref.view(torch.uint8)), (blocks, count)
+            assert scales is None or torch.equal(scales, ref_scales), (blocks, count)
+    comm.destroy()
+
+
+def _kernel_events(prof):
+    import json
+    import tempfile
+
+    with tempfile.NamedTemporaryFile(suffix=".json") as f:
+        prof.export_chrome_trace(f.name)
+        return [e for e in json.load(open(f.name))["traceEvents"] if e.get("cat") == "kernel"]
+
+
+@gpu
 @pytest.mark.parametrize("tokens,hidden", [(1, 8), (700, 24), (297, 512), (700, 1032), (300, 8192), (5, 8200), (300, 16376), (300, 16384)])
 def test_norm_single_rank_shapes(tokens, hidden):
     """Pieces of 16 and 32 bytes, one to four per thread, several rows per CTA and one; residual in place."""
