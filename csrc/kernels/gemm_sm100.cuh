@@ -153,10 +153,15 @@ struct Args {
   CommArgs comm;
 };
 
-// x / (1 + exp(-x)).  A zero skips the division, whose result it is: the division has a slow path for zero
-// numerators, and the accumulator rows beyond a small M hold nothing else.
+// x / (1 + exp(-x)).  The division has a slow path for zero numerators, which a whole warp walks through for one lane,
+// and the accumulator rows of a tile that lie beyond M hold nothing else: a zero, whose result is itself, divides 1
+// instead.  The compiler would see that this quotient is not used and divide x after all; the empty asm keeps it
+// from looking.  1212 x 10192 x 1760 (a last tile of 188 rows) in tiles of
+// 256 x 256: 57.5 us with the division by x, 42.5 now, 42.7 with 1280 rows.
 __device__ __forceinline__ float silu_f(float x) {
-  const float q = (x == 0.f ? 1.f : x) / (1.0f + __expf(-x));
+  float n = x == 0.f ? 1.f : x;
+  asm("" : "+f"(n));
+  const float q = n / (1.0f + __expf(-x));
   return x == 0.f ? x : q;
 }
 
