@@ -132,13 +132,21 @@ struct PlainPlan {
   int cg, bn, split;
 };
 
-// How to cut a GEMM without a collective.  Cycles of a candidate: waves of tiles x stages per tile x the longer of
-// the tensor cores' time for a stage (two cycles per accumulator column, at least a round trip of the ring) and its
-// loads (78 bytes per cycle and SM), at least the time of memory, plus a tile's epilogue or the exchange of the
-// parts.  The constants are a fit to 102 shapes with every candidate measured (1 to 6000 rows, B of 0.1 to 240 MB):
-// the choice is within 2% of the best candidate on average.  Both sides of some of its lines, in us: 64 x 4096 x 14336
-// 25.7 in four parts of 128 columns, 62 uncut; 2048 x 4096 x 4096 48 in pair tiles of 256, 54 of 160 or of single CTAs;
-// 2048 x 7168 x 4096 (SwiGLU) 86 in pair tiles of 224, 92 of 256; 512 x 4096 x 4096 20 in tiles of 128, 25 of 256.
+// How to cut a GEMM without a collective: the candidate with the fewest cycles by one of two formulas.
+//
+// A tile whole: waves of tiles x the longer of a tile's main loop and of the epilogue that runs beside the next tile's
+// (2150 cycles, and per output column 11, or 49 with silu and its division); at least the time of memory, and
+// at least that of all loads together (9000 bytes per cycle into all SMs).  A stage of the main loop takes what the tensor
+// cores need for it (two cycles per accumulator column, at least a round trip of the ring) or its loads (65 bytes
+// per cycle and SM).  A tile in parts of K: the same without the overlapped epilogue (one tile per cluster), plus
+// the exchange of the parts.
+//
+// The constants are fits to measurements with every candidate timed on operands that are not in L2: whole tiles to
+// 658 shapes (1 to 16384 rows, K of 64 to 14336), where the choice takes 1.2% more than the best candidate on average (an
+// earlier formula without the epilogue and the common load rate: 2.4%, and 20% on 4096 x 28672 x 512), the parts to 102
+// of them.  Both sides of some of the lines, in us: 64 x 4096 x 14336 25.3 in four parts of 128 columns, 62 uncut;
+// 4096 x 28672 x 512 111 in pair tiles of 256, 125 of 224; 8192 x 3592 x 4104 207 in pair tiles of 256, 244 of 192;
+// 200 x 28672 x 4096 51.6 in pair tiles of 224, 60.2 in single CTAs of 208; 512 x 4096 x 4096 20 in tiles of 128, 25 of 256.
 PlainPlan choosePlain(int M, int N, int K, bool swiglu, int max_ctas) {
   PlainPlan best = {1, 256, 1};
 #ifdef UCCL_EXPERIMENTS
@@ -165,11 +173,19 @@ PlainPlan choosePlain(int M, int N, int K, bool swiglu, int max_ctas) {
         const int tiles = tiles_m * ((out_n + out_bn - 1) / out_bn);
         if (split > 1 && tiles > resident) continue;
         const int waves = (tiles + resident - 1) / resident;
-        const double stage = std::max(std::max(2.0 * bn, 329.0) + 54.0, (a_rows + bn / cg) * 128.0 / 78.0);
-        const double memory = bytes / std::min(3500.0, std::min(tiles, resident) * cg * split * 83.0);
-        double t = std::max(memory, waves * kbs * stage) + waves * 34.0;
-        if (split == 1) t += 8.0 * bn;
-        else t += 3100.0 + 280.0 * split + 30.0 * bn * std::min(M, cg * gemm::BM) / (cg * gemm::BM);
+        const int ctas = std::min(tiles, resident) * cg * split;
+        const double mma = std::max(2.0 * bn, 329.0) + 54.0, stage_bytes = (a_rows + bn / cg) * 128.0;
+        double t;
+        if (split == 1) {
+          const double stage = std::max(mma, stage_bytes / 65.0), epilogue = 2150.0 + (swiglu ? 49.0 : 11.0) * out_bn;
+          const double memory = bytes / std::min(6100.0, ctas * 41.0);
+          const double loads = static_cast<double>(tiles) * cg * num_kb * stage_bytes / 9000.0;
+          t = std::max(std::max(memory, loads), waves * std::max(num_kb * stage + 34.0, epilogue)) + 0.1 * epilogue;
+        } else {
+          const double stage = std::max(mma, stage_bytes / 78.0);
+          const double memory = bytes / std::min(3500.0, ctas * 83.0);
+          t = std::max(memory, waves * kbs * stage) + waves * 34.0 + 3100.0 + 280.0 * split + 30.0 * bn * std::min(M, cg * gemm::BM) / (cg * gemm::BM);
+        }
         if (t < best_t) {
           best_t = t;
           best = {cg, bn, split};
