@@ -242,7 +242,7 @@ cudaError_t launchPlainT(const CUtensorMap& tmA, const CUtensorMap& tmB, const C
   cfg.attrs = attr;
   cfg.numAttrs = csize > 1 ? 2 : 1;
   e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, args);
-  (void)cudaGetLastError();  // a launch that was refused is reported here, not by the thread's next launch
+  if (e != cudaSuccess) (void)cudaGetLastError();  // a launch that was refused is reported here, not by the thread's next launch
   return e;
 }
 
