@@ -147,7 +147,7 @@ extern "C" ucclResult_t ucclAllReduceResidualRMSNorm(const void* x, const void* 
     a.dc.nranks = 1;
     a.inUser = static_cast<const char*>(x);
     a.resOutUser = static_cast<char*>(residualOut);
-    if (launchArNormKernel(a, 1, s) != cudaSuccess) {
+    if (launchArNormKernel(a, 0, s) != cudaSuccess) {
       commSetError(c, "norm kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
       return ucclSystemError;
     }

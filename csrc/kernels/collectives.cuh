@@ -128,6 +128,7 @@ struct ArNormArgs {
   int mcRows;  // switch path: rows per pass of the all-reduce phase (1, 2 or 4), own rows normalised in phase B; 0 = from registers, one row per pass
   int debug;  // experiment switches (UCCL_NORM_DEBUG): 1 no phase B, 2 no phase-A stores, 4 no phase A
 };
+// `blocks`: CTAs of a launch among ranks; on one rank the data decides and it is not read.
 cudaError_t launchArNormKernel(const ArNormArgs& a, int blocks, cudaStream_t stream);
 
 }  // namespace uccl

@@ -382,7 +382,7 @@ static cudaError_t launchNormLocal(const dev::NormLocalArgs& l, cudaStream_t s) 
   const unsigned grid = static_cast<unsigned>((static_cast<long>(l.tokens) + rows - 1) / rows);
   if (nv == 1) dev::add_norm_kernel<1, W><<<grid, lanes * rows, 0, s>>>(l, lanes);
   else if (nv == 2) dev::add_norm_kernel<2, W><<<grid, lanes * rows, 0, s>>>(l, lanes);
-  else dev::add_norm_kernel<4, W><<<grid, lanes * rows, 0, s>>>(l, lanes);
+  else if constexpr (W == 16) dev::add_norm_kernel<4, W><<<grid, lanes * rows, 0, s>>>(l, lanes);  // 32-byte pieces: two at most
   return cudaGetLastError();
 }
 

@@ -147,7 +147,7 @@ struct PlainPlan {
 // of them.  Both sides of some of the lines, in us: 64 x 4096 x 14336 25.3 in four parts of 128 columns, 62 uncut;
 // 4096 x 28672 x 512 111 in pair tiles of 256, 125 of 224; 8192 x 3592 x 4104 207 in pair tiles of 256, 244 of 192;
 // 200 x 28672 x 4096 51.6 in pair tiles of 224, 60.2 in single CTAs of 208; 512 x 4096 x 4096 20 in tiles of 128, 25 of 256.
-PlainPlan choosePlain(int M, int N, int K, bool swiglu, int max_ctas) {
+PlainPlan choosePlain(int M, int N, int K, bool swiglu) {
   PlainPlan best = {1, 256, 1};
 #ifdef UCCL_EXPERIMENTS
   if (const char* e = getenv("UCCL_GEMM_PLAN")) {
@@ -164,8 +164,7 @@ PlainPlan choosePlain(int M, int N, int K, bool swiglu, int max_ctas) {
     const int a_rows = cg == 1 && M < gemm::BM ? (M + 7) / 8 * 8 : gemm::BM;
     const int step = cg == 2 || swiglu ? 32 : 16;
     for (int split = 1; split * cg <= gemm::plain::MAX_CLUSTER && split <= num_kb; split *= 2) {
-      int resident = cg == 2 ? residentClusters<2>(2 * split) : residentClusters<1>(split);
-      if (max_ctas > 0) resident = std::max(1, std::min(resident, max_ctas / (cg * split)));
+      const int resident = cg == 2 ? residentClusters<2>(2 * split) : residentClusters<1>(split);
       const int kbs = (num_kb + split - 1) / split;
       for (int bn = step; bn <= gemm::BN; bn += step) {
         const int out_bn = swiglu ? bn / 2 : bn;
@@ -197,9 +196,9 @@ PlainPlan choosePlain(int M, int N, int K, bool swiglu, int max_ctas) {
 }
 
 // The choice is a function of the shape alone: each thread keeps a few.
-PlainPlan planFor(int M, int N, int K, bool swiglu, int max_ctas) {
+PlainPlan planFor(int M, int N, int K, bool swiglu) {
 #ifdef UCCL_EXPERIMENTS
-  return choosePlain(M, N, K, swiglu, max_ctas);
+  return choosePlain(M, N, K, swiglu);
 #endif
   struct Entry {
     int M, N, K, flags, dev;
@@ -208,11 +207,11 @@ PlainPlan planFor(int M, int N, int K, bool swiglu, int max_ctas) {
   static thread_local Entry table[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  const int flags = (swiglu ? 1 : 0) | (usePairKernel() ? 2 : 0) | (max_ctas << 2);
+  const int flags = (swiglu ? 1 : 0) | (usePairKernel() ? 2 : 0);
   const uint32_t h = static_cast<uint32_t>(M) * 2654435761u ^ static_cast<uint32_t>(N) * 2246822519u ^ static_cast<uint32_t>(K) * 3266489917u;
   Entry& e = table[(h >> 20) & 63];
   if (e.M != M || e.N != N || e.K != K || e.flags != flags || e.dev != dev) {
-    e.plan = choosePlain(M, N, K, swiglu, max_ctas);
+    e.plan = choosePlain(M, N, K, swiglu);
     e.M = M, e.N = N, e.K = K, e.flags = flags, e.dev = dev;
   }
   return e.plan;
@@ -249,7 +248,7 @@ cudaError_t launchPlainT(const CUtensorMap& tmA, const CUtensorMap& tmB, const C
 ucclResult_t launchPlain(const GemmLaunch& g, cudaStream_t stream) {
   const bool swiglu = g.epilogue == gemm::kEpiSwiGLU;
   const int out_n = swiglu ? g.N / 2 : g.N;
-  const PlainPlan p = planFor(g.M, g.N, g.K, swiglu, g.max_ctas);
+  const PlainPlan p = planFor(g.M, g.N, g.K, swiglu);
   gemm::plain::Args a = {};
   a.C = static_cast<__nv_bfloat16*>(g.C);
   a.ldc = g.ldc;
@@ -271,8 +270,7 @@ ucclResult_t launchPlain(const GemmLaunch& g, cudaStream_t stream) {
   const int ldc = g.M == 1 ? (out_n + 7) / 8 * 8 : g.ldc;
   const bool mapped = ldc >= out_n;
   a.tma_bn = mapped ? a.out_bn : 0;
-  int resident = p.cg == 2 ? maxResidentPairs() : deviceSmCount();
-  if (g.max_ctas > 0) resident = std::max(1, std::min(resident, g.max_ctas / p.cg));
+  const int resident = p.cg == 2 ? maxResidentPairs() : deviceSmCount();
   a.workers = p.split > 1 ? a.num_tiles : std::min(a.num_tiles, resident);
   CUtensorMap tmA, tmB, tmC = {};
   if (!makeTensorMap(&tmA, g.A, g.M, g.K, g.lda, gemm::BK, a.a_rows) || !makeTensorMap(&tmB, g.B, g.N, g.K, g.ldb, gemm::BK, swiglu || p.cg == 2 ? p.bn / 2 : p.bn) ||
@@ -337,7 +335,7 @@ ucclResult_t launchGemmBf16(const GemmLaunch& g, const GemmFusion* f, cudaStream
     cudaMemsetAsync(timesDev, 0, 48 * sizeof(unsigned long long), stream);
     a.times = timesDev;
   }
-  const int sms = g.max_ctas > 0 ? g.max_ctas : deviceSmCount();
+  const int sms = deviceSmCount();
   gemm::PeerMaps pm = {};
   int comm_ctas = 0;
   {
@@ -426,8 +424,7 @@ ucclResult_t launchGemmBf16(const GemmLaunch& g, const GemmFusion* f, cudaStream
     const int tiles2 = tiles_m2 * a.tiles_n;
     if (comm_ctas & 1) ++comm_ctas;
     a.comm_ctas = comm_ctas;
-    int maxPairs = maxResidentPairs();
-    if (g.max_ctas > 0) maxPairs = std::min(maxPairs, g.max_ctas / 2);
+    const int maxPairs = maxResidentPairs();
     // reducer CTAs (reduce-scatter only, and only with the shared work counter) come out of the
     // resident budget: they must run from the start, next to the GEMM CTAs
     int reducers = 0;

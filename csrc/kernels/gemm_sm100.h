@@ -16,7 +16,6 @@ struct GemmLaunch {
   int M = 0, N = 0, K = 0;
   int lda = 0, ldb = 0, ldc = 0;
   int epilogue = 0;         // 0 store, 1 SwiGLU
-  int max_ctas = 0;         // 0 = one per SM
   uint32_t* err = nullptr;  // optional device-visible error word
 };
 
