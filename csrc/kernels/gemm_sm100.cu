@@ -7,6 +7,7 @@
 #include <strings.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "../core/cuda_driver.h"
 #include "../core/log.h"
@@ -17,15 +18,15 @@
 namespace uccl {
 
 int deviceSmCount() {
-  static int cached[64];
+  static std::atomic<int> cached[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (cached[dev] == 0) {
-    int n = 0;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    cached[dev] = n > 0 ? n : 148;
+    cached[dev].store(n = n > 0 ? n : 148, std::memory_order_relaxed);
   }
-  return cached[dev];
+  return n;
 }
 
 namespace {
@@ -93,11 +94,12 @@ cudaError_t launchPairT(const CUtensorMap& tmA, const CUtensorMap& tmB, const ge
 // stays unused).
 template <int CG>
 int residentClusters(int csize) {
-  static int cached[64][gemm::plain::MAX_CLUSTER + 1];
+  static std::atomic<int> cached[64][gemm::plain::MAX_CLUSTER + 1];  // the same from every thread
   int dev = 0;
   cudaGetDevice(&dev);
   const bool keep = dev >= 0 && dev < 64;
-  if (keep && cached[dev][csize] != 0) return cached[dev][csize];
+  int n = keep ? cached[dev][csize].load(std::memory_order_relaxed) : 0;
+  if (n != 0) return n;
   auto kern = gemm::plain::gemm_plain_kernel<gemm::kEpiStore, CG>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm::plain::SMEM);
   cudaLaunchConfig_t cfg = {};
@@ -111,12 +113,11 @@ int residentClusters(int csize) {
   attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
     (void)cudaGetLastError();
     n = std::max(1, deviceSmCount() / csize - 4);
   }
-  if (keep) cached[dev][csize] = n;
+  if (keep) cached[dev][csize].store(n, std::memory_order_relaxed);
   UCCL_LOG(INFO, "gemm: %d clusters of %d CTAs can be resident on device %d", n, csize, dev);
   return n;
 }
