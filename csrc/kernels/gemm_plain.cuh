@@ -36,6 +36,7 @@ struct Args {
   int tiles_n;
   int bn, out_bn;        // accumulator columns and output columns of a tile
   int tma_bn;            // out_bn, or 0 if no tensor map describes C
+  int tma_n;             // a TMA store may start at columns below this one
   int b_half_rows;       // SwiGLU: row offset of the "up" half inside B
   int a_rows;            // rows of A in a stage (128, or fewer when M is)
   int stages, stage_bytes;
@@ -81,13 +82,15 @@ __device__ __forceinline__ void store16(const Args& a, int row, int col, const u
 
 // The whole tile of one warp (32 rows from row0): 64 output columns at a time through shared memory and TMA
 // stores, which clip what lies outside C; the columns that are left in units of 16 straight from registers.
+// A TMA store writes whole pieces of 16 bytes: where C ends inside of one, it would overwrite what the caller keeps
+// behind the row's end, so the last columns of such a C take the second way (tma_n).
 template <int EPI>
 __device__ __forceinline__ void store_tile(const Args& a, const CUtensorMap* tmC, uint32_t taddr, int row0, int col0, int lane,
                                            uint8_t* stage, uint32_t& stage_it) {
   if (row0 >= a.M) return;
   int c = 0;
 #pragma unroll 1
-  for (; c + 64 <= a.tma_bn && col0 + c < a.out_n; c += 64) {
+  for (; c + 64 <= a.tma_bn && col0 + c < a.tma_n; c += 64) {
     uint4 v[8];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {

@@ -271,6 +271,7 @@ ucclResult_t launchPlain(const GemmLaunch& g, cudaStream_t stream) {
   const int ldc = g.M == 1 ? (out_n + 7) / 8 * 8 : g.ldc;
   const bool mapped = ldc >= out_n;
   a.tma_bn = mapped ? a.out_bn : 0;
+  a.tma_n = out_n % 8 == 0 ? out_n : out_n - 63;
   const int resident = p.cg == 2 ? maxResidentPairs() : deviceSmCount();
   a.workers = p.split > 1 ? a.num_tiles : std::min(a.num_tiles, resident);
   CUtensorMap tmA, tmB, tmC = {};

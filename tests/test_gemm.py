@@ -56,6 +56,7 @@ def test_gemm_swiglu(M, N, K):
     (129, 512, 12288, 0),   # pairs in parts, second CTA with one row
     (40, 62, 512, 1), (64, 7168, 4096, 1), (250, 1024, 8192, 1),  # the same with gate and up
     (1000, 3592, 4104, 0), (4096, 7168, 1024, 1),  # tiles narrower than 256, more than one wave
+    (2048, 4093, 1024, 0), (2048, 8186, 1024, 1), (2048, 4033, 256, 0),  # wide tiles, rows that end inside a piece of 16 bytes
 ])
 def test_gemm_cuts(M, N, K, epilogue):
     """Every cut of the work, in an output with a border that has to stay as it is, the same bits twice."""
