@@ -31,6 +31,21 @@ int deviceSmCount() {
 
 namespace {
 
+// Columns of B rows in a tile come in steps: of what cta_group::2 takes, or of 16 gate and 16 up rows, or of 16.
+int cutStep(int cg, bool swiglu) { return cg == 2 || swiglu ? 32 : 16; }
+
+}  // namespace
+
+bool gemmCutRuns(const GemmCut& c, int K, bool swiglu) {
+  if (c.cg != 1 && c.cg != 2) return false;
+  if (c.bn < 16 || c.bn > gemm::BN || c.bn % cutStep(c.cg, swiglu) != 0) return false;
+  if (c.split < 1 || c.cg * c.split > gemm::plain::MAX_CLUSTER || c.split > (K + gemm::BK - 1) / gemm::BK) return false;
+  // every part ends up with whole steps of 16 output columns
+  return c.split == 1 || (swiglu ? c.bn / 2 : c.bn) % (16 * c.split) == 0;
+}
+
+namespace {
+
 // bf16 matrix [rows, cols] (row stride ld elements), 128-byte swizzled boxes of box_cols x box_rows.
 bool makeTensorMap(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_cols,
                    uint32_t box_rows) {
@@ -129,10 +144,6 @@ bool usePairKernel() {
   return (s && *s) ? atoi(s) != 0 : true;
 }
 
-struct PlainPlan {
-  int cg, bn, split;
-};
-
 // How to cut a GEMM without a collective: the candidate with the fewest cycles by one of two formulas.
 //
 // A tile whole: waves of tiles x the longer of a tile's main loop and of the epilogue that runs beside the next tile's
@@ -148,13 +159,8 @@ struct PlainPlan {
 // of them.  Both sides of some of the lines, in us: 64 x 4096 x 14336 25.3 in four parts of 128 columns, 62 uncut;
 // 4096 x 28672 x 512 111 in pair tiles of 256, 125 of 224; 8192 x 3592 x 4104 207 in pair tiles of 256, 244 of 192;
 // 200 x 28672 x 4096 51.6 in pair tiles of 224, 60.2 in single CTAs of 208; 512 x 4096 x 4096 20 in tiles of 128, 25 of 256.
-PlainPlan choosePlain(int M, int N, int K, bool swiglu) {
-  PlainPlan best = {1, 256, 1};
-#ifdef UCCL_EXPERIMENTS
-  if (const char* e = getenv("UCCL_GEMM_PLAN")) {
-    if (sscanf(e, "%d,%d,%d", &best.cg, &best.bn, &best.split) == 3) return best;
-  }
-#endif
+GemmCut choosePlain(int M, int N, int K, bool swiglu) {
+  GemmCut best = {1, 256, 1};
   const bool pairs = usePairKernel();
   const int num_kb = (K + gemm::BK - 1) / gemm::BK;
   const int out_n = swiglu ? N / 2 : N;
@@ -163,13 +169,13 @@ PlainPlan choosePlain(int M, int N, int K, bool swiglu) {
   for (int cg = 1; cg <= (pairs ? 2 : 1); ++cg) {
     const int tiles_m = (M + cg * gemm::BM - 1) / (cg * gemm::BM);
     const int a_rows = cg == 1 && M < gemm::BM ? (M + 7) / 8 * 8 : gemm::BM;
-    const int step = cg == 2 || swiglu ? 32 : 16;
+    const int step = cutStep(cg, swiglu);
     for (int split = 1; split * cg <= gemm::plain::MAX_CLUSTER && split <= num_kb; split *= 2) {
       const int resident = cg == 2 ? residentClusters<2>(2 * split) : residentClusters<1>(split);
       const int kbs = (num_kb + split - 1) / split;
       for (int bn = step; bn <= gemm::BN; bn += step) {
         const int out_bn = swiglu ? bn / 2 : bn;
-        if (split > 1 && out_bn % (16 * split) != 0) continue;
+        if (!gemmCutRuns({cg, bn, split}, K, swiglu)) continue;
         const int tiles = tiles_m * ((out_n + out_bn - 1) / out_bn);
         if (split > 1 && tiles > resident) continue;
         const int waves = (tiles + resident - 1) / resident;
@@ -197,13 +203,10 @@ PlainPlan choosePlain(int M, int N, int K, bool swiglu) {
 }
 
 // The choice is a function of the shape alone: each thread keeps a few.
-PlainPlan planFor(int M, int N, int K, bool swiglu) {
-#ifdef UCCL_EXPERIMENTS
-  return choosePlain(M, N, K, swiglu);
-#endif
+GemmCut cutFor(int M, int N, int K, bool swiglu) {
   struct Entry {
     int M, N, K, flags, dev;
-    PlainPlan plan;
+    GemmCut cut;
   };
   static thread_local Entry table[64] = {};
   int dev = 0;
@@ -212,10 +215,10 @@ PlainPlan planFor(int M, int N, int K, bool swiglu) {
   const uint32_t h = static_cast<uint32_t>(M) * 2654435761u ^ static_cast<uint32_t>(N) * 2246822519u ^ static_cast<uint32_t>(K) * 3266489917u;
   Entry& e = table[(h >> 20) & 63];
   if (e.M != M || e.N != N || e.K != K || e.flags != flags || e.dev != dev) {
-    e.plan = choosePlain(M, N, K, swiglu);
+    e.cut = choosePlain(M, N, K, swiglu);
     e.M = M, e.N = N, e.K = K, e.flags = flags, e.dev = dev;
   }
-  return e.plan;
+  return e.cut;
 }
 
 template <int EPI, int CG>
@@ -246,10 +249,11 @@ cudaError_t launchPlainT(const CUtensorMap& tmA, const CUtensorMap& tmB, const C
   return e;
 }
 
-ucclResult_t launchPlain(const GemmLaunch& g, cudaStream_t stream) {
+ucclResult_t launchPlain(const GemmLaunch& g, const GemmCut* cut, cudaStream_t stream) {
   const bool swiglu = g.epilogue == gemm::kEpiSwiGLU;
   const int out_n = swiglu ? g.N / 2 : g.N;
-  const PlainPlan p = planFor(g.M, g.N, g.K, swiglu);
+  if (cut && !gemmCutRuns(*cut, g.K, swiglu)) return ucclInvalidArgument;
+  const GemmCut p = cut ? *cut : cutFor(g.M, g.N, g.K, swiglu);
   gemm::plain::Args a = {};
   a.C = static_cast<__nv_bfloat16*>(g.C);
   a.ldc = g.ldc;
@@ -290,7 +294,9 @@ ucclResult_t launchPlain(const GemmLaunch& g, cudaStream_t stream) {
 
 }  // namespace
 
-ucclResult_t launchGemmBf16(const GemmLaunch& g, const GemmFusion* f, cudaStream_t stream) {
+GemmCut chooseGemmCut(int M, int N, int K, bool swiglu) { return cutFor(M, N, K, swiglu); }
+
+ucclResult_t launchGemmBf16(const GemmLaunch& g, const GemmFusion* f, cudaStream_t stream, const GemmCut* cut) {
   if (!g.A || !g.B || !g.C || g.M <= 0 || g.N <= 0 || g.K <= 0) return ucclInvalidArgument;
   if (g.K % 8 != 0 || g.lda % 8 != 0 || g.ldb % 8 != 0 || g.ldc % 8 != 0) return ucclInvalidArgument;
   if ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B) | reinterpret_cast<uintptr_t>(g.C)) & 15)
@@ -299,7 +305,7 @@ ucclResult_t launchGemmBf16(const GemmLaunch& g, const GemmFusion* f, cudaStream
   const int role = f ? f->role : 0;
   if (role == gemm::kCommReduceScatter && g.epilogue != gemm::kEpiStore)
     return ucclInvalidArgument;
-  if (role == 0) return launchPlain(g, stream);
+  if (role == 0) return launchPlain(g, cut, stream);
 
   CUtensorMap tmA, tmB;
   if (!makeTensorMap(&tmA, g.A, g.M, g.K, g.lda, gemm::BK, gemm::BM)) return ucclSystemError;

@@ -53,8 +53,16 @@ struct GemmFusion {
   uint32_t* tail_next = nullptr;
 };
 
-ucclResult_t launchGemmBf16(const GemmLaunch& g, const GemmFusion* fusion, cudaStream_t stream);
+// How a GEMM without a collective is cut (see gemm_plain.cuh): CTAs per tile, rows of B per tile, parts of K.
+struct GemmCut {
+  int cg, bn, split;
+};
+// The cut that the current device takes for a shape, and whether the kernel can run a cut on it.
+GemmCut chooseGemmCut(int M, int N, int K, bool swiglu);
+bool gemmCutRuns(const GemmCut& cut, int K, bool swiglu);
 
+// `cut`: of a launch without fusion, in place of the chosen one.
+ucclResult_t launchGemmBf16(const GemmLaunch& g, const GemmFusion* fusion, cudaStream_t stream, const GemmCut* cut = nullptr);
 
 // Number of SMs of the current device (cached per device).
 int deviceSmCount();

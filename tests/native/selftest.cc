@@ -19,6 +19,7 @@
 
 #include "host/host_coll.h"
 #include "host/ring_schedule.h"
+#include "kernels/gemm_sm100.h"
 #include "protocols/protocol.h"
 #include "transport/net_plugin.h"
 #include "core/bootstrap.h"
@@ -810,4 +811,21 @@ extern "C" int ucclSelfTestRun(const char* name, char* report, size_t reportLen)
   }
   if (report && reportLen) snprintf(report, reportLen, "no such self test: %s", name);
   return 2;
+}
+
+// The cut of a GEMM, read and set (tests/test_gemm.py).
+extern "C" void ucclTestGemmCut(int M, int N, int K, int swiglu, int* cut) {
+  const uccl::GemmCut c = uccl::chooseGemmCut(M, N, K, swiglu != 0);
+  cut[0] = c.cg, cut[1] = c.bn, cut[2] = c.split;
+}
+extern "C" int ucclTestGemmCutRuns(const int* cut, int K, int swiglu) { return uccl::gemmCutRuns({cut[0], cut[1], cut[2]}, K, swiglu != 0); }
+extern "C" int ucclTestGemmInCut(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int swiglu,
+                                 const int* cut, void* stream) {
+  uccl::GemmLaunch g;
+  g.A = A, g.B = B, g.C = C;
+  g.M = M, g.N = N, g.K = K;
+  g.lda = lda, g.ldb = ldb, g.ldc = ldc;
+  g.epilogue = swiglu;
+  const uccl::GemmCut c = {cut[0], cut[1], cut[2]};
+  return uccl::launchGemmBf16(g, nullptr, static_cast<cudaStream_t>(stream), &c);
 }

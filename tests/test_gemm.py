@@ -49,17 +49,17 @@ def test_gemm_swiglu(M, N, K):
 
 @gpu
 @pytest.mark.parametrize("M,N,K,epilogue", [
-    (1, 8, 12288, 0),       # one tile, K in eight parts
+    (1, 8, 12288, 0),       # one row, a long K
     (9, 30, 4104, 0),       # columns that end inside 16, K that ends inside a stage
-    (64, 4096, 14336, 0),   # A rows of half a tile, four parts
-    (127, 6160, 264, 0),    # one stage less than a ring
-    (129, 512, 12288, 0),   # pairs in parts, second CTA with one row
+    (64, 4096, 14336, 0),   # A rows of half a tile
+    (127, 6160, 264, 0),    # few stages
+    (129, 512, 12288, 0),   # a second row tile with one row
     (40, 62, 512, 1), (64, 7168, 4096, 1), (250, 1024, 8192, 1),  # the same with gate and up
-    (1000, 3592, 4104, 0), (4096, 7168, 1024, 1),  # tiles narrower than 256, more than one wave
+    (1000, 3592, 4104, 0), (4096, 7168, 1024, 1),  # many tiles
     (2048, 4093, 1024, 0), (2048, 8186, 1024, 1), (2048, 4033, 256, 0),  # wide tiles, rows that end inside a piece of 16 bytes
 ])
 def test_gemm_cuts(M, N, K, epilogue):
-    """Every cut of the work, in an output with a border that has to stay as it is, the same bits twice."""
+    """The cuts that the library chooses, in an output with a border that has to stay as it is, the same bits twice."""
     from unified_ccl_b200.ops import gemm_bf16
 
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
@@ -80,6 +80,80 @@ def test_gemm_cuts(M, N, K, epilogue):
     # is below K * 2^-24 of their sum of magnitudes (K * 0.013), in the SwiGLU carried by factors of a few
     bound = ref.abs() * 2.0 ** -8 + K * 2.0 ** -24 * K * 0.013 * (8 if epilogue else 1) + 1e-6
     assert ((out.double() - ref).abs() <= bound).all()
+
+
+def _cut_lib():
+    import ctypes
+    import os
+
+    return ctypes.CDLL(os.path.join(os.path.dirname(os.path.abspath(__file__)), "native", "libuccl_selftest.so"))
+
+
+@gpu
+@pytest.mark.parametrize("M,N,K,epilogue,cut", [
+    (1, 8, 512, 0, (1, 128, 8)),                                  # eight parts of one stage each
+    (129, 512, 12288, 0, (2, 64, 2)), (129, 512, 12288, 0, (2, 128, 4)),  # pairs in parts, second CTA with one row
+    (255, 1030, 1096, 1, (2, 128, 2)), (200, 100, 4096, 0, (1, 64, 4)), (300, 500, 1032, 1, (1, 256, 8)),
+    (300, 192, 440, 0, (1, 64, 1)), (300, 192, 512, 0, (1, 64, 1)), (300, 192, 520, 0, (1, 64, 1)),  # 7, 8 and 9 stages in a ring of 8
+    (600, 512, 320, 0, (2, 256, 1)), (600, 512, 384, 0, (2, 256, 1)), (600, 512, 392, 0, (2, 256, 1)),  # 5, 6 and 7 in a ring of 6
+    (8, 48, 1480, 0, (1, 16, 1)), (8, 48, 1536, 0, (1, 16, 1)), (8, 48, 1544, 0, (1, 16, 1)),  # 24, 24 and 25 in the longest ring
+    (64, 4752, 200, 0, (1, 16, 1)), (40, 9504, 72, 1, (1, 32, 1)),  # few rows, more than two waves: both accumulators in turn
+    (4096, 5160, 128, 0, (2, 256, 1)), (2560, 5160, 72, 0, (1, 240, 1)),  # the same with all rows
+    (300, 325, 512, 0, (2, 160, 1)), (300, 321, 512, 0, (1, 64, 1)),  # TMA stores that end inside 16 bytes, after five elements and one
+    (300, 650, 512, 1, (1, 128, 1)), (300, 386, 512, 1, (2, 256, 1)),
+])
+def test_gemm_in_cut(M, N, K, epilogue, cut):
+    """A given cut, in an output with a border that has to stay as it is; whole K gives the bits of every other cut."""
+    import ctypes
+
+    lib = _cut_lib()
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    b = (torch.randn(N, K, device="cuda", generator=g) * 0.02).to(torch.bfloat16)
+    n_out = N // 2 if epilogue else N
+    ld = (n_out + 7) // 8 * 8 + 8
+
+    def run(c):
+        border = torch.full((M + 1, ld), 7.0, device="cuda", dtype=torch.bfloat16)
+        ptr = [ctypes.c_void_p(t.data_ptr()) for t in (a, b, border)]
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert lib.ucclTestGemmInCut(*ptr, M, N, K, K, K, ld, epilogue, (ctypes.c_int * 3)(*c), stream) == 0
+        assert (border[M] == 7).all() and (border[:M, n_out:] == 7).all()
+        return border[:M, :n_out]
+
+    out = run(cut)
+    assert torch.equal(run(cut), out)
+    if cut[2] == 1:
+        assert torch.equal(run((1, 256, 1)), out)
+    ref = a.double() @ b.double().t()
+    if epilogue:
+        ref = torch.nn.functional.silu(ref[:, :n_out]) * ref[:, n_out:]
+    # as in test_gemm_cuts
+    bound = ref.abs() * 2.0 ** -8 + K * 2.0 ** -24 * K * 0.013 * (8 if epilogue else 1) + 1e-6
+    assert ((out.double() - ref).abs() <= bound).all()
+
+
+def test_gemm_cut_choice_runs():
+    """What is chosen can run, for shapes over the whole range; what cannot run is refused."""
+    import ctypes
+    import random
+
+    lib = _cut_lib()
+    rng = random.Random(1)
+    cut = (ctypes.c_int * 3)()
+    seen = set()
+    for _ in range(2000):
+        swiglu = rng.randrange(2)
+        M, N, K = (int(2 ** rng.uniform(0, hi)) for hi in (14, 14.8, 13.8))
+        N, K = max(2, N // 2 * 2), 8 * max(1, K // 8)
+        lib.ucclTestGemmCut(M, N, K, swiglu, cut)
+        assert lib.ucclTestGemmCutRuns(cut, K, swiglu), (M, N, K, swiglu, list(cut))
+        seen.add((cut[0], cut[2]))
+    assert {(1, 1), (2, 1), (1, 2), (1, 4), (1, 8), (2, 2), (2, 4)} <= seen, seen
+    for bad, K, swiglu in (((3, 64, 1), 512, 0), ((0, 64, 1), 512, 0), ((2, 48, 1), 512, 0), ((1, 48, 1), 512, 1), ((1, 24, 1), 512, 0),
+                           ((1, 0, 1), 512, 0), ((1, 272, 1), 512, 0), ((2, 128, 8), 4096, 0), ((1, 128, 8), 448, 0), ((1, 64, 8), 4096, 0),
+                           ((1, 64, 4), 4096, 1), ((1, 128, 0), 512, 0)):
+        assert not lib.ucclTestGemmCutRuns((ctypes.c_int * 3)(*bad), K, swiglu), bad
 
 
 @gpu
