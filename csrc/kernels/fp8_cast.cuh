@@ -1,4 +1,5 @@
-// Block-scaled fp8-e4m3 quantisation shared by the dispatch and cast kernels: per 128 elements
+// Block-scaled fp8-e4m3 quantisation shared by the kernels of moe.cu and fused_cast.cu (moe_noalloc.cu divides
+// for itself, same bytes): per 128 elements
 // scale = max(amax, 1e-10) / 448 and q = e4m3(x / scale), the quotient correctly rounded in fp32.
 #pragma once
 #include <cuda_fp8.h>

@@ -13,8 +13,8 @@
 // peer loads, eight in flight per thread, or multimem.ld_reduce through the switch), scales,
 // converts and stores locally -> rank barrier (peers are done reading my memory).
 // Work is cut in units of 128 elements so that an fp8 scale block never straddles two CTAs, and
-// the 128 elements of a block sit in consecutive lanes of one warp (16 lanes for 16-bit input,
-// 32 for fp32 input), which makes the block's amax a shuffle reduction.
+// the 128 elements of a block sit in consecutive lanes of one warp (16 lanes for 16-bit input, 32 for fp32
+// input; half as many in the one-rank kernel, whose pieces are twice as long), which makes the block's amax a shuffle reduction.
 #include <type_traits>
 
 #include "coll_device.cuh"

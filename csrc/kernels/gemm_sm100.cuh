@@ -1186,8 +1186,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     // The whole warp walks the loop and one elected lane issues.  The tensor core holds few
     // instructions ahead, so the issuer's own path between two stages shows: with a single lane in a
     // divergent branch and one commit per CTA a stage of 512 tensor cycles took 670 (no loads at all
-    // made no difference), in this form 525.  16384 x 4096 x 14336: 1571 -> 1397 us (1.38 PFLOP/s,
-    // against the power cap), zeros 1153 -> 997 us; 2048 x 4096 x 4096: 58 -> 51 us.
+    // made no difference), in this form 525.  16384 x 4096 x 14336: 1571 -> 1388 and
+    // 1397 us in two runs (1.38 PFLOP/s, against the power cap), zeros 1153 -> 997 us; 2048 x 4096 x 4096: 58 -> 51 us.
     if (leader) {
       constexpr uint32_t idesc = ptx::umma_idesc_f16(1u, 2 * BM, BN);
       const bool issue = ptx::elect_one();

@@ -10,6 +10,9 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, swiglu
 
     With ``swiglu=True`` the rows of ``b`` are ``[gate (N/2); up (N/2)]`` and the result is
     ``silu(a @ gate.T) * (a @ up.T)`` of shape [M, N/2], computed in the GEMM epilogue.
+
+    Sums are fp32.  Two runs of a shape give the same bits; where few rows leave SMs idle, K is summed in up to eight
+    parts, so a row can come out rounded differently in a batch of 64 rows than in one of 4096.
     """
     if not (a.is_cuda and b.is_cuda):
         raise ValueError("gemm_bf16 needs CUDA tensors")
