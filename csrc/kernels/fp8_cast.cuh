@@ -5,6 +5,8 @@
 #include <cuda_fp8.h>
 #include <stdint.h>
 
+#include "ptx.cuh"
+
 namespace uccl {
 namespace fp8 {
 
@@ -16,22 +18,8 @@ __device__ __forceinline__ uint32_t pack4(float a, float b, float c, float d) {
   return static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
 }
 
-// Two elements per instruction.
-__device__ __forceinline__ float2 mul2(float2 x, float2 y) {
-  float2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;"
-      : "=l"(reinterpret_cast<unsigned long long&>(r))
-      : "l"(reinterpret_cast<const unsigned long long&>(x)), "l"(reinterpret_cast<const unsigned long long&>(y)));
-  return r;
-}
-__device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {
-  float2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(reinterpret_cast<unsigned long long&>(r))
-      : "l"(reinterpret_cast<const unsigned long long&>(x)), "l"(reinterpret_cast<const unsigned long long&>(y)),
-        "l"(reinterpret_cast<const unsigned long long&>(z)));
-  return r;
-}
+using ptx::fma2;
+using ptx::mul2;
 
 // Correctly rounded quotients by one divisor, for the many elements that share a scale.  Markstein's
 // theorem ("Computation of elementary functions on the IBM RISC System/6000 processor", 1990): with y =

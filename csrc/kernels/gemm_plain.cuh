@@ -65,9 +65,8 @@ template <int EPI>
 __device__ __forceinline__ void pack16(const uint32_t (&x)[16], const uint32_t (&y)[16], uint32_t (&o)[8]) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const float p = __uint_as_float(x[2 * j]), q = __uint_as_float(x[2 * j + 1]);
-    if (EPI == kEpiSwiGLU) o[j] = ptx::pack_bf16x2(silu_f(p) * __uint_as_float(y[2 * j]), silu_f(q) * __uint_as_float(y[2 * j + 1]));
-    else o[j] = ptx::pack_bf16x2(p, q);
+    if (EPI == kEpiSwiGLU) o[j] = swiglu2(&x[2 * j], &y[2 * j]);
+    else o[j] = ptx::pack_bf16x2(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1]));
   }
 }
 __device__ __forceinline__ void store16(const Args& a, int row, int col, const uint32_t (&o)[8]) {

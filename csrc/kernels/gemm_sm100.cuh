@@ -35,6 +35,7 @@
 #pragma once
 #include <cuda.h>
 #include "ptx.cuh"
+#include "swiglu.cuh"
 
 // Phase-skipping switches (Args.debug) and in-kernel time stamps (Args.times) exist only in builds
 // made with UCCL_EXPERIMENTS=1 (benchmarks/tp_breakdown.py); product builds compile them out.
@@ -152,18 +153,6 @@ struct Args {
                             // 32 / 64 all-gather without remote / local copies
   CommArgs comm;
 };
-
-// x / (1 + exp(-x)).  The division has a slow path for zero numerators, which a whole warp walks through for one lane,
-// and the accumulator rows of a tile that lie beyond M hold nothing else: a zero, whose result is itself, divides 1
-// instead.  The compiler would see that this quotient is not used and divide x after all; the empty asm keeps it
-// from looking.  1212 x 10192 x 1760 (a last tile of 188 rows) in tiles of
-// 256 x 256: 57.5 us with the division by x, 42.5 now, 42.7 with 1280 rows.
-__device__ __forceinline__ float silu_f(float x) {
-  float n = x == 0.f ? 1.f : x;
-  asm("" : "+f"(n));
-  const float q = n / (1.0f + __expf(-x));
-  return x == 0.f ? x : q;
-}
 
 // Bounded wait until *flag >= target. Returns false on timeout / abort.
 // Relaxed polls with a growing pause, one system-scope fence on success.
@@ -727,15 +716,7 @@ __device__ __forceinline__ void epilogue_tile(const Args& a, const PeerMaps& pm,
           ptx::tmem_ld_32x32b_x32(taddr + BN / 2 + g * 64 + h * 32, up);
           ptx::tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float o[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = silu_f(__uint_as_float(gt[8 * j + e])) * __uint_as_float(up[8 * j + e]);
-            v[h * 4 + j].x = ptx::pack_bf16x2(o[0], o[1]);
-            v[h * 4 + j].y = ptx::pack_bf16x2(o[2], o[3]);
-            v[h * 4 + j].z = ptx::pack_bf16x2(o[4], o[5]);
-            v[h * 4 + j].w = ptx::pack_bf16x2(o[6], o[7]);
-          }
+          for (int j = 0; j < 4; ++j) v[h * 4 + j] = swiglu8(gt + 8 * j, up + 8 * j);
         }
         const int col0 = nb * (BN / 2) + g * 64;
         stage_and_store<NBUF>(cmap, v, col0, crow0, col0 < out_n && crow0 < a.M, lane, stage, stage_it);
@@ -819,21 +800,14 @@ __device__ __forceinline__ void epilogue_tile(const Args& a, const PeerMaps& pm,
       if (row < a.M) {
         if (col0 + 32 <= out_n) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float h[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) h[e] = silu_f(__uint_as_float(g[8 * j + e])) * __uint_as_float(u[8 * j + e]);
-            uint4 v;
-            v.x = ptx::pack_bf16x2(h[0], h[1]);
-            v.y = ptx::pack_bf16x2(h[2], h[3]);
-            v.z = ptx::pack_bf16x2(h[4], h[5]);
-            v.w = ptx::pack_bf16x2(h[6], h[7]);
-            *reinterpret_cast<uint4*>(crow + c * 32 + j * 8) = v;
-          }
+          for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(crow + c * 32 + j * 8) = swiglu8(g + 8 * j, u + 8 * j);
         } else {
-          for (int j = 0; j < 32; ++j)
-            if (col0 + j < out_n)
-              crow[c * 32 + j] = __float2bfloat16(silu_f(__uint_as_float(g[j])) * __uint_as_float(u[j]));
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const uint32_t w = swiglu2(g + j, u + j);
+            if (col0 + j < out_n) reinterpret_cast<uint16_t*>(crow)[c * 32 + j] = static_cast<uint16_t>(w);
+            if (col0 + j + 1 < out_n) reinterpret_cast<uint16_t*>(crow)[c * 32 + j + 1] = static_cast<uint16_t>(w >> 16);
+          }
         }
       }
     }

@@ -433,6 +433,24 @@ __device__ __forceinline__ void umma_commit_both(uint64_t* bar, int leader = 0) 
                : "memory");
 }
 
+// ---------------------------------------------------------------- packed arithmetic
+// Two elements per instruction.
+__device__ __forceinline__ float2 mul2(float2 x, float2 y) {
+  float2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<const unsigned long long&>(x)), "l"(reinterpret_cast<const unsigned long long&>(y)));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {
+  float2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<const unsigned long long&>(x)), "l"(reinterpret_cast<const unsigned long long&>(y)),
+        "l"(reinterpret_cast<const unsigned long long&>(z)));
+  return r;
+}
+
 // ---------------------------------------------------------------- conversions
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);

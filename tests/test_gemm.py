@@ -157,6 +157,28 @@ def test_gemm_cut_choice_runs():
 
 
 @gpu
+def test_swiglu_over_the_range_of_gates():
+    """silu of gates over the whole range, where exp(-x) is infinite and where it vanishes, against fp64."""
+    from unified_ccl_b200.ops import gemm_bf16
+
+    mag = torch.cat([torch.logspace(-30, 38, 2037, dtype=torch.float64), torch.linspace(80, 92, 2048, dtype=torch.float64)])
+    x = torch.cat([mag, -mag, torch.zeros(6, dtype=torch.float64)]).to("cuda", torch.bfloat16)  # 8176 gates, a row of B each
+    b = torch.zeros(2 * x.numel(), 64, device="cuda", dtype=torch.bfloat16)
+    b[:x.numel(), 0] = x
+    b[x.numel():, 0] = 1.0
+    a = torch.zeros(256, 64, device="cuda", dtype=torch.bfloat16)
+    a[:, 0] = 1.0
+    ref = torch.nn.functional.silu(x.double())
+    for rows in (3, 256):
+        out = gemm_bf16(a[:rows], b, swiglu=True).double()
+        # one rounding to bf16; exp(-x) of 2 units in its last place and of |x| units by its rounded argument; where it is
+        # infinite the result is zero, and below 2^-126 bf16 has fewer digits
+        bound = ref.abs() * (2.0 ** -8 + x.double().abs().clamp(max=100) * 2.0 ** -23) + 3e-37
+        assert ((out - ref).abs() <= bound).all()
+        assert (out[:, -6:] == 0).all()
+
+
+@gpu
 @pytest.mark.parametrize("tokens", [5, 300])
 def test_gemm_chain_captured(tokens):
     """Launches that come up early wait for the ones before: each operand and each output of a GEMM is written or read
