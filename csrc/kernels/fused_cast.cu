@@ -21,6 +21,7 @@
 #include "collectives.cuh"
 #include "fp8_cast.cuh"
 #include "gemm_sm100.h"
+#include "launch.cuh"
 
 namespace uccl {
 namespace dev {
@@ -250,6 +251,8 @@ __device__ __forceinline__ void cast_share(const CastLocalArgs& a, size_t first)
 }
 template <int DT, int OUT, int U>
 __global__ void __launch_bounds__(kCastThreads, 4) cast_local_kernel(const __grid_constant__ CastLocalArgs a) {
+  ptx::launch_dependents();
+  ptx::wait_dependencies();
   cast_share<DT, OUT, U>(a, static_cast<size_t>(blockIdx.x) * (kCastThreads * U));
 }
 // Fewer CTAs than shares, for a communicator whose CTAs are limited.  A kernel of its own: with this loop around the
@@ -257,6 +260,8 @@ __global__ void __launch_bounds__(kCastThreads, 4) cast_local_kernel(const __gri
 template <int DT, int OUT>
 __global__ void __launch_bounds__(kCastThreads, 4) cast_limited_kernel(const __grid_constant__ CastLocalArgs a) {
   constexpr size_t kShare = kCastThreads * 4, E = 32 / Vec<DT>::ES;
+  ptx::launch_dependents();
+  ptx::wait_dependencies();
   for (size_t first = blockIdx.x * kShare; first < (a.elems + E - 1) / E; first += gridDim.x * kShare) cast_share<DT, OUT, 4>(a, first);
 }
 
@@ -271,10 +276,9 @@ static cudaError_t launchLocal(const dev::CastLocalArgs& a, int limit, cudaStrea
   constexpr size_t T = dev::kCastThreads;
   const bool four = pieces >= static_cast<size_t>(deviceSmCount()) * 4 * T * 4;
   const size_t share = four ? 4 * T : T, ctas = (pieces + share - 1) / share;
-  if (limit > 0 && ctas > static_cast<size_t>(limit)) dev::cast_limited_kernel<DT, OUT><<<limit, T, 0, s>>>(a);
-  else if (four) dev::cast_local_kernel<DT, OUT, 4><<<static_cast<unsigned>(ctas), T, 0, s>>>(a);
-  else dev::cast_local_kernel<DT, OUT, 1><<<static_cast<unsigned>(ctas), T, 0, s>>>(a);
-  return cudaGetLastError();
+  if (limit > 0 && ctas > static_cast<size_t>(limit)) return launchOverlapped(dev::cast_limited_kernel<DT, OUT>, limit, T, 0, s, a);
+  if (four) return launchOverlapped(dev::cast_local_kernel<DT, OUT, 4>, static_cast<unsigned>(ctas), T, 0, s, a);
+  return launchOverlapped(dev::cast_local_kernel<DT, OUT, 1>, static_cast<unsigned>(ctas), T, 0, s, a);
 }
 
 template <int DT>

@@ -18,6 +18,7 @@
 
 #include "coll_device.cuh"
 #include "collectives.cuh"
+#include "launch.cuh"
 #include "gemm_sm100.h"
 
 #ifdef UCCL_EXPERIMENTS
@@ -330,6 +331,8 @@ __global__ void __launch_bounds__(NV * W > 32 ? 512 : 1024) add_norm_kernel(cons
       ptx::st_global_v4(p, v[0]);
     }
   };
+  ptx::launch_dependents();
+  ptx::wait_dependencies();
 #pragma unroll
   for (int j = 0; j < NV; ++j) {
     const int v = t + j * lanes;
@@ -380,10 +383,11 @@ static cudaError_t launchNormLocal(const dev::NormLocalArgs& l, cudaStream_t s) 
   const int lanes = ((pieces + nv - 1) / nv + 31) / 32 * 32;
   const int rows = lanes >= 256 ? 1 : 256 / lanes;
   const unsigned grid = static_cast<unsigned>((static_cast<long>(l.tokens) + rows - 1) / rows);
-  if (nv == 1) dev::add_norm_kernel<1, W><<<grid, lanes * rows, 0, s>>>(l, lanes);
-  else if (nv == 2) dev::add_norm_kernel<2, W><<<grid, lanes * rows, 0, s>>>(l, lanes);
-  else if constexpr (W == 16) dev::add_norm_kernel<4, W><<<grid, lanes * rows, 0, s>>>(l, lanes);  // 32-byte pieces: two at most
-  return cudaGetLastError();
+  if (nv == 1) return launchOverlapped(dev::add_norm_kernel<1, W>, grid, lanes * rows, 0, s, l, lanes);
+  if constexpr (W == 16) {  // 32-byte pieces: two at most
+    if (nv > 2) return launchOverlapped(dev::add_norm_kernel<4, W>, grid, lanes * rows, 0, s, l, lanes);
+  }
+  return launchOverlapped(dev::add_norm_kernel<2, W>, grid, lanes * rows, 0, s, l, lanes);
 }
 
 cudaError_t launchArNormKernel(const ArNormArgs& a, int blocks, cudaStream_t stream) {

@@ -1,0 +1,28 @@
+// Launches that come up while the one before ends.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace uccl {
+
+// Launches `kern`, which calls ptx::wait_dependencies before it touches memory, with programmatic serialization: its CTAs
+// start as soon as the kernel before has none left to start, and the launch's latency and their set-up go by while that
+// one ends: about 2 us of a launch (residual + RMSNorm 8192 x 8192 82.7 -> 80.5 us, 7 rows of it 5.7 -> 5.0, MoE combine 84.7
+// -> 82.8, 128 MiB cast to fp8 36.9 -> 35.5, an MoE layer of 96 tokens 28.3 -> 26.4).  A launch that was refused is reported here and not by the thread's next one.
+template <typename... Params, typename... Args>
+cudaError_t launchOverlapped(void (*kern)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(block, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e;
+}
+
+}  // namespace uccl

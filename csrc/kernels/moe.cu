@@ -20,6 +20,7 @@
 #include "coll_device.cuh"
 #include "fp8_cast.cuh"
 #include "gemm_sm100.h"
+#include "launch.cuh"
 #include "moe.h"
 
 namespace uccl {
@@ -81,6 +82,8 @@ __global__ void __launch_bounds__(512, 2) moe_dispatch_kernel(const __grid_const
     return -1;
   };
 
+  if (n == 1) ptx::launch_dependents();
+  ptx::wait_dependencies();
   int buf = 0;
   load(blockIdx.x);
   if (threadIdx.x < 32) {
@@ -147,12 +150,9 @@ __global__ void __launch_bounds__(512, 2) moe_dispatch_kernel(const __grid_const
     }
     buf = buf + 1 == kMoeBufs ? 0 : buf + 1;
   }
-  // Every bulk copy of this thread has completed (written, not just read) before the CTA reports in; with
-  // one rank the end of the kernel completes them.
-  if (router) {
-    if (n > 1) ptx::tma_store_wait<0>();
-    else ptx::tma_store_wait_read<0>();
-  }
+  // Every bulk copy of this thread has completed (written, not just read) before the CTA reports in, and before a
+  // launch that has come up early may read the rows.
+  if (router) ptx::tma_store_wait<0>();
 
   // ---- completion: the last CTA publishes counts and flags, then waits for every source
   __shared__ int s_last;
@@ -208,6 +208,8 @@ __global__ void __launch_bounds__(kCombineThreads, TK > 8 ? 3 : TK > 4 ? 5 : 6) 
   const int t = static_cast<int>(item / chunks), c = static_cast<int>(item - static_cast<long>(t) * chunks);
   if (t >= a.tokens) return;
   const int H = a.hidden, el = c * 256 + lane * 8;
+  if (a.dc.nranks == 1) ptx::launch_dependents();
+  ptx::wait_dependencies();
   int slot = -1;
   float weight = 0.f;
   if (lane < a.topk) {
@@ -251,6 +253,8 @@ cudaError_t launchMoeDispatch(const MoeArgs& a, cudaStream_t stream) {
   // as many CTAs as fit at once: 64 registers a thread
   const int perSm = 1024 / threads;
   const int ctas = std::max(1, std::min(a.tokens, deviceSmCount() * perSm));
+  // ranks that wait for one another keep to the plain launch
+  if (a.dc.nranks == 1) return launchOverlapped(dev::moe_dispatch_kernel, ctas, threads, smem, stream, a);
   dev::moe_dispatch_kernel<<<ctas, threads, smem, stream>>>(a);
   return cudaGetLastError();
 }
@@ -260,11 +264,14 @@ cudaError_t launchMoeCombine(const MoeArgs& a, cudaStream_t stream) {
   const int chunks = (a.hidden + 255) / 256;
   constexpr int warps = dev::kCombineThreads / 32;
   const unsigned ctas = static_cast<unsigned>((static_cast<long>(a.tokens) * chunks + warps - 1) / warps);
-  if (a.topk <= 2) dev::moe_combine_kernel<2><<<ctas, dev::kCombineThreads, 0, stream>>>(a, chunks);
-  else if (a.topk <= 4) dev::moe_combine_kernel<4><<<ctas, dev::kCombineThreads, 0, stream>>>(a, chunks);
-  else if (a.topk <= 8) dev::moe_combine_kernel<8><<<ctas, dev::kCombineThreads, 0, stream>>>(a, chunks);
-  else dev::moe_combine_kernel<16><<<ctas, dev::kCombineThreads, 0, stream>>>(a, chunks);
-  return cudaGetLastError();
+  auto launch = [&](void (*kern)(MoeArgs, int)) {
+    if (a.dc.nranks == 1) return launchOverlapped(kern, ctas, dev::kCombineThreads, 0, stream, a, chunks);
+    kern<<<ctas, dev::kCombineThreads, 0, stream>>>(a, chunks);
+    return cudaGetLastError();
+  };
+  if (a.topk <= 2) return launch(dev::moe_combine_kernel<2>);
+  if (a.topk <= 4) return launch(dev::moe_combine_kernel<4>);
+  return a.topk <= 8 ? launch(dev::moe_combine_kernel<8>) : launch(dev::moe_combine_kernel<16>);
 }
 
 }  // namespace uccl
