@@ -48,10 +48,13 @@ CU_OBJS := $(patsubst %.cu,$(BUILD)/%.cu.o,$(CU_SRCS))
 ifeq ($(UCCL_BUILD_PYTHON),1)
 PYINC     := $(shell $(PYTHON) -c "import sysconfig; print(sysconfig.get_paths()['include'])")
 PYBINDINC := $(shell $(PYTHON) -c "import pybind11; print(pybind11.get_include())")
+TORCHDIR  := $(shell $(PYTHON) -c "import importlib.util as u; s = u.find_spec('torch'); print(s.submodule_search_locations[0] if s else '')")
 EXTSUFFIX := $(shell $(PYTHON) -c "import sysconfig; print(sysconfig.get_config_var('EXT_SUFFIX'))")
 endif
 LIB       := $(PKG)/libuccl.so
 PYMOD     := $(PKG)/_uccl_bindings$(EXTSUFFIX)
+# the calls on torch tensors; left out (and with it only their shortcut) where torch has no headers
+TENSORMOD := $(PKG)/_uccl_tensor_calls$(EXTSUFFIX)
 PLUGIN    := plugins/sample/libuccl-net-sample.so
 UCXPLUGIN := plugins/ucx/libuccl-net-ucx.so
 # test-only code: native self tests of the host runtime, kernels that call the device-side RMA
@@ -66,6 +69,9 @@ PUBLIC_HEADERS := include/uccl.h include/uccl_net.h include/uccl_device.cuh incl
 TARGETS := $(LIB) $(BASELINE)
 ifeq ($(UCCL_BUILD_PYTHON),1)
 TARGETS += $(PYMOD)
+ifneq ($(wildcard $(TORCHDIR)/include/torch/csrc/autograd/python_variable.h),)
+TARGETS += $(TENSORMOD)
+endif
 endif
 ifeq ($(UCCL_BUILD_PLUGIN),1)
 TARGETS += $(PLUGIN)
@@ -93,6 +99,10 @@ $(LIB): $(CC_OBJS) $(CU_OBJS)
 $(PYMOD): csrc/python/bindings.cc $(LIB) $(wildcard include/*.h)
 	$(CXX) $(CXXFLAGS) -fvisibility=hidden -I$(PYINC) -I$(PYBINDINC) -shared $< -o $@ \
 	    -L$(PKG) -luccl -Wl,-rpath,'$$ORIGIN'
+
+$(TENSORMOD): csrc/python/tensor_calls.cc $(LIB) $(wildcard include/*.h)
+	$(CXX) $(filter-out -g,$(CXXFLAGS)) -fvisibility=hidden -I$(PYINC) -isystem $(TORCHDIR)/include -isystem $(TORCHDIR)/include/torch/csrc/api/include \
+	    -shared $< -o $@ -L$(PKG) -luccl -L$(TORCHDIR)/lib -ltorch_python -ltorch_cpu -lc10 -Wl,-rpath,'$$ORIGIN'
 
 $(PLUGIN): plugins/sample/plugin.cc include/uccl_net.h include/uccl.h
 	$(CXX) $(CXXFLAGS) -shared $< -o $@

@@ -2,7 +2,7 @@
 import torch
 
 from .. import _C
-from ..communicator import current_raw_stream
+from ..communicator import current_raw_stream, tensor_calls
 
 
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, swiglu: bool = False) -> torch.Tensor:
@@ -14,6 +14,8 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, swiglu
     Sums are fp32.  Two runs of a shape give the same bits; where few rows leave SMs idle, K is summed in up to eight
     parts, so a row can come out rounded differently in a batch of 64 rows than in one of 4096.
     """
+    if out is not None and tensor_calls.gemm(a, b, out, swiglu):
+        return out
     if not (a.is_cuda and b.is_cuda):
         raise ValueError("gemm_bf16 needs CUDA tensors")
     if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:

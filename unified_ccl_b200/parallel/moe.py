@@ -2,7 +2,7 @@
 import torch
 
 from .. import _C
-from ..communicator import Communicator, _tensor_from_ptr
+from ..communicator import Communicator, _tensor_from_ptr, tensor_calls
 
 
 class MoeDispatcher:
@@ -32,6 +32,9 @@ class MoeDispatcher:
         self._tokens = 0
 
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor):
+        if tensor_calls.moe_dispatch(self._ctx, self.comm._device, self.hidden, self.topk, x, topk_idx):
+            self._tokens = x.shape[0]
+            return self.recv_x, self.recv_scale, self.recv_meta, self.recv_counts
         if x.dtype != torch.bfloat16 or not x.is_contiguous() or x.shape[1] != self.hidden:
             raise TypeError("x must be contiguous bf16 [tokens, hidden]")
         if topk_idx.dtype != torch.int32 or not topk_idx.is_contiguous() or topk_idx.shape != (x.shape[0], self.topk):
@@ -41,6 +44,8 @@ class MoeDispatcher:
         return self.recv_x, self.recv_scale, self.recv_meta, self.recv_counts
 
     def combine(self, topk_weight: torch.Tensor, out: torch.Tensor = None) -> torch.Tensor:
+        if out is not None and tensor_calls.moe_combine(self._ctx, self.comm._device, self._tokens, self.hidden, self.topk, topk_weight, out):
+            return out
         if topk_weight.dtype != torch.float32 or not topk_weight.is_contiguous() or topk_weight.shape != (self._tokens, self.topk):
             raise TypeError("topk_weight must be contiguous fp32 [tokens, topk] of the last dispatch")
         if out is None:

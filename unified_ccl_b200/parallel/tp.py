@@ -2,7 +2,7 @@
 import torch
 
 from .. import _C
-from ..communicator import Communicator
+from ..communicator import Communicator, tensor_calls
 
 
 def _bf16(*ts):
@@ -19,6 +19,10 @@ def allreduce_residual_rmsnorm(comm: Communicator, x: torch.Tensor, residual: to
     ``residual_out`` with ``comm.empty``; other tensors are staged (size limited by UCCL_STAGING_BYTES).
     ``residual_out`` may be ``residual`` itself.
     """
+    if out is not None:
+        h = residual if residual_out is None else residual_out
+        if tensor_calls.norm(comm.handle, comm._device, x, residual, gamma, eps, out, h):
+            return out, h
     _bf16(x, residual, gamma)
     tokens, hidden = x.shape
     if out is None:
