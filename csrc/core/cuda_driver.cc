@@ -46,6 +46,7 @@ const DriverApi& driverApi() {
     ok &= resolve("cuGetErrorString", &api.getErrorString);
     ok &= resolve("cuCtxGetCurrent", &api.ctxGetCurrent);
     ok &= resolve("cuMemGetAddressRange", &api.memGetAddressRange);
+    ok &= resolve("cuPointerGetAttributes", &api.pointerGetAttributes);
     // Multicast objects are optional (absent on drivers/GPUs without NVLS).
     resolve("cuMulticastCreate", &api.multicastCreate);
     resolve("cuMulticastAddDevice", &api.multicastAddDevice);

@@ -31,6 +31,7 @@ struct DriverApi {
   decltype(&cuGetErrorString) getErrorString = nullptr;
   decltype(&cuCtxGetCurrent) ctxGetCurrent = nullptr;
   decltype(&cuMemGetAddressRange) memGetAddressRange = nullptr;
+  decltype(&cuPointerGetAttributes) pointerGetAttributes = nullptr;
 };
 
 // Returns the process-wide table; `ok` is false when no driver is present.

@@ -131,4 +131,7 @@ struct ArNormArgs {
 // `blocks`: CTAs of a launch among ranks; on one rank the data decides and it is not read.
 cudaError_t launchArNormKernel(const ArNormArgs& a, int blocks, cudaStream_t stream);
 
+// dst = src, both 16-byte aligned memory of this GPU that does not overlap (one rank).
+cudaError_t launchLocalCopy(const void* src, void* dst, size_t bytes, cudaStream_t stream);
+
 }  // namespace uccl
