@@ -246,6 +246,9 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   if (CG == 2) ptx::cluster_sync();  // both CTAs' barriers and TMEM exist before anybody signals the other
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  // The first tile's place takes divisions: done while the launch before runs, not between its end and the first load.
+  int first_mt, first_nt;
+  coords<CG == 2 ? 8 : 16>(a, worker, first_mt, first_nt);
   // Everything up to here may run while the launch before is still at work; no operand is read and C not
   // touched before that one has ended.
   ptx::launch_dependents();
@@ -259,8 +262,8 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       int s = 0;
       uint32_t ph = 1;
       for (int tile = worker; tile < a.num_tiles && !*bail; tile += a.workers) {
-        int mt, nt;
-        coords<CG == 2 ? 8 : 16>(a, tile, mt, nt);
+        int mt = first_mt, nt = first_nt;
+        if (tile != worker) coords<CG == 2 ? 8 : 16>(a, tile, mt, nt);
         const int m0 = (mt * CG + half) * BM;
         const int b0 = nt * (EPI == kEpiSwiGLU ? a.out_bn : a.bn);
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -332,10 +335,10 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     uint32_t tcount = 0, stage_it = 0;
     for (int tile = worker; tile < a.num_tiles; tile += a.workers, ++tcount) {
       const uint32_t acc = tcount & 1, acc_ph = (tcount >> 1) & 1;
+      int mt = first_mt, nt = first_nt;
+      if (tile != worker) coords<CG == 2 ? 8 : 16>(a, tile, mt, nt);
       if (!warp_wait(&tfull_bar[acc], acc_ph, bail)) break;
       if (a.split > 1) break;  // one tile, finished below
-      int mt, nt;
-      coords<CG == 2 ? 8 : 16>(a, tile, mt, nt);
       ptx::tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
       store_tile<EPI>(a, &tmC, taddr, (mt * CG + half) * BM + q * 32, nt * a.out_bn, lane, stage, stage_it);
@@ -353,8 +356,7 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   ptx::tc_fence_before();
   __syncthreads();
   if (a.split > 1) {
-    int mt, nt;
-    coords<CG == 2 ? 8 : 16>(a, worker, mt, nt);
+    const int mt = first_mt, nt = first_nt;
     const int q = warp & 3, r = q * 32 + lane, row = (mt * CG + half) * BM + r;
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const bool busy = warp >= 2 && row - lane < a.M;
