@@ -220,6 +220,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// Whether the phase has completed, without waiting for it: one lane (`act` != 0) of a whole warp looks, the others get 0.
+__device__ __forceinline__ uint32_t mbar_test_from(uint32_t act, uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 q, %3, 0;\n\t"
+      "setp.ne.b32 p, 0, 0;\n\t"
+      "@q mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(act)
+      : "memory");
+  return ok;
+}
 // Bounded wait. Returns false if `max_polls` try_wait rounds passed without the phase
 // completing (each try_wait itself blocks for a hardware-defined short time), or if the
 // CTA-wide `*bail` word became non-zero.
@@ -310,6 +324,24 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// The same from a whole warp of which one lane (`act` != 0) issues.  With no branch around it the compiler keeps the
+// operands in uniform registers: four MMAs of 128 columns take 258 cycles, behind a branch 302 to 490.
+__device__ __forceinline__ void umma_f16_from(uint32_t act, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(act)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_from(uint32_t act, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(act)
       : "memory");
 }
 // Arrive on an mbarrier of this CTA once all previously issued MMAs have completed.
