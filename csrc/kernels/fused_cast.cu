@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, 1) reduce_cast_kernel(const __grid_c
 
 // One rank: nothing to add and nobody to meet, so the work is a stream from memory to memory.  Every
 // thread takes U pieces of 32 input bytes (16 elements of a 16-bit type, 8 of fp32) that lie one CTA
-// width apart, with all their loads in flight before the first use: four pieces at four 256-thread
+// width apart, with all their loads in flight before the first use: four pieces (fp8 output: two) at four 256-thread
 // CTAs per SM are 128 KiB in flight, where the shared kernel above, with one 16-byte load per thread
 // on at most kMaxBlocks CTAs, reached a fifth of the memory bandwidth.  A 128-element scale block is
 // 8 (or 16) consecutive lanes.
@@ -171,8 +171,7 @@ __device__ __forceinline__ float piece_amax(const uint32_t (&raw)[8]) {
 // One CTA's share: U pieces per thread from piece `first` on.
 template <int DT, int OUT, int U>
 __device__ __forceinline__ void cast_share(const CastLocalArgs& a, size_t first) {
-  using V = Vec<DT>;
-  constexpr int E = 32 / V::ES;     // elements per piece
+  constexpr int E = 32 / Vec<DT>::ES;  // elements per piece
   constexpr int LANES = 128 / E;    // lanes that share one scale block
   const size_t pieces = (a.elems + E - 1) / E;
   const size_t c0 = first + threadIdx.x;
@@ -202,16 +201,14 @@ __device__ __forceinline__ void cast_share(const CastLocalArgs& a, size_t first)
     const bool live = c < pieces, whole = (c + 1) * E <= a.elems;
     // 0 + x, as a sum starts: a zero comes out positive
     float2 v[E / 2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      V::add(acc, make_uint4(raw[u][4 * h], raw[u][4 * h + 1], raw[u][4 * h + 2], raw[u][4 * h + 3]));
-#pragma unroll
-      for (int e = 0; e < E / 4; ++e) v[h * (E / 4) + e] = make_float2(acc[2 * e], acc[2 * e + 1]);
-    }
     const float factor = OUT == OUT_FP8 ? -a.scale : a.scale;  // the divisor takes its elements negated
 #pragma unroll
-    for (int e = 0; e < E / 2; ++e) v[e] = fp8::mul2(v[e], make_float2(factor, factor));
+    for (int e = 0; e < E / 2; ++e) {
+      float2 x;
+      if constexpr (DT == DT_F32) x = make_float2(__uint_as_float(raw[u][2 * e]), __uint_as_float(raw[u][2 * e + 1]));
+      else x = DT == DT_BF16 ? ptx::unpack_bf16x2(raw[u][e]) : ptx::unpack_f16x2(raw[u][e]);
+      v[e] = ptx::mul2(ptx::add2(make_float2(0.f, 0.f), x), make_float2(factor, factor));
+    }
     char* out = a.out + c * E * (OUT == OUT_FP8 ? 1 : OUT == OUT_F32 ? 4 : 2);
     if (OUT == OUT_FP8) {
       const float blockScale = fp8::block_scale(fabsf(piece_amax<DT, LANES>(raw[u]) * a.scale));
@@ -249,8 +246,13 @@ __device__ __forceinline__ void cast_share(const CastLocalArgs& a, size_t first)
     }
   }
 }
+// Pieces per thread of a large launch, and CTAs per SM.  A conversion to fp8 takes some hundred instructions a piece, and
+// two pieces on six CTAs put more of them beside other CTAs' loads than four pieces on four: 64 Mi bf16 33.0 -> 31.4 us, 16 Mi
+// 11.4 -> 10.1, 6 Mi fp32 6.7 -> 5.8; with the rest, bound by its loads and stores, it is the same.
+template <int OUT>
+constexpr int kCastPieces = OUT == OUT_FP8 ? 2 : 4;
 template <int DT, int OUT, int U>
-__global__ void __launch_bounds__(kCastThreads, 4) cast_local_kernel(const __grid_constant__ CastLocalArgs a) {
+__global__ void __launch_bounds__(kCastThreads, U == 2 ? 6 : 4) cast_local_kernel(const __grid_constant__ CastLocalArgs a) {
   ptx::launch_dependents();
   ptx::wait_dependencies();
   cast_share<DT, OUT, U>(a, static_cast<size_t>(blockIdx.x) * (kCastThreads * U));
@@ -271,13 +273,14 @@ __global__ void __launch_bounds__(kCastThreads, 4) cast_limited_kernel(const __g
 template <int DT, int OUT>
 static cudaError_t launchLocal(const dev::CastLocalArgs& a, int limit, cudaStream_t s) {
   const size_t pieces = (a.elems + 32 / dev::Vec<DT>::ES - 1) / (32 / dev::Vec<DT>::ES);
-  // four pieces per thread once that still gives every SM its four CTAs; below that one piece per
+  // several pieces per thread once four would still give every SM its four CTAs; below that one piece per
   // thread spreads the work over more SMs
   constexpr size_t T = dev::kCastThreads;
-  const bool four = pieces >= static_cast<size_t>(deviceSmCount()) * 4 * T * 4;
-  const size_t share = four ? 4 * T : T, ctas = (pieces + share - 1) / share;
+  constexpr int U = dev::kCastPieces<OUT>;
+  const bool many = pieces >= static_cast<size_t>(deviceSmCount()) * 4 * T * 4;
+  const size_t share = many ? U * T : T, ctas = (pieces + share - 1) / share;
   if (limit > 0 && ctas > static_cast<size_t>(limit)) return launchOverlapped(dev::cast_limited_kernel<DT, OUT>, limit, T, 0, s, a);
-  if (four) return launchOverlapped(dev::cast_local_kernel<DT, OUT, 4>, static_cast<unsigned>(ctas), T, 0, s, a);
+  if (many) return launchOverlapped(dev::cast_local_kernel<DT, OUT, U>, static_cast<unsigned>(ctas), T, 0, s, a);
   return launchOverlapped(dev::cast_local_kernel<DT, OUT, 1>, static_cast<unsigned>(ctas), T, 0, s, a);
 }
 

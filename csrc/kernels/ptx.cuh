@@ -474,6 +474,13 @@ __device__ __forceinline__ float2 mul2(float2 x, float2 y) {
       : "l"(reinterpret_cast<const unsigned long long&>(x)), "l"(reinterpret_cast<const unsigned long long&>(y)));
   return r;
 }
+__device__ __forceinline__ float2 add2(float2 x, float2 y) {
+  float2 r;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<const unsigned long long&>(x)), "l"(reinterpret_cast<const unsigned long long&>(y)));
+  return r;
+}
 __device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {
   float2 r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;"
