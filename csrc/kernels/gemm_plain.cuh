@@ -18,9 +18,9 @@
 // is further from fp64 in parts, and of 64 x 4096 x 14336 0.21% of the elements are not the rounded exact value, uncut 0.79%.
 //
 // Bound by memory when rows are few, by the tensor cores (and then the power cap) when they are many.  Against pair
-// tiles of 256 x 256 alone, 20 launches in a row on operands that are not in L2: 64 x 4096 x 14336 78 -> 25.7 us (4.6
-// TB/s), SwiGLU 64 x 28672 x 4096 80 -> 48.0 us (4.9 TB/s), 512 x 4096 x 4096 29 -> 20.5 us, 1000 x 3592 x 4104
-// 35 -> 30.5 us, SwiGLU 4096 x 7168 x 4096 180 -> 153 us.
+// tiles of 256 x 256 alone, launches in a row on operands that are not in L2: 64 x 4096 x 14336 78 -> 23.7 us (5.0
+// TB/s), SwiGLU 64 x 28672 x 4096 80 -> 40.3 us (5.9 TB/s), 512 x 4096 x 4096 29 -> 19 us, 1000 x 3592 x 4104
+// 35 -> 29.3 us, SwiGLU 4096 x 7168 x 4096 180 -> 156 us.
 #pragma once
 #include "gemm_sm100.cuh"
 

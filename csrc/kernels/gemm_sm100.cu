@@ -147,7 +147,7 @@ bool usePairKernel() {
 // How to cut a GEMM without a collective: the candidate with the fewest cycles by one of two formulas.
 //
 // A tile whole: waves of tiles x the longer of a tile's main loop and of the epilogue that runs beside the next tile's
-// (2150 cycles, and per output column 11, or 49 with silu and its division); at least the time of memory, and
+// (2150 cycles, and per output column 11, or 49 with silu, which has become cheaper since); at least the time of memory, and
 // at least that of all loads together (9000 bytes per cycle into all SMs).  A stage of the main loop takes what the tensor
 // cores need for it (two cycles per accumulator column, at least a round trip of the ring) or its loads (65 bytes
 // per cycle and SM).  A tile in parts of K: the same without the overlapped epilogue (one tile per cluster), plus
@@ -156,7 +156,8 @@ bool usePairKernel() {
 // The constants are fits to measurements with every candidate timed on operands that are not in L2: whole tiles to
 // 658 shapes (1 to 16384 rows, K of 64 to 14336), where the choice takes 1.2% more than the best candidate on average (an
 // earlier formula without the epilogue and the common load rate: 2.4%, and 20% on 4096 x 28672 x 512), the parts to 102
-// of them.  Both sides of some of the lines, in us: 64 x 4096 x 14336 25.3 in four parts of 128 columns, 62 uncut;
+// of them; with the issuer and the epilogue as they are now, the choice takes 0.6% more than the best candidate on 200
+// other shapes.  Both sides of some of the lines, in us: 64 x 4096 x 14336 25.3 in four parts of 128 columns, 62 uncut;
 // 4096 x 28672 x 512 111 in pair tiles of 256, 125 of 224; 8192 x 3592 x 4104 207 in pair tiles of 256, 244 of 192;
 // 200 x 28672 x 4096 51.6 in pair tiles of 224, 60.2 in single CTAs of 208; 512 x 4096 x 4096 20 in tiles of 128, 25 of 256.
 GemmCut choosePlain(int M, int N, int K, bool swiglu) {
