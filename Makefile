@@ -58,7 +58,7 @@ TENSORMOD := $(PKG)/_uccl_tensor_calls$(EXTSUFFIX)
 PLUGIN    := plugins/sample/libuccl-net-sample.so
 UCXPLUGIN := plugins/ucx/libuccl-net-ucx.so
 # test-only code: native self tests of the host runtime, kernels that call the device-side RMA
-# API, and a C++ client of the C ABI
+# API or the epilogue's silu, and a C++ client of the C ABI
 SELFTEST  := tests/native/libuccl_selftest.so
 DEVTEST   := tests/native/libuccl_devtest.so
 CLIENT    := tests/native/c_api_client
@@ -119,8 +119,8 @@ ucx-fake: plugins/ucx/libuccl-net-ucx-fake.so
 $(SELFTEST): tests/native/selftest.cc tests/native/uccl_selftest.h $(LIB) $(wildcard include/*.h csrc/*/*.h)
 	$(CXX) $(CXXFLAGS) -Itests/native -shared $< -o $@ -L$(PKG) -luccl -Wl,-rpath,'$$ORIGIN/../../$(PKG)'
 
-$(DEVTEST): tests/native/rma_device_test.cu include/uccl_device.cuh include/uccl.h $(LIB)
-	$(NVCC) $(NVFLAGS) -shared $< -o $@ -L$(PKG) -luccl -Xlinker -rpath,'$$ORIGIN/../../$(PKG)' -lcudart_static
+$(DEVTEST): tests/native/rma_device_test.cu tests/native/swiglu_device_test.cu include/uccl_device.cuh include/uccl.h csrc/kernels/swiglu.cuh $(LIB)
+	$(NVCC) $(NVFLAGS) -shared $(filter %.cu,$^) -o $@ -L$(PKG) -luccl -Xlinker -rpath,'$$ORIGIN/../../$(PKG)' -lcudart_static
 
 $(BASELINE): baseline/swiglu_kernel.cu
 	$(NVCC) $(NVFLAGS) -shared $< -o $@ -lcudart_static

@@ -19,9 +19,11 @@ __device__ __forceinline__ float rcp_ftz(float x) {
 // -x / (1 + exp(-x)), the quotient rounded to nearest as a division rounds it.  Markstein's method ("Computation of
 // elementary functions on the IBM RISC System/6000 processor", 1990): one Newton step makes the reciprocal y of d right to
 // the last place but for rare mantissas, and q + (x - d q) y is then the rounded quotient.  Both d and x are taken a
-// quarter, so that 1 / d stays a normal number up to where exp(-x) is infinite.  There, for infinite x, and for zeros (whose
-// sign the residual would lose) x y is the answer as it stands.
-// The results are those of x / (1.f + __expf(-x)) for every x but |x| < 2^-124, whose quarter is rounded.
+// quarter, so that 1 / d stays a normal number up to where exp(-x) is infinite.  There, for infinite x, for zeros (whose
+// sign the residual would lose) and for gates so small that their quarter is rounded, x times a quarter of y is the answer as
+// it stands: exp(-x) is 1 for small gates, and the halves of subnormal numbers round once.  What takes the first way is at least
+// 2^-122: the smallest quotient of a large negative gate, -88.7 / exp(88.7), is 2^-121.5.
+// The results are those of x / (1.f + __expf(-x)) for every x, all 2^32 of them compared.
 //
 // A division as such has a slow path, and the branch to it ties each element to the one before: 49 cycles per column of a
 // warp.  Without a branch the elements of a register block overlap: SwiGLU 4096 x 28672 x 512 220 -> 101 us, 16384 x 4096
@@ -35,12 +37,12 @@ __device__ __forceinline__ float2 silu2_negated(float2 x) {
   const float2 nd = ptx::fma2(t, make_float2(-0.25f, -0.25f), make_float2(-0.25f, -0.25f));
   const float2 xq = ptx::mul2(x, make_float2(0.25f, 0.25f));
   float2 ny = make_float2(rcp_ftz(nd.x), rcp_ftz(nd.y));
-  const float2 plain = ptx::mul2(xq, ny);
+  const float2 plain = ptx::mul2(x, ptx::mul2(ny, make_float2(0.25f, 0.25f)));
   ny = ptx::fma2(ptx::fma2(d, ny, make_float2(1.f, 1.f)), ny, ny);
   float2 nq = ptx::mul2(xq, ny);
   nq = ptx::fma2(ptx::fma2(d, nq, xq), ny, nq);
-  nq.x = fabsf(nq.x) > 0.f ? nq.x : plain.x;
-  nq.y = fabsf(nq.y) > 0.f ? nq.y : plain.y;
+  nq.x = fabsf(nq.x) >= 0x1p-122f ? nq.x : plain.x;
+  nq.y = fabsf(nq.y) >= 0x1p-122f ? nq.y : plain.y;
   return nq;
 }
 

@@ -179,6 +179,22 @@ def test_swiglu_over_the_range_of_gates():
 
 
 @gpu
+def test_silu_is_the_quotient_for_every_gate():
+    """The epilogue's branch-free silu has the bits of x / (1.f + __expf(-x)) for all 2^32 gates: zeros, subnormals, infinities
+    and NaN (as NaN), rare mantissas of the reciprocal, and the gates around -88.7 where exp(-x) becomes infinite."""
+    import ctypes
+    import os
+
+    lib = ctypes.CDLL(os.path.join(os.path.dirname(os.path.abspath(__file__)), "native", "libuccl_devtest.so"))
+    lib.ucclDevTestSilu.argtypes = [ctypes.c_uint, ctypes.c_uint, ctypes.c_void_p, ctypes.c_void_p]
+    out = torch.zeros(2, device="cuda", dtype=torch.int32)
+    for first in range(0, 1 << 32, 1 << 30):
+        assert lib.ucclDevTestSilu(first, 1 << 30, out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    wrong, bits = out.tolist()
+    assert wrong == 0, f"{wrong & 0xffffffff} gates differ, one of them {bits & 0xffffffff:#010x}"
+
+
+@gpu
 @pytest.mark.parametrize("tokens", [5, 300])
 def test_gemm_chain_captured(tokens):
     """Launches that come up early wait for the ones before: each operand and each output of a GEMM is written or read
