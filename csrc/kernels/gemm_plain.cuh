@@ -95,22 +95,25 @@ __device__ __forceinline__ void store_tile(const Args& a, const CUtensorMap* tmC
   int c = 0;
 #pragma unroll 1
   for (; c + 64 <= a.tma_bn && col0 + c < a.tma_n; c += 64) {
-    uint4 v[8];
+    if constexpr (EPI == kEpiSwiGLU) {
+      swiglu_and_store<2>(tmC, taddr + c, taddr + a.out_bn + c, col0 + c, row0, true, lane, stage, stage_it);
+    } else {
+      uint4 v[8];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      uint32_t x[32], y[32];
-      ptx::tmem_ld_32x32b_x32(taddr + c + h * 32, x);
-      if (EPI == kEpiSwiGLU) ptx::tmem_ld_32x32b_x32(taddr + a.out_bn + c + h * 32, y);
-      ptx::tmem_ld_wait();
+      for (int h = 0; h < 2; ++h) {
+        uint32_t x[32];
+        ptx::tmem_ld_32x32b_x32(taddr + c + h * 32, x);
+        ptx::tmem_ld_wait();
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        uint32_t o[8];
-        pack16<EPI>(*reinterpret_cast<const uint32_t(*)[16]>(&x[g * 16]), *reinterpret_cast<const uint32_t(*)[16]>(&y[g * 16]), o);
-        v[h * 4 + g * 2] = make_uint4(o[0], o[1], o[2], o[3]);
-        v[h * 4 + g * 2 + 1] = make_uint4(o[4], o[5], o[6], o[7]);
+        for (int g = 0; g < 4; ++g) {
+          uint32_t o[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[j] = ptx::pack_bf16x2(__uint_as_float(x[8 * g + 2 * j]), __uint_as_float(x[8 * g + 2 * j + 1]));
+          v[h * 4 + g] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
       }
+      stage_and_store<2>(tmC, v, col0 + c, row0, true, lane, stage, stage_it);
     }
-    stage_and_store<2>(tmC, v, col0 + c, row0, true, lane, stage, stage_it);
   }
 #pragma unroll 1
   for (; c < a.out_bn && col0 + c < a.out_n; c += 16) {
@@ -196,7 +199,7 @@ __device__ __forceinline__ void sum_parts(const Args& a, const uint8_t* ring, ui
 }
 
 template <int EPI, int CG>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(EPI == kEpiSwiGLU ? SWIGLU_BOUND : NUM_THREADS, 1)
 gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmC, const __grid_constant__ Args a) {
   extern __shared__ uint8_t smem_raw[];

@@ -56,6 +56,7 @@ constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr int NUM_THREADS = 192;
 constexpr int NUM_THREADS_FWD = 224;  // all-gather fusion: one more warp, the forwarder of "spread" mode
+constexpr int SWIGLU_BOUND = 512;     // bound of the SwiGLU kernels' threads: with it the compiler keeps to 128 registers
 constexpr int TMEM_COLS = 512;
 
 // single-CTA kernel: 4 stages of (A 16 KiB + B 32 KiB)
@@ -655,26 +656,67 @@ __device__ void reduce_scatter_tail(const Args& a, uint8_t* smem, uint64_t* tbar
   }
 }
 
+// Bound of a kernel's threads.  SwiGLU kernels are given a wider one than they launch with (SWIGLU_BOUND).
+template <int EPI, int COMM>
+constexpr int kMostThreads = EPI == kEpiSwiGLU ? SWIGLU_BOUND : COMM == kCommAllGather ? NUM_THREADS_FWD : NUM_THREADS;
+
 // ------------------------------------------------------------------ epilogue of one tile, one warp
-// `taddr` addresses this warp's 32 TMEM lanes of the accumulator; `mb` is the 128-row block.
 // 64 columns x 32 rows of bf16 (eight 16-byte pieces per lane) -> 128-byte-swizzled staging buffer
-// -> one TMA store at (col0, row0) of `map`.  One bulk group per call.
+// -> one TMA store at (col0, row0) of `map`.  One bulk group per stage_take and stage_send.
 template <int NBUF>
-__device__ __forceinline__ void stage_and_store(const CUtensorMap* map, const uint4 (&v)[8], int col0, int row0, bool inside,
-                                                int lane, uint8_t* stage, uint32_t& stage_it) {
+__device__ __forceinline__ uint8_t* stage_take(uint8_t* stage, uint32_t& stage_it, int lane) {
   uint8_t* buf = stage + (stage_it % NBUF) * EPI_BUF_BYTES;
   ++stage_it;
   if (lane == 0) ptx::tma_store_wait_read<NBUF - 1>();  // the store that last used this buffer has read it
   __syncwarp();
-  uint8_t* myrow = buf + lane * 128;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) *reinterpret_cast<uint4*>(myrow + ((k ^ (lane & 7)) << 4)) = v[k];  // 128-byte swizzle
+  return buf;
+}
+__device__ __forceinline__ void stage_put(uint8_t* buf, int lane, int k, uint4 v) {  // 128-byte swizzle
+  *reinterpret_cast<uint4*>(buf + lane * 128 + ((k ^ (lane & 7)) << 4)) = v;
+}
+__device__ __forceinline__ void stage_send(const CUtensorMap* map, uint8_t* buf, int col0, int row0, bool inside, int lane) {
   ptx::fence_proxy_async_smem();
   __syncwarp();
   if (lane == 0 && inside) ptx::tma_store_2d(map, buf, col0, row0);
   if (lane == 0) ptx::tma_store_commit();
 }
+template <int NBUF>
+__device__ __forceinline__ void stage_and_store(const CUtensorMap* map, const uint4 (&v)[8], int col0, int row0, bool inside,
+                                                int lane, uint8_t* stage, uint32_t& stage_it) {
+  uint8_t* buf = stage_take<NBUF>(stage, stage_it, lane);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) stage_put(buf, lane, k, v[k]);
+  stage_send(map, buf, col0, row0, inside, lane);
+}
 
+// 64 output columns of silu(gate) * up from the accumulator's columns at `gate` and `up`, in blocks of 16 columns of which
+// the next is read from TMEM while one is computed.  Blocks of 32, all 64 columns kept until their store, took 253
+// registers a thread: beside such a CTA an SM has room for 16 K registers, and no collective's CTA (512 threads of up to 72)
+// fits.  With these blocks and the bound of SWIGLU_BOUND threads it is 128 registers without a spill, at the same speed:
+// 64 x 28672 x 4096 40.8 us with either, 4096 x 28672 x 512 102.9 and 103.3, 16384 x 28672 x 4096 2740 and 2751, 8 x 512 x
+// 256 3.20 and 3.17.  (Without the early read, blocks of 16 take 1.1 to 1.5 times as long where K is 256 or less.)
+template <int NBUF>
+__device__ __forceinline__ void swiglu_and_store(const CUtensorMap* map, uint32_t gate, uint32_t up, int col0, int row0, bool inside,
+                                                 int lane, uint8_t* stage, uint32_t& stage_it) {
+  uint32_t g[2][16], u[2][16];
+  ptx::tmem_ld_32x32b_x16(gate, g[0]);
+  ptx::tmem_ld_32x32b_x16(up, u[0]);
+  uint8_t* buf = stage_take<NBUF>(stage, stage_it, lane);
+  ptx::tmem_ld_wait();
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    if (h < 3) {
+      ptx::tmem_ld_32x32b_x16(gate + (h + 1) * 16, g[(h + 1) & 1]);
+      ptx::tmem_ld_32x32b_x16(up + (h + 1) * 16, u[(h + 1) & 1]);
+    }
+    stage_put(buf, lane, 2 * h, swiglu8(g[h & 1], u[h & 1]));
+    stage_put(buf, lane, 2 * h + 1, swiglu8(g[h & 1] + 8, u[h & 1] + 8));
+    if (h < 3) ptx::tmem_ld_wait();
+  }
+  stage_send(map, buf, col0, row0, inside, lane);
+}
+
+// `taddr` addresses this warp's 32 TMEM lanes of the accumulator; `mb` is the 128-row block.
 // `cmap` != nullptr: C is written through shared memory and TMA stores (whole 128-byte lines, rows
 // and columns beyond the matrix clipped by the copy engine) at rows crow0 ... of that map; else
 // every lane stores its own row with 16-byte stores.
@@ -708,18 +750,8 @@ __device__ __forceinline__ void epilogue_tile(const Args& a, const PeerMaps& pm,
       const int out_n = a.N / 2;
 #pragma unroll 1
       for (int g = 0; g < BN / 128; ++g) {
-        uint4 v[8];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t gt[32], up[32];
-          ptx::tmem_ld_32x32b_x32(taddr + g * 64 + h * 32, gt);
-          ptx::tmem_ld_32x32b_x32(taddr + BN / 2 + g * 64 + h * 32, up);
-          ptx::tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 4; ++j) v[h * 4 + j] = swiglu8(gt + 8 * j, up + 8 * j);
-        }
         const int col0 = nb * (BN / 2) + g * 64;
-        stage_and_store<NBUF>(cmap, v, col0, crow0, col0 < out_n && crow0 < a.M, lane, stage, stage_it);
+        swiglu_and_store<NBUF>(cmap, taddr + g * 64, taddr + BN / 2 + g * 64, col0, crow0, col0 < out_n && crow0 < a.M, lane, stage, stage_it);
       }
     }
     return;
@@ -839,7 +871,7 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
 
 // ------------------------------------------------------------------ single-CTA kernel
 template <int EPI, int COMM>
-__global__ void __launch_bounds__(COMM == kCommAllGather ? NUM_THREADS_FWD : NUM_THREADS, 1)
+__global__ void __launch_bounds__(kMostThreads<EPI, COMM>, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ PeerMaps pm, const Args a) {
   extern __shared__ uint8_t smem_raw[];
@@ -1041,7 +1073,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // instead of once per 128, which cuts shared-memory fill traffic by a third and leaves room for
 // six pipeline stages.
 template <int EPI, int COMM>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(COMM == kCommAllGather ? NUM_THREADS_FWD : NUM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMostThreads<EPI, COMM>, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ PeerMaps pm, const Args a) {
   // The reduce-scatter fusion trades one pipeline stage for a deeper epilogue staging area: a

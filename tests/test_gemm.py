@@ -195,6 +195,40 @@ def test_silu_is_the_quotient_for_every_gate():
 
 
 @gpu
+def test_swiglu_gemm_leaves_room_for_another_kernel():
+    """A SwiGLU GEMM holds every SM for its whole time.  CTAs of 512 threads, as a collective among ranks has them, come up beside
+    its CTAs: a norm of 8192 columns on another stream ends long before the GEMM does."""
+    import os
+
+    from unified_ccl_b200 import Communicator
+    from unified_ccl_b200.ops import gemm_bf16
+    from unified_ccl_b200.parallel import allreduce_residual_rmsnorm
+
+    os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    comm = Communicator(0, 1)
+    new = lambda *s: torch.ones(*s, device="cuda", dtype=torch.bfloat16)  # noqa: E731
+    a, b, c = new(8192, 4096), new(28672, 4096), new(8192, 14336)
+    x, res, gamma, out = new(148, 8192), new(148, 8192), new(8192), new(148, 8192)
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    start, gemm_end, norm_end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+    early = []
+    for _ in range(4):
+        torch.cuda.synchronize()
+        with torch.cuda.stream(one):
+            start.record()
+            gemm_bf16(a, b, out=c, swiglu=True)
+            gemm_end.record()
+        with torch.cuda.stream(two):
+            torch.cuda._sleep(200000)  # some 0.1 ms of 1.3, so that the GEMM is there first
+            allreduce_residual_rmsnorm(comm, x, res, gamma, out=out)
+            norm_end.record()
+        torch.cuda.synchronize()
+        early.append(norm_end.elapsed_time(gemm_end) / start.elapsed_time(gemm_end))
+    comm.destroy()
+    assert max(early[1:]) > 0.5, early
+
+
+@gpu
 @pytest.mark.parametrize("tokens", [5, 300])
 def test_gemm_chain_captured(tokens):
     """Launches that come up early wait for the ones before: each operand and each output of a GEMM is written or read
