@@ -702,7 +702,7 @@ __device__ __forceinline__ void swiglu_and_store(const CUtensorMap* map, uint32_
   ptx::tmem_ld_32x32b_x16(gate, g[0]);
   ptx::tmem_ld_32x32b_x16(up, u[0]);
   uint8_t* buf = stage_take<NBUF>(stage, stage_it, lane);
-  ptx::tmem_ld_wait();
+  ptx::tmem_ld_wait_for(g[0], u[0]);
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
     if (h < 3) {
@@ -711,7 +711,7 @@ __device__ __forceinline__ void swiglu_and_store(const CUtensorMap* map, uint32_
     }
     stage_put(buf, lane, 2 * h, swiglu8(g[h & 1], u[h & 1]));
     stage_put(buf, lane, 2 * h + 1, swiglu8(g[h & 1] + 8, u[h & 1] + 8));
-    if (h < 3) ptx::tmem_ld_wait();
+    if (h < 3) ptx::tmem_ld_wait_for(g[(h + 1) & 1], u[(h + 1) & 1]);
   }
   stage_send(map, buf, col0, row0, inside, lane);
 }
