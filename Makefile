@@ -116,8 +116,8 @@ plugins/ucx/libuccl-net-ucx-fake.so: plugins/ucx/plugin.cc plugins/ucx/fake_ucp.
 	$(CXX) $(CXXFLAGS) -DUCCL_HAS_UCX=1 -Iplugins/ucx/fake_ucp -shared plugins/ucx/plugin.cc plugins/ucx/fake_ucp.cc -o $@
 ucx-fake: plugins/ucx/libuccl-net-ucx-fake.so
 
-$(SELFTEST): tests/native/selftest.cc tests/native/uccl_selftest.h $(LIB) $(wildcard include/*.h csrc/*/*.h)
-	$(CXX) $(CXXFLAGS) -Itests/native -shared $< -o $@ -L$(PKG) -luccl -Wl,-rpath,'$$ORIGIN/../../$(PKG)'
+$(SELFTEST): tests/native/selftest.cc tests/native/local_copy_test.cc csrc/core/local_copy.cc tests/native/uccl_selftest.h $(LIB) $(wildcard include/*.h csrc/*/*.h)
+	$(CXX) $(CXXFLAGS) -Itests/native -shared $(filter tests/native/%.cc,$^) -o $@ -L$(PKG) -luccl -Wl,-rpath,'$$ORIGIN/../../$(PKG)'
 
 $(DEVTEST): tests/native/rma_device_test.cu tests/native/swiglu_device_test.cu include/uccl_device.cuh include/uccl.h csrc/kernels/swiglu.cuh $(LIB)
 	$(NVCC) $(NVFLAGS) -shared $(filter %.cu,$^) -o $@ -L$(PKG) -luccl -Xlinker -rpath,'$$ORIGIN/../../$(PKG)' -lcudart_static
@@ -142,7 +142,7 @@ endif
 # plugin loader, ring schedules, tuner, groups, CPU collectives) as a plain executable.
 SAN_FLAGS_asan := -fsanitize=address,undefined -fno-omit-frame-pointer
 SAN_FLAGS_tsan := -fsanitize=thread
-SAN_SRCS := $(CC_SRCS) tests/native/selftest.cc tests/native/selftest_main.cc
+SAN_SRCS := $(CC_SRCS) tests/native/selftest.cc tests/native/local_copy_test.cc tests/native/selftest_main.cc
 
 define SAN_RULES
 $(BUILD)/$(1)/%.o: %.cc $$(wildcard include/*.h csrc/*/*.h tests/native/*.h)

@@ -18,7 +18,6 @@
 #include "../host/host_coll.h"
 #include "../kernels/coll_device_types.h"
 #include "../kernels/collectives.cuh"
-#include "cuda_driver.h"
 #include "log.h"
 #include "trace.h"
 
@@ -394,42 +393,6 @@ ucclResult_t a2aDirect(Comm* c, const CollOp& op, size_t chunk, const TuneChoice
     a.chunkBytes = a.userBytes = len;
     ucclResult_t r = launch(c, KERN_A2A_PULL, a, blocks, op.stream);
     if (r != ucclSuccess) return r;
-  }
-  return ucclSuccess;
-}
-
-// Whether [p, p + bytes) is memory that a kernel on this GPU may read and write: in one allocation of its own.
-bool ownMemory(const Comm* c, const void* p, size_t bytes) {
-  const DriverApi& d = driverApi();
-  if (!d.ok) return false;
-  unsigned type = 0, managed = 1, flags = 0;
-  int device = -1;
-  CUdeviceptr start = 0;
-  size_t size = 0;
-  CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
-                                CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
-  void* to[] = {&type, &managed, &device, &start, &size, &flags};
-  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
-  if (d.pointerGetAttributes(6, what, to, at) != CUDA_SUCCESS) return false;
-  return type == CU_MEMORYTYPE_DEVICE && managed == 0 && device == c->cudaDev && flags == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE && at >= start &&
-         size >= bytes && at - start <= size - bytes;
-}
-
-// A kernel where nothing speaks against it: it costs the host less than cudaMemcpyAsync and comes up while the launch
-// before ends.  The runtime's copy takes what is not 16-byte aligned, other memory than this GPU's (which it may refuse), and
-// all of it where the communicator's CTAs are limited or its data are to go by copy engines.
-ucclResult_t localCopy(Comm* c, const void* src, void* dst, size_t bytes, cudaStream_t s) {
-  if (src == dst || bytes == 0) return ucclSuccess;
-  const bool free = c->nRanks == 1 && c->forcedBlocks <= 0 && c->cfg.maxCtas <= 0 && c->cfg.execMode == EXEC_SM_ONLY;
-  if (free && aligned16(src) && aligned16(dst) && ownMemory(c, src, bytes) && ownMemory(c, dst, bytes)) {
-    const cudaError_t e = launchLocalCopy(src, dst, bytes, s);
-    if (e == cudaSuccess) return ucclSuccess;
-    commSetError(c, "copy kernel launch failed: %s", cudaGetErrorString(e));
-    return ucclSystemError;
-  }
-  if (cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
-    commSetError(c, "cudaMemcpyAsync failed: %s", cudaGetErrorString(cudaGetLastError()));
-    return ucclSystemError;
   }
   return ucclSuccess;
 }

@@ -36,6 +36,9 @@ TuneChoice chooseFor(Comm* c, ucclCollKind_t kind, size_t bytes, bool symmetric,
 // Staging area inside the arena.
 size_t stagingOffset(const Comm* c);
 
+// Copy within this GPU (local_copy.cc).
+ucclResult_t localCopy(Comm* c, const void* src, void* dst, size_t bytes, cudaStream_t s);
+
 // device-side algorithms that live in their own translation units
 ucclResult_t enqueueRing(Comm* c, const CollOp& op, ucclProto_t proto, int blocks);
 ucclResult_t enqueueCopyEngine(Comm* c, const CollOp& op);

@@ -29,6 +29,7 @@
 #include "core/tuner.h"
 
 namespace uccl {
+std::string testLocalCopy();  // local_copy_test.cc
 namespace {
 
 std::string fmt(const char* f, ...) {
@@ -775,6 +776,7 @@ struct Case {
 };
 const std::vector<Case>& cases() {
   static const std::vector<Case> all = {
+      {"local_copy", testLocalCopy},
       {"proxy_in_order", testProxyInOrder},
       {"proxy_immediate_completion", testProxyImmediateCompletion},
       {"proxy_busy_and_signal", testProxyBusyAndSignal},
