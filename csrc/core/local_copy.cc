@@ -7,19 +7,24 @@ namespace uccl {
 
 namespace {
 
-// Whether [p, p + bytes) is memory that a kernel on this GPU may read and write: in one allocation of its own.
+// Whether [p, p + bytes) is memory that a kernel on this GPU may read and write: in one allocation of its own, made in the
+// context that the launch goes to (memory that is mapped by address belongs to no context).  Another context's memory is
+// mapped for that one alone; the runtime's copy looks contexts up by the address.
 bool ownMemory(const Comm* c, const void* p, size_t bytes) {
   const DriverApi& d = driverApi();
   if (!d.ok) return false;
   unsigned type = 0, managed = 1, flags = 0;
   int device = -1;
+  CUcontext owner = nullptr, current = nullptr;
   CUdeviceptr start = 0;
   size_t size = 0;
   CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
-                                CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
-  void* to[] = {&type, &managed, &device, &start, &size, &flags};
+                                CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS,
+                                CU_POINTER_ATTRIBUTE_CONTEXT};
+  void* to[] = {&type, &managed, &device, &start, &size, &flags, &owner};
   const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
-  if (d.pointerGetAttributes(6, what, to, at) != CUDA_SUCCESS) return false;
+  if (d.pointerGetAttributes(7, what, to, at) != CUDA_SUCCESS || d.ctxGetCurrent(&current) != CUDA_SUCCESS) return false;
+  if (owner != nullptr && owner != current) return false;
   return type == CU_MEMORYTYPE_DEVICE && managed == 0 && device == c->cudaDev && flags == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE && at >= start &&
          size >= bytes && at - start <= size - bytes;
 }

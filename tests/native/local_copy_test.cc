@@ -12,6 +12,7 @@ namespace {
 struct World {
   unsigned type = CU_MEMORYTYPE_DEVICE, managed = 0, access = CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE;
   int device = 3;
+  uintptr_t owner = 7, current = 7;  // contexts
   uintptr_t start = 0x10000;  // of the one allocation that there is
   size_t size = 4096;
   cudaError_t launch = cudaSuccess, copy = cudaSuccess;
@@ -28,15 +29,21 @@ CUresult fakePointerGetAttributes(unsigned n, CUpointer_attribute* what, void** 
       case CU_POINTER_ATTRIBUTE_RANGE_START_ADDR: *static_cast<CUdeviceptr*>(to[i]) = world.start; break;
       case CU_POINTER_ATTRIBUTE_RANGE_SIZE: *static_cast<size_t*>(to[i]) = world.size; break;
       case CU_POINTER_ATTRIBUTE_ACCESS_FLAGS: *static_cast<unsigned*>(to[i]) = world.access; break;
+      case CU_POINTER_ATTRIBUTE_CONTEXT: *static_cast<CUcontext*>(to[i]) = reinterpret_cast<CUcontext>(world.owner); break;
       default: return CUDA_ERROR_INVALID_VALUE;
     }
   }
+  return CUDA_SUCCESS;
+}
+CUresult fakeCtxGetCurrent(CUcontext* c) {
+  *c = reinterpret_cast<CUcontext>(world.current);
   return CUDA_SUCCESS;
 }
 const DriverApi& fakeDriverApi() {
   static DriverApi api;
   api.ok = true;
   api.pointerGetAttributes = fakePointerGetAttributes;
+  api.ctxGetCurrent = fakeCtxGetCurrent;
   return api;
 }
 cudaError_t fakeLaunch(const void*, void*, size_t, cudaStream_t) { return ++world.launches, world.launch; }
@@ -76,6 +83,8 @@ std::string testLocalCopy() {
   expect("host memory", 0, 1, ucclSuccess, [](Comm&) { world.type = CU_MEMORYTYPE_HOST; });
   expect("managed memory", 0, 1, ucclSuccess, [](Comm&) { world.managed = 1; });
   expect("another GPU's memory", 0, 1, ucclSuccess, [](Comm&) { world.device = 2; });
+  expect("another context's memory", 0, 1, ucclSuccess, [](Comm&) { world.owner = 8; });
+  expect("memory of no context", 1, 0, ucclSuccess, [](Comm&) { world.owner = 0; });
   expect("read-only memory", 0, 1, ucclSuccess, [](Comm&) { world.access = CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READ; });
   expect("limited CTAs", 0, 1, ucclSuccess, [](Comm& c) { c.forcedBlocks = 2; });
   expect("limited CTAs of the configuration", 0, 1, ucclSuccess, [](Comm& c) { c.cfg.maxCtas = 2; });
