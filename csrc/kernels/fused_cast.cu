@@ -17,6 +17,8 @@
 // input; half as many in the one-rank kernel, whose pieces are twice as long), which makes the block's amax a shuffle reduction.
 #include <type_traits>
 
+#include <algorithm>
+
 #include "coll_device.cuh"
 #include "collectives.cuh"
 #include "fp8_cast.cuh"
@@ -139,6 +141,7 @@ struct CastLocalArgs {
   size_t elems;  // a multiple of 16 input bytes, and of 128 for fp8 output
   float scale;
   int wide;      // both buffers are 32-byte aligned
+  int early;     // the launch behind this one may come up while it runs
 };
 
 constexpr int kCastThreads = 256;
@@ -253,7 +256,7 @@ template <int OUT>
 constexpr int kCastPieces = OUT == OUT_FP8 ? 2 : 4;
 template <int DT, int OUT, int U>
 __global__ void __launch_bounds__(kCastThreads, U == 2 ? 6 : 4) cast_local_kernel(const __grid_constant__ CastLocalArgs a) {
-  ptx::launch_dependents();
+  if (a.early) ptx::launch_dependents();
   ptx::wait_dependencies();
   cast_share<DT, OUT, U>(a, static_cast<size_t>(blockIdx.x) * (kCastThreads * U));
 }
@@ -262,14 +265,14 @@ __global__ void __launch_bounds__(kCastThreads, U == 2 ? 6 : 4) cast_local_kerne
 template <int DT, int OUT>
 __global__ void __launch_bounds__(kCastThreads, 4) cast_limited_kernel(const __grid_constant__ CastLocalArgs a) {
   constexpr size_t kShare = kCastThreads * 4, E = 32 / Vec<DT>::ES;
-  ptx::launch_dependents();
-  ptx::wait_dependencies();
   for (size_t first = blockIdx.x * kShare; first < (a.elems + E - 1) / E; first += gridDim.x * kShare) cast_share<DT, OUT, 4>(a, first);
 }
 
 }  // namespace dev
 
-// `limit`: the most CTAs the launch may have, 0 for none
+// `limit`: the most CTAs the launch may have, 0 for none.  A limit is there to keep SMs free for other work, so no launch under
+// one comes up beside the launch before, nor lets the one behind it come up early: that would hold room on the SMs for as long
+// as the limited launch takes.
 template <int DT, int OUT>
 static cudaError_t launchLocal(const dev::CastLocalArgs& a, int limit, cudaStream_t s) {
   const size_t pieces = (a.elems + 32 / dev::Vec<DT>::ES - 1) / (32 / dev::Vec<DT>::ES);
@@ -279,7 +282,12 @@ static cudaError_t launchLocal(const dev::CastLocalArgs& a, int limit, cudaStrea
   constexpr int U = dev::kCastPieces<OUT>;
   const bool many = pieces >= static_cast<size_t>(deviceSmCount()) * 4 * T * 4;
   const size_t share = many ? U * T : T, ctas = (pieces + share - 1) / share;
-  if (limit > 0 && ctas > static_cast<size_t>(limit)) return launchOverlapped(dev::cast_limited_kernel<DT, OUT>, limit, T, 0, s, a);
+  if (limit > 0) {
+    void (*kern)(dev::CastLocalArgs) = many ? dev::cast_local_kernel<DT, OUT, U> : dev::cast_local_kernel<DT, OUT, 1>;
+    if (ctas > static_cast<size_t>(limit)) kern = dev::cast_limited_kernel<DT, OUT>;
+    kern<<<static_cast<unsigned>(std::min<size_t>(ctas, limit)), T, 0, s>>>(a);
+    return cudaGetLastError();
+  }
   if (many) return launchOverlapped(dev::cast_local_kernel<DT, OUT, U>, static_cast<unsigned>(ctas), T, 0, s, a);
   return launchOverlapped(dev::cast_local_kernel<DT, OUT, 1>, static_cast<unsigned>(ctas), T, 0, s, a);
 }
@@ -314,6 +322,7 @@ cudaError_t launchCastKernel(const CastArgs& a, int limit, cudaStream_t s) {
   l.outScales = a.outScales;
   l.elems = a.chunkElems;
   l.scale = a.scale;
+  l.early = limit <= 0;
   l.wide = ((reinterpret_cast<uintptr_t>(l.in) | reinterpret_cast<uintptr_t>(l.out)) & 31) == 0;
   switch (a.inType) {
     case ucclFloat16: return launchLocalOut<dev::DT_F16>(l, a.outType, limit, s);

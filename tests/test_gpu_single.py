@@ -99,6 +99,78 @@ def test_cast_single_rank_keeps_to_its_ctas(din, dout):
     comm.destroy()
 
 
+def _edge_types(calls):
+    """What connects the kernels of these calls in a captured graph: 0 a full dependency, 1 one that lets the second come up early."""
+    import ctypes
+
+    cu = ctypes.CDLL("libcuda.so.1")
+    side = torch.cuda.Stream()
+    stream, graph, n = ctypes.c_void_p(side.cuda_stream), ctypes.c_void_p(), ctypes.c_size_t(16)
+    torch.cuda.synchronize()
+    assert cu.cuStreamBeginCapture_v2(stream, 2) == 0
+    with torch.cuda.stream(side):
+        for call in calls:
+            call()
+    assert cu.cuStreamEndCapture(stream, ctypes.byref(graph)) == 0
+    ends, data = [(ctypes.c_void_p * 16)() for _ in range(2)], (ctypes.c_ubyte * 8 * 16)()  # CUgraphEdgeData: its third byte is the type
+    assert cu.cuGraphGetEdges_v2(graph, ends[0], ends[1], data, ctypes.byref(n)) == 0
+    cu.cuGraphDestroy(graph)
+    return [data[i][2] for i in range(n.value)]
+
+
+@gpu
+def test_limited_casts_do_not_come_up_early():
+    """Under a limit on the CTAs, at once or in rounds, a cast starts after the launch before it has ended; without one it may
+    come up before."""
+    import os
+
+    from unified_ccl_b200 import Communicator
+
+    os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    comm = Communicator(0, 1)
+    x, y = torch.ones(1 << 16, device="cuda"), torch.empty(1 << 16, device="cuda", dtype=torch.bfloat16)
+    cast = lambda: comm.reduce_scatter_cast(x, y, 0.5)  # noqa: E731
+    for blocks, kind in ((0, 1), (2, 0), (48, 0)):  # 32 CTAs of their own, two, 32
+        comm.set_blocks(blocks)
+        cast()
+        assert _edge_types([cast] * 3) == [kind] * 2, blocks
+    comm.destroy()
+
+
+@gpu
+def test_limited_cast_keeps_sms_free():
+    """While a cast on two CTAs runs, the GEMM behind it does not wait on the SMs' shared memory: a GEMM of another stream runs
+    and ends long before the cast does."""
+    import os
+
+    from unified_ccl_b200 import Communicator
+    from unified_ccl_b200.ops import gemm_bf16
+
+    os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    comm = Communicator(0, 1)
+    comm.set_blocks(2)
+    x, y = torch.ones(1 << 26, device="cuda"), torch.empty(1 << 26, device="cuda", dtype=torch.bfloat16)
+    a, c, d = (torch.ones(4096, 4096, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    start, cast_end, other_end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+    early = []
+    for _ in range(4):
+        torch.cuda.synchronize()
+        with torch.cuda.stream(one):
+            start.record()
+            comm.reduce_scatter_cast(x, y, 0.5)
+            gemm_bf16(a, a, out=c)
+            cast_end.record()
+        with torch.cuda.stream(two):
+            torch.cuda._sleep(200000)  # some 0.1 ms, so that the first stream's launches are all there
+            gemm_bf16(a, a, out=d)
+            other_end.record()
+        torch.cuda.synchronize()
+        early.append(other_end.elapsed_time(cast_end) / start.elapsed_time(cast_end))
+    comm.destroy()
+    assert max(early[1:]) > 0.5, early
+
+
 def _kernel_events(prof):
     import json
     import tempfile
