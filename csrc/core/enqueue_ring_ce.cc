@@ -31,8 +31,9 @@ int devDtype(ucclDataType_t dt) {
   return dt == ucclFloat16 ? DEVDT_F16 : (dt == ucclBfloat16 ? DEVDT_BF16 : DEVDT_F32);
 }
 
-ucclResult_t cudaFail(Comm* c, const char* what) {
-  commSetError(c, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
+// A launcher hands the error over that it has cleared.
+ucclResult_t cudaFail(Comm* c, const char* what, cudaError_t e = cudaGetLastError()) {
+  commSetError(c, "%s: %s", what, cudaGetErrorString(e));
   return ucclSystemError;
 }
 
@@ -201,7 +202,8 @@ ucclResult_t localReduce(Comm* c, char* dst, const char* slots, int nslots, size
   a.userBytes = bytes;
   a.root = nslots;
   int blocks = static_cast<int>(std::min<size_t>(32, std::max<size_t>(1, bytes / (256u << 10))));
-  if (launchCollKernel(KERN_LOCAL_REDUCE, a, blocks, s) != cudaSuccess) return cudaFail(c, "reduce kernel launch");
+  const cudaError_t e = launchCollKernel(KERN_LOCAL_REDUCE, a, blocks, s);
+  if (e != cudaSuccess) return cudaFail(c, "reduce kernel launch", e);
   return ucclSuccess;
 }
 
@@ -217,7 +219,8 @@ ucclResult_t enqueueBarrier(Comm* c, cudaStream_t s) {
   CollArgs a;
   memset(&a, 0, sizeof(a));
   a.dc = c->dev;
-  if (launchCollKernel(KERN_BARRIER, a, 1, s) != cudaSuccess) return cudaFail(c, "barrier kernel launch");
+  const cudaError_t e = launchCollKernel(KERN_BARRIER, a, 1, s);
+  if (e != cudaSuccess) return cudaFail(c, "barrier kernel launch", e);
   return ucclSuccess;
 }
 

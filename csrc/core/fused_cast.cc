@@ -92,8 +92,10 @@ extern "C" ucclResult_t ucclReduceScatterEx(const void* sendbuff, void* recvbuff
     a.chunkElems = recvcount;
     a.out = static_cast<char*>(recvbuff);
     a.outScales = blockScales;
-    if (launchCastKernel(a, limit, s) != cudaSuccess) return ucclSystemError;
-    return ucclSuccess;
+    const cudaError_t e = launchCastKernel(a, limit, s);
+    if (e == cudaSuccess) return ucclSuccess;
+    commSetError(c, "cast kernel launch failed: %s", cudaGetErrorString(e));
+    return ucclSystemError;
   }
   int blocks = limit > 0 ? std::min(limit, kMaxBlocks) : kMaxBlocks;
   blocks = static_cast<int>(std::max<size_t>(1, std::min<size_t>(blocks, (recvcount + 4095) / 4096)));
@@ -107,8 +109,9 @@ extern "C" ucclResult_t ucclReduceScatterEx(const void* sendbuff, void* recvbuff
     a.chunkElems = recvcount;
     a.out = static_cast<char*>(recvbuff);
     a.outScales = blockScales;
-    if (launchReduceCastKernel(a, blocks, s) != cudaSuccess) {
-      commSetError(c, "kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+    const cudaError_t e = launchReduceCastKernel(a, blocks, s);
+    if (e != cudaSuccess) {
+      commSetError(c, "cast kernel launch failed: %s", cudaGetErrorString(e));
       return ucclSystemError;
     }
     return ucclSuccess;
@@ -131,8 +134,9 @@ extern "C" ucclResult_t ucclReduceScatterEx(const void* sendbuff, void* recvbuff
     a.chunkElems = len;
     a.out = static_cast<char*>(recvbuff) + eo * outEs;
     a.outScales = blockScales ? blockScales + eo / 128 : nullptr;
-    if (launchReduceCastKernel(a, blocks, s) != cudaSuccess) {
-      commSetError(c, "kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+    const cudaError_t e = launchReduceCastKernel(a, blocks, s);
+    if (e != cudaSuccess) {
+      commSetError(c, "cast kernel launch failed: %s", cudaGetErrorString(e));
       return ucclSystemError;
     }
   }

@@ -147,8 +147,9 @@ extern "C" ucclResult_t ucclAllReduceResidualRMSNorm(const void* x, const void* 
     a.dc.nranks = 1;
     a.inUser = static_cast<const char*>(x);
     a.resOutUser = static_cast<char*>(residualOut);
-    if (launchArNormKernel(a, 0, s) != cudaSuccess) {
-      commSetError(c, "norm kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+    const cudaError_t e = launchArNormKernel(a, 0, s);
+    if (e != cudaSuccess) {
+      commSetError(c, "norm kernel launch failed: %s", cudaGetErrorString(e));
       return ucclSystemError;
     }
     return ucclSuccess;
@@ -184,8 +185,9 @@ extern "C" ucclResult_t ucclAllReduceResidualRMSNorm(const void* x, const void* 
   int blocks = c->cfg.maxCtas > 0 ? std::min(c->cfg.maxCtas, kMaxBlocks) : kMaxBlocks;
   if (c->forcedBlocks > 0) blocks = std::min(c->forcedBlocks, kMaxBlocks);
   blocks = std::min(blocks, std::max(1, (tokens + n - 1) / n));
-  if (launchArNormKernel(a, blocks, s) != cudaSuccess) {
-    commSetError(c, "fused norm kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+  const cudaError_t e = launchArNormKernel(a, blocks, s);
+  if (e != cudaSuccess) {
+    commSetError(c, "fused norm kernel launch failed: %s", cudaGetErrorString(e));
     return ucclSystemError;
   }
   return ucclSuccess;

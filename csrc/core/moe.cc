@@ -193,8 +193,9 @@ extern "C" ucclResult_t ucclMoeDispatch(ucclMoeContext_t m, const void* x, const
   a.topkIdx = topkIdx;
   m->lastTokens = tokens;
   commCount(c, ucclCollAllToAll, static_cast<size_t>(tokens) * m->topk * (m->hidden + m->hidden / 32), ucclAlgoTwoShot);
-  if (launchMoeDispatch(a, s) != cudaSuccess) {
-    commSetError(c, "MoE dispatch launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+  const cudaError_t e = launchMoeDispatch(a, s);
+  if (e != cudaSuccess) {
+    commSetError(c, "MoE dispatch launch failed: %s", cudaGetErrorString(e));
     return ucclSystemError;
   }
   return ucclSuccess;
@@ -215,8 +216,9 @@ extern "C" ucclResult_t ucclMoeCombine(ucclMoeContext_t m, const float* topkWeig
   a.topkWeight = topkWeight;
   a.out = out;
   commCount(c, ucclCollAllToAll, static_cast<size_t>(tokens) * m->topk * m->hidden * 2, ucclAlgoTwoShot);
-  if (launchMoeCombine(a, s) != cudaSuccess) {
-    commSetError(c, "MoE combine launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+  const cudaError_t e = launchMoeCombine(a, s);
+  if (e != cudaSuccess) {
+    commSetError(c, "MoE combine launch failed: %s", cudaGetErrorString(e));
     return ucclSystemError;
   }
   // peers have finished pulling from this rank before expertOut is overwritten

@@ -298,8 +298,9 @@ extern "C" ucclResult_t ucclSignal(int peer, int sigIdx, int ctx, unsigned int f
   UCCL_LOG(TRACE, "ucclSignal peer=%d window=%d", peer, w->slot);
   DeviceGuard guard(c->cudaDev);
   const int lp = c->peers[peer].localRank;
-  if (launchRmaSignal(w->remoteSignals[lp] + c->localRank, static_cast<cudaStream_t>(stream)) != cudaSuccess) {
-    commSetError(c, "signal kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+  const cudaError_t e = launchRmaSignal(w->remoteSignals[lp] + c->localRank, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) {
+    commSetError(c, "signal kernel launch failed: %s", cudaGetErrorString(e));
     return ucclSystemError;
   }
   return ucclSuccess;
@@ -327,8 +328,9 @@ extern "C" ucclResult_t ucclWaitSignal(int nDesc, ucclWaitSignalDesc_t* signalDe
   }
   UCCL_LOG(TRACE, "ucclWaitSignal n=%d", nDesc);
   DeviceGuard guard(c->cudaDev);
-  if (launchRmaWait(a, static_cast<cudaStream_t>(stream)) != cudaSuccess) {
-    commSetError(c, "wait kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+  const cudaError_t e = launchRmaWait(a, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) {
+    commSetError(c, "wait kernel launch failed: %s", cudaGetErrorString(e));
     return ucclSystemError;
   }
   return ucclSuccess;

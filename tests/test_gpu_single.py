@@ -99,6 +99,49 @@ def test_cast_single_rank_keeps_to_its_ctas(din, dout):
     comm.destroy()
 
 
+@gpu
+def test_refused_launches_say_why():
+    """A launch that the driver refuses (its stream is in a capture that has been invalidated, an error of the host alone) fails
+    the call, and the communicator's last error names the driver's reason."""
+    import ctypes
+    import os
+
+    from unified_ccl_b200 import Communicator
+    from unified_ccl_b200.parallel import MoeDispatcher, allreduce_residual_rmsnorm
+
+    os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    cu = ctypes.CDLL("libcuda.so.1")
+    comm = Communicator(0, 1)
+    disp = MoeDispatcher(comm, 8, 256, 4, 2)
+    x, res, out, out2 = (torch.ones(8, 256, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    gamma, w = torch.ones(256, device="cuda", dtype=torch.bfloat16), torch.ones(8, 2, device="cuda")
+    idx, f32 = torch.zeros(8, 2, device="cuda", dtype=torch.int32), torch.ones(2048, device="cuda")
+    calls = {
+        "norm": lambda: allreduce_residual_rmsnorm(comm, x, res, gamma, out=out, residual_out=out2),
+        "cast": lambda: comm.reduce_scatter_cast(x.view(-1), f32, 0.5),
+        "dispatch": lambda: disp.dispatch(x, idx),
+        "combine": lambda: disp.combine(w, out=out),
+        "Memcpy": lambda: comm.allgather(x, out),
+    }
+    for blocks in (0, 1):
+        comm.set_blocks(blocks)
+        for name, call in calls.items():
+            call()  # the kernel is loaded now
+            torch.cuda.synchronize()
+            side = torch.cuda.Stream()
+            stream, graph = ctypes.c_void_p(side.cuda_stream), ctypes.c_void_p()
+            assert cu.cuStreamBeginCapture_v2(stream, 2) == 0  # CU_STREAM_CAPTURE_MODE_RELAXED
+            assert cu.cuStreamQuery(stream) == 900             # CUDA_ERROR_STREAM_CAPTURE_UNSUPPORTED: ends the capture's validity
+            with torch.cuda.stream(side), pytest.raises(RuntimeError):
+                call()
+            assert cu.cuStreamEndCapture(stream, ctypes.byref(graph)) == 901  # CUDA_ERROR_STREAM_CAPTURE_INVALIDATED
+            assert name in comm.last_error() and "capture" in comm.last_error(), (name, comm.last_error())
+            call()
+    torch.cuda.synchronize()
+    disp.close()
+    comm.destroy()
+
+
 def _edge_types(calls):
     """What connects the kernels of these calls in a captured graph: 0 a full dependency, 1 one that lets the second come up early."""
     import ctypes
