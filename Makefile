@@ -159,6 +159,6 @@ $(eval $(call SAN_RULES,asan))
 $(eval $(call SAN_RULES,tsan))
 
 clean:
-	rm -rf $(BUILD) $(LIB) $(PYMOD) $(PLUGIN) $(SELFTEST) $(DEVTEST) $(CLIENT) $(BASELINE) plugins/ucx/*.so
+	rm -rf $(BUILD) $(LIB) $(PYMOD) $(TENSORMOD) $(PLUGIN) $(SELFTEST) $(DEVTEST) $(CLIENT) $(BASELINE) plugins/ucx/*.so
 
 .PHONY: all clean asan tsan install ucx-fake

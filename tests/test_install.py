@@ -30,3 +30,13 @@ def test_make_install_and_link_a_client(tmp_path):
     env = dict(os.environ, UCCL_BACKEND="cpu", UCCL_BOOTSTRAP_IFNAME="lo")
     p = subprocess.run([str(exe), "initall", "2"], env=env, capture_output=True, timeout=120)
     assert p.returncode == 0 and p.stdout.count(b"ok") == 2, (p.stdout[-500:], p.stderr[-1500:])
+
+
+def test_clean_names_all_that_is_built():
+    """`make clean` leaves no library behind that Python would still import."""
+    if shutil.which("make") is None:
+        pytest.skip("no make")
+    p = subprocess.run(["make", "-C", ROOT, "-n", "clean"], capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]
+    for name in ("libuccl.so", "_uccl_bindings", "_uccl_tensor_calls", "libuccl_selftest.so", "libuccl_devtest.so", "libbaseline_swiglu.so"):
+        assert name in p.stdout, name
