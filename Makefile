@@ -49,6 +49,8 @@ ifeq ($(UCCL_BUILD_PYTHON),1)
 PYINC     := $(shell $(PYTHON) -c "import sysconfig; print(sysconfig.get_paths()['include'])")
 PYBINDINC := $(shell $(PYTHON) -c "import pybind11; print(pybind11.get_include())")
 TORCHDIR  := $(shell $(PYTHON) -c "import importlib.util as u; s = u.find_spec('torch'); print(s.submodule_search_locations[0] if s else '')")
+# what the tensor-call module is built against, and refuses to be loaded into another than
+TORCHVER  := $(shell $(PYTHON) -c "import runpy; v = runpy.run_path('$(TORCHDIR)/version.py'); print(v['__version__'] + '_' + str(v['git_version']))" 2>/dev/null)
 EXTSUFFIX := $(shell $(PYTHON) -c "import sysconfig; print(sysconfig.get_config_var('EXT_SUFFIX'))")
 endif
 LIB       := $(PKG)/libuccl.so
@@ -100,8 +102,10 @@ $(PYMOD): csrc/python/bindings.cc $(LIB) $(wildcard include/*.h)
 	$(CXX) $(CXXFLAGS) -fvisibility=hidden -I$(PYINC) -I$(PYBINDINC) -shared $< -o $@ \
 	    -L$(PKG) -luccl -Wl,-rpath,'$$ORIGIN'
 
-$(TENSORMOD): csrc/python/tensor_calls.cc $(LIB) $(wildcard include/*.h)
-	$(CXX) $(filter-out -g,$(CXXFLAGS)) -fvisibility=hidden -I$(PYINC) -isystem $(TORCHDIR)/include -isystem $(TORCHDIR)/include/torch/csrc/api/include \
+$(BUILD)/torch-$(TORCHVER):
+	@mkdir -p $(BUILD) && touch $@
+$(TENSORMOD): csrc/python/tensor_calls.cc $(LIB) $(wildcard include/*.h) $(BUILD)/torch-$(TORCHVER)
+	$(CXX) $(filter-out -g,$(CXXFLAGS)) -fvisibility=hidden -DUCCL_TORCH_VERSION='"$(TORCHVER)"' -I$(PYINC) -isystem $(TORCHDIR)/include -isystem $(TORCHDIR)/include/torch/csrc/api/include \
 	    -shared $< -o $@ -L$(PKG) -luccl -L$(TORCHDIR)/lib -ltorch_python -ltorch_cpu -lc10 -Wl,-rpath,'$$ORIGIN'
 
 $(PLUGIN): plugins/sample/plugin.cc include/uccl_net.h include/uccl.h

@@ -269,9 +269,25 @@ PyMethodDef methods[] = {method<gemm>("gemm"), method<norm>("norm"), method<redu
                          method<moeDispatch>("moe_dispatch"), method<moeCombine>("moe_combine"), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_uccl_tensor_calls", "Per-step calls on torch tensors", -1, methods, nullptr, nullptr, nullptr, nullptr};
 
+// The layout of a tensor is compiled in.  A torch that was exchanged after the build may have another one and all the symbols.
+bool builtForThisTorch() {
+  PyObject* v = PyImport_ImportModule("torch.version");
+  PyObject* number = v ? PyObject_GetAttrString(v, "__version__") : nullptr;
+  PyObject* git = number ? PyObject_GetAttrString(v, "git_version") : nullptr;
+  PyObject* here = git ? PyUnicode_FromFormat("%S_%S", number, git) : nullptr;
+  const bool same = here && PyUnicode_CompareWithASCIIString(here, UCCL_TORCH_VERSION) == 0;
+  if (here && !same) PyErr_Format(PyExc_ImportError, "built for torch %s, this is %U", UCCL_TORCH_VERSION, here);
+  Py_XDECREF(here);
+  Py_XDECREF(git);
+  Py_XDECREF(number);
+  Py_XDECREF(v);
+  return same;
+}
+
 }  // namespace
 
 PyMODINIT_FUNC PyInit__uccl_tensor_calls() {
+  if (!builtForThisTorch()) return nullptr;
   PyObject* bindings = PyImport_ImportModule("unified_ccl_b200._uccl_bindings");
   PyObject* torch = bindings ? PyImport_ImportModule("torch._C") : nullptr;
   if (torch) {

@@ -116,3 +116,20 @@ def test_taken_calls_equal_the_general_path(monkeypatch):
         gone.reduce_scatter(f32, f32)
     disp.close()
     comm.destroy()
+
+
+@pytest.mark.parametrize("name,value", [("__version__", "2.10.0+cu128"), ("git_version", "0" * 40)])
+def test_module_of_another_torch_is_not_loaded(name, value):
+    """Into a torch other than the one that it was built for the native module does not load, and says so once."""
+    import subprocess
+
+    code = (f"import warnings, torch; torch.version.{name} = {value!r}\n"
+            "with warnings.catch_warnings(record=True) as w:\n"
+            "    warnings.simplefilter('always')\n"
+            "    from unified_ccl_b200 import communicator\n"
+            "assert communicator.tensor_calls is communicator._GeneralPath\n"
+            f"assert len(w) == 1 and {value!r} in str(w[0].message), [str(x.message) for x in w]\n"
+            "assert 'unified_ccl_b200._uccl_tensor_calls' not in __import__('sys').modules\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]

@@ -11,6 +11,7 @@ communicator created with ``UCCL_BACKEND=cpu`` or on a machine without GPUs.
 import contextlib
 import os
 import threading
+import warnings
 
 import torch
 
@@ -23,17 +24,22 @@ current_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 class _GeneralPath:
-    """In the place of the native module where there is none (a torch without CUDA): no call is taken."""
+    """In the place of the native module where there is none (not built, a torch without CUDA or another than it was built for):
+    no call is taken."""
 
     gemm = norm = reduce_scatter = allgather = reduce_scatter_cast = allreduce_cast = moe_dispatch = moe_combine = staticmethod(lambda *args: False)
 
 
 # Calls on ordinary tensors, looked at and launched natively: 5.5 -> 2.9 us for a small residual + RMSNorm.  What they do
 # not take (they say so) goes on as written here.
-try:
-    from . import _uccl_tensor_calls as tensor_calls
-except ImportError:
-    tensor_calls = _GeneralPath
+tensor_calls = _GeneralPath
+if current_raw_stream is not None:
+    try:
+        from . import _uccl_tensor_calls as tensor_calls
+    except ModuleNotFoundError:
+        pass
+    except ImportError as why:
+        warnings.warn(f"calls on tensors take the slower general path: {why}")
 
 _DTYPES = {
     torch.float16: 0,
