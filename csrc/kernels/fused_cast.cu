@@ -141,7 +141,6 @@ struct CastLocalArgs {
   size_t elems;  // a multiple of 16 input bytes, and of 128 for fp8 output
   float scale;
   int wide;      // both buffers are 32-byte aligned
-  int early;     // the launch behind this one may come up while it runs
 };
 
 constexpr int kCastThreads = 256;
@@ -256,7 +255,7 @@ template <int OUT>
 constexpr int kCastPieces = OUT == OUT_FP8 ? 2 : 4;
 template <int DT, int OUT, int U>
 __global__ void __launch_bounds__(kCastThreads, U == 2 ? 6 : 4) cast_local_kernel(const __grid_constant__ CastLocalArgs a) {
-  if (a.early) ptx::launch_dependents();
+  ptx::launch_dependents();
   ptx::wait_dependencies();
   cast_share<DT, OUT, U>(a, static_cast<size_t>(blockIdx.x) * (kCastThreads * U));
 }
@@ -271,8 +270,8 @@ __global__ void __launch_bounds__(kCastThreads, 4) cast_limited_kernel(const __g
 }  // namespace dev
 
 // `limit`: the most CTAs the launch may have, 0 for none.  A limit is there to keep SMs free for other work, so no launch under
-// one comes up beside the launch before, nor lets the one behind it come up early: that would hold room on the SMs for as long
-// as the limited launch takes.
+// one comes up beside the launch before, and one that goes in rounds does not let the one behind it come up: that would hold
+// room on the SMs for as long as the rounds take.
 template <int DT, int OUT>
 static cudaError_t launchLocal(const dev::CastLocalArgs& a, int limit, cudaStream_t s) {
   const size_t pieces = (a.elems + 32 / dev::Vec<DT>::ES - 1) / (32 / dev::Vec<DT>::ES);
@@ -322,7 +321,6 @@ cudaError_t launchCastKernel(const CastArgs& a, int limit, cudaStream_t s) {
   l.outScales = a.outScales;
   l.elems = a.chunkElems;
   l.scale = a.scale;
-  l.early = limit <= 0;
   l.wide = ((reinterpret_cast<uintptr_t>(l.in) | reinterpret_cast<uintptr_t>(l.out)) & 31) == 0;
   switch (a.inType) {
     case ucclFloat16: return launchLocalOut<dev::DT_F16>(l, a.outType, limit, s);
