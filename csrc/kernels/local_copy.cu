@@ -49,8 +49,10 @@ template <int W>
 static cudaError_t launchCopy(const void* src, void* dst, size_t bytes, cudaStream_t s) {
   constexpr size_t T = dev::kCopyThreads;
   const size_t pieces = bytes / W;
-  // as the casts: four pieces per thread once that still gives every SM its CTAs
-  const bool four = pieces >= static_cast<size_t>(deviceSmCount()) * 8 * T * 4;
+  // Four pieces per thread once that still gives every SM the CTAs that it holds of this kernel (44 registers with 32-byte
+  // pieces, 28 with 16).  One piece and four, in us: 24 MiB 9.0 and 8.9, 28 MiB 10.1 and 10.0, 32 MiB 11.4 and 11.3.
+  constexpr int kResident = W == 32 ? 5 : 8;
+  const bool four = pieces >= static_cast<size_t>(deviceSmCount()) * kResident * T * 4;
   const size_t share = four ? 4 * T : T, ctas = std::max<size_t>(1, (pieces + share - 1) / share);
   if (ctas > 0x7fffffffu) return cudaErrorInvalidValue;
   const char* from = static_cast<const char*>(src);

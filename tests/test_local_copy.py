@@ -20,7 +20,7 @@ def _kernels(f):
 
 @gpu
 @pytest.mark.parametrize("count", [1, 15, 16, 31, 32, 33, 8191, 8192, 8193, 8225, 8192 * 32 + 7,  # around a piece and a CTA of pieces
-                                   148 * 8 * 256 * 4 * 16 - 32, 148 * 8 * 256 * 4 * 32 - 16, 148 * 8 * 256 * 4 * 32, 148 * 8 * 256 * 4 * 32 + 4097])  # of four pieces
+                                   148 * 8 * 256 * 4 * 16 - 32, 148 * 5 * 256 * 4 * 32 - 32, 148 * 5 * 256 * 4 * 32, 148 * 8 * 256 * 4 * 32 - 16, 148 * 8 * 256 * 4 * 32, 148 * 8 * 256 * 4 * 32 + 4097])  # of four pieces
 @pytest.mark.parametrize("src_off,dst_off", [(0, 0), (16, 0), (32, 64), (1, 0), (3, 8)])
 def test_one_rank_copy(count, src_off, dst_off):
     os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
