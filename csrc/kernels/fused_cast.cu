@@ -250,7 +250,8 @@ __device__ __forceinline__ void cast_share(const CastLocalArgs& a, size_t first)
 }
 // Pieces per thread of a large launch, and CTAs per SM.  A conversion to fp8 takes some hundred instructions a piece, and
 // two pieces on six CTAs put more of them beside other CTAs' loads than four pieces on four: 64 Mi bf16 33.0 -> 31.4 us, 16 Mi
-// 11.4 -> 10.1, 6 Mi fp32 6.7 -> 5.8; with the rest, bound by its loads and stores, it is the same.
+// 11.4 -> 10.1, 6 Mi fp32 6.7 -> 5.8; with the rest, bound by its loads and stores, it is the same.  Six CTAs leave 40 registers, and
+// 16-bit input spills 8 bytes; five (47 registers, no spill) are slower: 64 Mi bf16 31.1 and 31.5 us, 32 Mi fp32 25.3 and 26.4.
 template <int OUT>
 constexpr int kCastPieces = OUT == OUT_FP8 ? 2 : 4;
 template <int DT, int OUT, int U>

@@ -329,8 +329,9 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       // Single CTAs run the narrow tiles, whose four MMAs of a stage take about as long as the warp's wait for it, 200 cycles
       // also where there is nothing to wait for.  So the next stage's barrier is looked at while this one is issued, and no
       // branch parts the MMAs from the warp.  Device time back to back: 1 x 4096 x 14336 23.5 -> 22.4 us, 64 x 4096 x 14336
-      // 24.6 -> 23.7, 32 x 4096 x 4096 11.2 -> 10.6, 16 x 4096 x 1792 8.1 -> 7.8.  Pairs, whose MMAs are wider, gain and lose
-      // one or two percent by either and keep the plain form.
+      // 24.6 -> 23.7, 32 x 4096 x 4096 11.2 -> 10.6, 16 x 4096 x 1792 8.1 -> 7.8.  SwiGLU of a few rows with K below 600 loses by
+      // it: 8 x 512 x 256 3.09 -> 3.11 us, 32 x 1792 x 256 3.14 -> 3.16.  Pairs, whose MMAs are wider, gain and lose one or two
+      // percent by either and keep the plain form.
       const uint32_t idesc = ptx::umma_idesc_f16(1u, BM, static_cast<uint32_t>(a.bn));
       const uint32_t act = ptx::elect_one() ? 1u : 0u, ring = ptx::smem_u32(smem), base = __shfl_sync(0xffffffffu, tmem_base, 0);
       int s = 0;

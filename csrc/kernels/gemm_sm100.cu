@@ -147,19 +147,24 @@ bool usePairKernel() {
 // How to cut a GEMM without a collective: the candidate with the fewest cycles by one of two formulas.
 //
 // A tile whole: waves of tiles x the longer of a tile's main loop and of the epilogue that runs beside the next tile's
-// (2150 cycles, and per output column 11, or 49 with silu, which has become cheaper since); at least the time of memory, and
-// at least that of all loads together (9000 bytes per cycle into all SMs).  A stage of the main loop takes what the tensor
-// cores need for it (two cycles per accumulator column, at least a round trip of the ring) or its loads (65 bytes
-// per cycle and SM).  A tile in parts of K: the same without the overlapped epilogue (one tile per cluster), plus
-// the exchange of the parts.
+// (2150 cycles, and per output column 11, or 49 with silu); at least the time of memory, and at least that of all loads
+// together (9000 bytes per cycle into all SMs).  A stage of the main loop takes what the tensor cores need for it (two
+// cycles per accumulator column, at least a round trip of the ring) or its loads (65 bytes per cycle and SM).  A tile in
+// parts of K: the same without the overlapped epilogue (one tile per cluster), plus the exchange of the parts.
 //
 // The constants are fits to measurements with every candidate timed on operands that are not in L2: whole tiles to
 // 658 shapes (1 to 16384 rows, K of 64 to 14336), where the choice takes 1.2% more than the best candidate on average (an
 // earlier formula without the epilogue and the common load rate: 2.4%, and 20% on 4096 x 28672 x 512), the parts to 102
 // of them; with the issuer and the epilogue as they are now, the choice takes 0.6% more than the best candidate on 200
-// other shapes.  Both sides of some of the lines, in us: 64 x 4096 x 14336 25.3 in four parts of 128 columns, 62 uncut;
+// other shapes.  Both sides of some of the lines, in us, when they were fitted: 64 x 4096 x 14336 25.3 in four parts of 128 columns, 62 uncut;
 // 4096 x 28672 x 512 111 in pair tiles of 256, 125 of 224; 8192 x 3592 x 4104 207 in pair tiles of 256, 244 of 192;
 // 200 x 28672 x 4096 51.6 in pair tiles of 224, 60.2 in single CTAs of 208; 512 x 4096 x 4096 20 in tiles of 128, 25 of 256.
+//
+// The 49 cycles are those of the division that the epilogue once had.  The silu of today takes about 25 (4096 x 28672 x 64
+// 69 us, 16384 x 4096 x 128 40 us, both bound by it), and the fit has not been made anew.  What that costs, on 40 SwiGLU
+// shapes with K of 64 to 1024: 32 are cut as the best candidate and four more lose up to 2.1%; 2 x 12752 x 72 goes into two
+// parts and takes 6.5 us, 4.1 in whole tiles of 96; 10605 x 320 x 520 12.5 and 11.1, 1 x 1152 x 872 6.0 and 5.5, 9373 x 4208 x
+// 824 66.1 and 61.9.
 GemmCut choosePlain(int M, int N, int K, bool swiglu) {
   GemmCut best = {1, 256, 1};
   const bool pairs = usePairKernel();

@@ -6,9 +6,9 @@ namespace uccl {
 
 // Launches `kern`, which calls ptx::wait_dependencies before it touches memory, with programmatic serialization: its CTAs
 // start as soon as the kernel before has none left to start, and the launch's latency and their set-up go by while that
-// one ends.  About 2 us of a launch: residual + RMSNorm 8192 x 8192 82.7 -> 80.5 us, 7 rows of it 5.7 -> 5.0, MoE combine
-// 84.7 -> 82.8, 128 MiB cast to fp8 36.9 -> 35.5, an MoE layer of 96 tokens 28.3 -> 26.4.  A launch that was refused is
-// reported here and not by the thread's next one.
+// one ends.  0.7 to 2 us of a launch: residual + RMSNorm 8192 x 8192 82.7 -> 80.5 us, 7 rows of it 5.7 -> 5.0, an MoE layer of
+// 96 tokens (three launches) 28.3 -> 26.4.  The error of a launch that was refused is returned and cleared, so that the
+// thread's next launch does not report it.
 template <typename... Params, typename... Args>
 cudaError_t launchOverlapped(void (*kern)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, const Args&... args) {
   cudaLaunchConfig_t cfg = {};

@@ -326,8 +326,9 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// The same from a whole warp of which one lane (`act` != 0) issues.  With no branch around it the compiler keeps the
-// operands in uniform registers: four MMAs of 128 columns take 258 cycles, behind a branch 302 to 490.
+// The same from a whole warp of which one lane (`act` != 0) issues, with no branch around it: four MMAs of 128 columns took
+// 258 cycles, behind a branch 302 to 490.  (Perhaps because the operands then need not leave the uniform registers; that
+// has not been shown.)
 __device__ __forceinline__ void umma_f16_from(uint32_t act, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"

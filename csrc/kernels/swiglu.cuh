@@ -28,7 +28,7 @@ __device__ __forceinline__ float rcp_ftz(float x) {
 // A division as such has a slow path, and the branch to it ties each element to the one before: 49 cycles per column of a
 // warp.  Without a branch the elements of a register block overlap: SwiGLU 4096 x 28672 x 512 220 -> 101 us, 16384 x 4096
 // x 128 119 -> 47 us, 1212 x 10192 x 1760 40.3 -> 34.4 us, 64 x 28672 x 4096 (one tile per CTA, whose epilogue nothing
-// hides) 45.1 -> 40.3 us.
+// hides) 45.1 -> 40.3 us.  What the blocks are and what registers they cost stands with swiglu_and_store.
 // Signs: the negated reciprocal and quotient are carried, because the packed instructions cannot negate an operand.
 __device__ __forceinline__ float2 silu2_negated(float2 x) {
   const float2 p = ptx::mul2(x, make_float2(-1.4426950408889634f, -1.4426950408889634f));

@@ -76,7 +76,7 @@ def test_gemm_cuts(M, N, K, epilogue):
     ref = a.double() @ b.double().t()
     if epilogue:
         ref = torch.nn.functional.silu(ref[:, :n_out]) * ref[:, n_out:]
-    # one rounding to bf16 (2^-9 of the value), fp32 sums of K products of N(0, 1) x N(0, 0.02) numbers whose error
+    # one rounding to bf16 (2^-8 of the value), fp32 sums of K products of N(0, 1) x N(0, 0.02) numbers whose error
     # is below K * 2^-24 of their sum of magnitudes (K * 0.013), in the SwiGLU carried by factors of a few
     bound = ref.abs() * 2.0 ** -8 + K * 2.0 ** -24 * K * 0.013 * (8 if epilogue else 1) + 1e-6
     assert ((out.double() - ref).abs() <= bound).all()
