@@ -82,7 +82,8 @@ std::string testLocalCopy() {
   expect("destination ends beyond it", 0, 1, ucclSuccess, [](Comm&) {}, 0, 2049);
   expect("host memory", 0, 1, ucclSuccess, [](Comm&) { world.type = CU_MEMORYTYPE_HOST; });
   expect("managed memory", 0, 1, ucclSuccess, [](Comm&) { world.managed = 1; });
-  expect("another GPU's memory", 0, 1, ucclSuccess, [](Comm&) { world.device = 2; });
+  expect("another GPU's memory", 0, 1, ucclSuccess, [](Comm&) { world.device = 2, world.owner = 8; });
+  expect("another GPU's memory of no context", 0, 1, ucclSuccess, [](Comm&) { world.device = 2, world.owner = 0; });
   expect("another context's memory", 0, 1, ucclSuccess, [](Comm&) { world.owner = 8; });
   expect("memory of no context", 1, 0, ucclSuccess, [](Comm&) { world.owner = 0; });
   expect("read-only memory", 0, 1, ucclSuccess, [](Comm&) { world.access = CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READ; });
