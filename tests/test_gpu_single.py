@@ -74,8 +74,7 @@ def test_cast_single_rank_keeps_to_its_ctas(din, dout):
     last round that is nearly empty, and the same bits as without a limit."""
     import os
 
-    from torch.profiler import ProfilerActivity, profile
-
+    from graph_util import nodes
     from unified_ccl_b200 import Communicator
 
     os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
@@ -88,12 +87,9 @@ def test_cast_single_rank_keeps_to_its_ctas(din, dout):
             comm.set_blocks(0)
             ref_scales = comm.reduce_scatter_cast(x, ref, 0.37)[1]
             comm.set_blocks(blocks)
-            torch.cuda.synchronize()
-            with profile(activities=[ProfilerActivity.CUDA]) as prof:
-                scales = comm.reduce_scatter_cast(x, out, 0.37)[1]
-                torch.cuda.synchronize()
-            grids = [e["args"]["grid"] for e in _kernel_events(prof) if "cast" in e["name"]]
-            assert len(grids) == 1 and grids[0][0] <= blocks and grids[0][1:] == [1, 1], (count, grids)
+            scales = comm.reduce_scatter_cast(x, out, 0.37)[1]
+            grids = [grid for _, name, grid in nodes(lambda: comm.reduce_scatter_cast(x, out, 0.37, scales=scales)) if "cast" in name]
+            assert len(grids) == 1 and grids[0][0] <= blocks and grids[0][1:] == (1, 1), (count, grids)
             assert torch.equal(out.view(torch.uint8), ref.view(torch.uint8)), (blocks, count)
             assert scales is None or torch.equal(scales, ref_scales), (blocks, count)
     comm.destroy()
@@ -142,31 +138,13 @@ def test_refused_launches_say_why():
     comm.destroy()
 
 
-def _edge_types(calls):
-    """What connects the kernels of these calls in a captured graph: 0 a full dependency, 1 one that lets the second come up early."""
-    import ctypes
-
-    cu = ctypes.CDLL("libcuda.so.1")
-    side = torch.cuda.Stream()
-    stream, graph, n = ctypes.c_void_p(side.cuda_stream), ctypes.c_void_p(), ctypes.c_size_t(16)
-    torch.cuda.synchronize()
-    assert cu.cuStreamBeginCapture_v2(stream, 2) == 0
-    with torch.cuda.stream(side):
-        for call in calls:
-            call()
-    assert cu.cuStreamEndCapture(stream, ctypes.byref(graph)) == 0
-    ends, data = [(ctypes.c_void_p * 16)() for _ in range(2)], (ctypes.c_ubyte * 8 * 16)()  # CUgraphEdgeData: its third byte is the type
-    assert cu.cuGraphGetEdges_v2(graph, ends[0], ends[1], data, ctypes.byref(n)) == 0
-    cu.cuGraphDestroy(graph)
-    return [data[i][2] for i in range(n.value)]
-
-
 @gpu
 def test_limited_casts_do_not_come_up_early():
     """Under a limit on the CTAs, at once or in rounds, a cast starts after the launch before it has ended; without one it may
     come up before."""
     import os
 
+    from graph_util import edge_types
     from unified_ccl_b200 import Communicator
 
     os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
@@ -176,7 +154,7 @@ def test_limited_casts_do_not_come_up_early():
     for blocks, kind in ((0, 1), (2, 0), (48, 0)):  # 32 CTAs of their own, two, 32
         comm.set_blocks(blocks)
         cast()
-        assert _edge_types([cast] * 3) == [kind] * 2, blocks
+        assert edge_types(cast, cast, cast) == [kind] * 2, blocks
     comm.destroy()
 
 
@@ -212,15 +190,6 @@ def test_limited_cast_keeps_sms_free():
         early.append(other_end.elapsed_time(cast_end) / start.elapsed_time(cast_end))
     comm.destroy()
     assert max(early[1:]) > 0.5, early
-
-
-def _kernel_events(prof):
-    import json
-    import tempfile
-
-    with tempfile.NamedTemporaryFile(suffix=".json") as f:
-        prof.export_chrome_trace(f.name)
-        return [e for e in json.load(open(f.name))["traceEvents"] if e.get("cat") == "kernel"]
 
 
 @gpu

@@ -7,17 +7,6 @@ import torch
 gpu = pytest.mark.gpu
 
 
-def _kernels(f):
-    from torch.profiler import ProfilerActivity, profile
-
-    f()
-    torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        f()
-        torch.cuda.synchronize()
-    return [e.name for e in prof.events()]
-
-
 @gpu
 @pytest.mark.parametrize("count", [1, 15, 16, 31, 32, 33, 8191, 8192, 8193, 8225, 8192 * 32 + 7,  # around a piece and a CTA of pieces
                                    148 * 8 * 256 * 4 * 16 - 32, 148 * 5 * 256 * 4 * 32 - 32, 148 * 5 * 256 * 4 * 32, 148 * 8 * 256 * 4 * 32 - 16, 148 * 8 * 256 * 4 * 32, 148 * 8 * 256 * 4 * 32 + 4097])  # of four pieces
@@ -39,11 +28,18 @@ def test_one_rank_copy(count, src_off, dst_off):
 def test_which_copy():
     """The kernel for aligned memory of this GPU; the runtime's copy for the rest and where CTAs are limited."""
     os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    from graph_util import KERNEL, MEMCPY, nodes
     from unified_ccl_b200 import Communicator, _C
 
     comm = Communicator(0, 1)
     x, y = torch.randn(4096, device="cuda"), torch.empty(4096, device="cuda")
-    kernel = lambda f: any("local_copy_kernel" in n for n in _kernels(f))  # noqa: E731
+
+    def kernel(call):
+        call()
+        (kind, name, _), = nodes(call)
+        assert kind == MEMCPY or "local_copy_kernel" in name
+        return kind == KERNEL
+
     assert kernel(lambda: comm.allgather(x, y))
     assert not kernel(lambda: comm.allgather(x[1:4000], y[:3999]))
     comm.set_blocks(4)
@@ -51,8 +47,7 @@ def test_which_copy():
     comm.set_blocks(0)
     # pinned host memory, by address: copied as ever
     h = torch.arange(4096, dtype=torch.float32).pin_memory()
-    stream = torch.cuda.current_stream().cuda_stream
-    assert not kernel(lambda: _C.allgather(comm.handle, h.data_ptr(), y.data_ptr(), 4096, 2, stream))
+    assert not kernel(lambda: _C.allgather(comm.handle, h.data_ptr(), y.data_ptr(), 4096, 2, torch.cuda.current_stream().cuda_stream))
     torch.cuda.synchronize()
     assert torch.equal(y.cpu(), h)
     comm.destroy()
