@@ -60,7 +60,7 @@ TENSORMOD := $(PKG)/_uccl_tensor_calls$(EXTSUFFIX)
 PLUGIN    := plugins/sample/libuccl-net-sample.so
 UCXPLUGIN := plugins/ucx/libuccl-net-ucx.so
 # test-only code: native self tests of the host runtime, kernels that call the device-side RMA
-# API or the epilogue's silu, and a C++ client of the C ABI
+# API, the epilogue's silu or the fp8 quantisation, and a C++ client of the C ABI
 SELFTEST  := tests/native/libuccl_selftest.so
 DEVTEST   := tests/native/libuccl_devtest.so
 CLIENT    := tests/native/c_api_client
@@ -123,7 +123,7 @@ ucx-fake: plugins/ucx/libuccl-net-ucx-fake.so
 $(SELFTEST): tests/native/selftest.cc tests/native/local_copy_test.cc csrc/core/local_copy.cc tests/native/uccl_selftest.h $(LIB) $(wildcard include/*.h csrc/*/*.h)
 	$(CXX) $(CXXFLAGS) -Itests/native -shared $(filter tests/native/%.cc,$^) -o $@ -L$(PKG) -luccl -Wl,-rpath,'$$ORIGIN/../../$(PKG)'
 
-$(DEVTEST): tests/native/rma_device_test.cu tests/native/swiglu_device_test.cu include/uccl_device.cuh include/uccl.h csrc/kernels/swiglu.cuh $(LIB)
+$(DEVTEST): tests/native/rma_device_test.cu tests/native/swiglu_device_test.cu tests/native/fp8_device_test.cu include/uccl_device.cuh include/uccl.h csrc/kernels/swiglu.cuh csrc/kernels/fp8_cast.cuh csrc/kernels/ptx.cuh $(LIB)
 	$(NVCC) $(NVFLAGS) -shared $(filter %.cu,$^) -o $@ -L$(PKG) -luccl -Xlinker -rpath,'$$ORIGIN/../../$(PKG)' -lcudart_static
 
 $(BASELINE): baseline/swiglu_kernel.cu

@@ -175,6 +175,7 @@ template <int DT, int OUT, int U>
 __device__ __forceinline__ void cast_share(const CastLocalArgs& a, size_t first) {
   constexpr int E = 32 / Vec<DT>::ES;  // elements per piece
   constexpr int LANES = 128 / E;    // lanes that share one scale block
+  using T2 = typename std::conditional<DT == DT_BF16, __nv_bfloat162, __half2>::type;
   const size_t pieces = (a.elems + E - 1) / E;
   const size_t c0 = first + threadIdx.x;
   uint32_t raw[U][8];
@@ -207,9 +208,14 @@ __device__ __forceinline__ void cast_share(const CastLocalArgs& a, size_t first)
 #pragma unroll
     for (int e = 0; e < E / 2; ++e) {
       float2 x;
-      if constexpr (DT == DT_F32) x = make_float2(__uint_as_float(raw[u][2 * e]), __uint_as_float(raw[u][2 * e + 1]));
-      else x = DT == DT_BF16 ? ptx::unpack_bf16x2(raw[u][e]) : ptx::unpack_f16x2(raw[u][e]);
-      v[e] = ptx::mul2(ptx::add2(make_float2(0.f, 0.f), x), make_float2(factor, factor));
+      if constexpr (DT == DT_F32) {
+        x = ptx::add2(make_float2(0.f, 0.f), make_float2(__uint_as_float(raw[u][2 * e]), __uint_as_float(raw[u][2 * e + 1])));
+      } else {  // exact in the 16-bit type, and half the instructions there
+        uint32_t z = 0;
+        *reinterpret_cast<T2*>(&z) = __hadd2(*reinterpret_cast<T2*>(&z), *reinterpret_cast<T2*>(&raw[u][e]));
+        x = DT == DT_BF16 ? ptx::unpack_bf16x2(z) : ptx::unpack_f16x2(z);
+      }
+      v[e] = ptx::mul2(x, make_float2(factor, factor));
     }
     char* out = a.out + c * E * (OUT == OUT_FP8 ? 1 : OUT == OUT_F32 ? 4 : 2);
     if (OUT == OUT_FP8) {
@@ -248,10 +254,10 @@ __device__ __forceinline__ void cast_share(const CastLocalArgs& a, size_t first)
     }
   }
 }
-// Pieces per thread of a large launch, and CTAs per SM.  A conversion to fp8 takes some hundred instructions a piece, and
+// Pieces per thread of a large launch, and CTAs per SM.  A conversion to fp8 takes some eighty instructions a piece, and
 // two pieces on six CTAs put more of them beside other CTAs' loads than four pieces on four: 64 Mi bf16 33.0 -> 31.4 us, 16 Mi
-// 11.4 -> 10.1, 6 Mi fp32 6.7 -> 5.8; with the rest, bound by its loads and stores, it is the same.  Six CTAs leave 40 registers, and
-// 16-bit input spills 8 bytes; five (47 registers, no spill) are slower: 64 Mi bf16 31.1 and 31.5 us, 32 Mi fp32 25.3 and 26.4.
+// 11.4 -> 10.1, 6 Mi fp32 6.7 -> 5.8 (measured with a longer quotient, and five CTAs then slower than six: 64 Mi bf16 31.5 and
+// 31.1 us, 32 Mi fp32 26.4 and 25.3); with the rest, bound by its loads and stores, it is the same.
 template <int OUT>
 constexpr int kCastPieces = OUT == OUT_FP8 ? 2 : 4;
 template <int DT, int OUT, int U>

@@ -68,6 +68,61 @@ def test_cast_single_rank(din, dout):
 
 
 @gpu
+def test_fp8_quantisation_is_the_division():
+    """The one-step quotient gives the byte of a correctly rounded division for every divisor (all significands, the ends of the
+    range of a scale) at every place where the byte changes, and a scale has the bits of amax / 448 for every amax."""
+    import ctypes
+    import os
+
+    lib = ctypes.CDLL(os.path.join(os.path.dirname(os.path.abspath(__file__)), "native", "libuccl_devtest.so"))
+    lib.ucclDevTestFp8Divisor.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
+    lib.ucclDevTestFp8Scale.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+    stream = torch.cuda.current_stream().cuda_stream
+    out = torch.zeros(2, device="cuda", dtype=torch.int32)
+    for exponent in (-42, 0, 118):  # 1e-10 / 448 to the largest float / 448
+        assert lib.ucclDevTestFp8Divisor(exponent, out.data_ptr(), stream) == 0
+    assert lib.ucclDevTestFp8Scale(out.data_ptr(), stream) == 0
+    wrong, bits = out.tolist()
+    assert wrong == 0, f"{wrong & 0xffffffff} differ, one of them {bits & 0xffffffff:#010x}"
+
+
+@gpu
+@pytest.mark.parametrize("din", [torch.bfloat16, torch.float16, torch.float32])
+def test_cast_of_zeros_infinities_and_nan(din):
+    """Blocks of signed zeros, of subnormals, with an infinity, with a NaN and all NaN, to every output type."""
+    import os
+
+    from unified_ccl_b200 import Communicator
+
+    os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    comm = Communicator(0, 1)
+    x = torch.randn(6, 128, device="cuda")
+    x[0] = 0.0
+    x[0, ::2] = -0.0
+    x[1] *= torch.finfo(din).tiny / 4
+    x[2, 5], x[2, 9] = float("inf"), -0.0
+    x[3, 7], x[3, 8] = float("nan"), 0.0
+    x[4] = float("nan")
+    x[5, 0], x[5, 1] = -0.0, -torch.finfo(din).tiny
+    x = x.to(din).view(-1)
+    ref = (x.float() + 0.0) * torch.tensor(0.37, device="cuda")
+    for dout in (torch.bfloat16, torch.float16, torch.float32, torch.float8_e4m3fn):
+        out, scales = comm.reduce_scatter_cast(x, torch.empty(x.numel(), device="cuda", dtype=dout), 0.37)
+        want = ref
+        if dout == torch.float8_e4m3fn:
+            blocks = ref.view(-1, 128)
+            sc = torch.where(blocks.isnan(), torch.zeros_like(blocks), blocks).abs().amax(-1, keepdim=True).clamp_min(1e-10)
+            sc = sc / torch.full_like(sc, 448.0)
+            assert torch.equal(scales, sc.view(-1))
+            want = (blocks / sc).view(-1)
+        want, got = want.to(dout).float(), out.float()
+        assert torch.equal(got.isnan(), want.isnan()), dout
+        keep = ~want.isnan()
+        assert torch.equal(got[keep].view(torch.int32), want[keep].view(torch.int32)), dout
+    comm.destroy()
+
+
+@gpu
 @pytest.mark.parametrize("din,dout", [(torch.bfloat16, torch.float8_e4m3fn), (torch.float32, torch.bfloat16)])
 def test_cast_single_rank_keeps_to_its_ctas(din, dout):
     """A limit on the CTAs of a communicator's kernels holds for one rank too, with one and with four pieces per thread, a
