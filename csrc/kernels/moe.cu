@@ -1,6 +1,7 @@
 // MoE expert-parallel dispatch and combine as single kernels over NVLink peer memory.
 //
-// dispatch : a CTA takes one token after the other, sixteen elements per thread.  Quantise: every thread
+// dispatch (among ranks; one rank has a simpler kernel of its own, below):
+//            a CTA takes one token after the other, sixteen elements per thread.  Quantise: every thread
 //            has loaded its 32 bytes of the bf16 row while the CTA dealt with the token before, eight
 //            lanes agree on the fp32 scale of their 128 elements (amax / 448), convert to fp8 e4m3 and
 //            write one 16-byte piece into one of three row buffers in shared memory.  Scatter: lane k of
@@ -32,9 +33,114 @@ constexpr int kMoeBufs = 3;
 // shared memory of one row buffer: the quantised row, then its scales
 __host__ __device__ constexpr int moe_row_smem(int hidden) { return hidden + ((hidden / 128 * 4 + 15) & ~15); }
 
-// Bound by memory (a token is 2 H bytes in and topk (H + H / 32) out), then by latencies when tokens are few.
-// A token per CTA instead of one per warp: 4096 tokens x 7168 on 3552 warps were two uneven rounds of long
-// serial chains, 91 us, and 96 tokens kept 12 SMs busy for 27 us; now 55 us (5.4 TB/s) and 7 us.
+// 32 bytes of a bf16 row; `wide`: they start on a 32-byte boundary
+__device__ __forceinline__ void load16(const char* p, bool wide, uint32_t (&raw)[8]) {
+  if (wide) {
+    ptx::ld_stream_v8(p, raw);
+  } else {
+    const uint4 lo = ptx::ld_stream_v4(p), hi = ptx::ld_stream_v4(p + 16);
+    raw[0] = lo.x, raw[1] = lo.y, raw[2] = lo.z, raw[3] = lo.w, raw[4] = hi.x, raw[5] = hi.y, raw[6] = hi.z, raw[7] = hi.w;
+  }
+}
+// Sixteen bf16 elements of a thread as e4m3, and the scale of the 128 that it shares with seven other lanes (whole warps).
+__device__ __forceinline__ uint4 quantise16(const uint32_t (&raw)[8], float& scale) {
+  __nv_bfloat162 m = __habs2(reinterpret_cast<const __nv_bfloat162&>(raw[0]));
+#pragma unroll
+  for (int j = 1; j < 8; ++j) m = __hmax2(m, __habs2(reinterpret_cast<const __nv_bfloat162&>(raw[j])));
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, reinterpret_cast<const uint32_t&>(m), o);
+    m = __hmax2(m, reinterpret_cast<const __nv_bfloat162&>(other));
+  }
+  const float2 mf = __bfloat1622float2(m);
+  scale = fp8::block_scale(fmaxf(mf.x, mf.y));
+  const fp8::Divisor div(scale);
+  uint32_t q[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)  // the divisor takes its elements negated
+    q[j] = div.quantise4(ptx::unpack_bf16x2(raw[2 * j] ^ 0x80008000u), ptx::unpack_bf16x2(raw[2 * j + 1] ^ 0x80008000u));
+  return make_uint4(q[0], q[1], q[2], q[3]);
+}
+
+// One rank: nobody to tell and nobody to wait for, so a token is a CTA of its own, which stores its row straight from
+// registers.  Each token takes its rows with one atomic on a 64-bit counter (rows below, tokens above); the CTA that sees all
+// the others there publishes the number of rows and clears the counter, long before the rows are written: the launch behind
+// waits for the end of this one before it touches any of it.
+//
+// Bound by memory (a token is 2 H bytes in and topk (H + H / 32) out), and by its latencies when tokens are few: experts, one
+// atomic, the stores.  Before, 296 CTAs with an equal share of the tokens each and a bulk copy per row: 4096 x 7168 top-8
+// 54.8 us, now 47.8 (6.3 TB/s), 96 tokens of it 5.7 and 4.0, 1000 x 2048 top-2 4.9 and 3.3.  A loop around plain stores alone took
+// 53.6: with equal shares the slowest SMs end the launch, with a CTA per token all end together (a kernel that only reads and
+// writes these bytes takes 51.5 us on 296 CTAs, 46.0 on 4096).
+// CTAS, of 512 threads per SM, sets the registers: four (32 registers) where the tokens are more than fit at once, two (50, whose
+// loads are out earlier) where they are not: 4096 x 7168 47.8 and 56.6 us, 512 x 8192 8.7 and 10.1; 96 x 7168 4.4 and 4.0, 1000 x
+// 2048 3.75 and 3.3, 300 x 5120 top-4 4.1 and 3.6.
+template <int CTAS>
+__global__ void __launch_bounds__(512, CTAS) moe_dispatch_one_kernel(const __grid_constant__ MoeArgs a) {
+  __shared__ __align__(16) int s_slot[kMoeMaxTopk];
+  __shared__ float s_scale[64];
+  const int t = blockIdx.x, lane = threadIdx.x & 31;
+  const int H = a.hidden, nblk = H / 128, e0 = threadIdx.x * 16;
+  ptx::launch_dependents();
+  ptx::wait_dependencies();
+  if (t >= a.tokens) {  // no tokens at all
+    if (threadIdx.x == 0) a.recvCounts[0][0] = 0;
+    return;
+  }
+  // the first warp's chain of experts, rows and their slots runs beside the conversion
+  const bool router = threadIdx.x < 32;
+  int expert = -1;
+  if (router && lane < a.topk) expert = a.topkIdx[static_cast<size_t>(t) * a.topk + lane];
+  uint32_t raw[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (e0 < H) load16(static_cast<const char*>(a.x) + (static_cast<size_t>(t) * H + e0) * 2, (reinterpret_cast<uintptr_t>(a.x) & 31) == 0, raw);
+  unsigned long long* counter = reinterpret_cast<unsigned long long*>(a.sendCount);
+  unsigned long long seen = 0;
+  unsigned valid = 0;
+  if (router) {
+    valid = __ballot_sync(0xffffffffu, expert >= 0 && expert < a.numExperts);
+    if (lane == 0) seen = atomicAdd(counter, (1ull << 32) + __popc(valid));
+  }
+  float scale;
+  const uint4 q = quantise16(raw, scale);
+  if (router) {
+    int slot = __shfl_sync(0xffffffffu, static_cast<int>(static_cast<uint32_t>(seen)), 0) + __popc(valid & ((1u << lane) - 1));
+    if (!(valid >> lane & 1)) {
+      slot = -1;
+    } else if (slot >= a.rowsPerSource) {
+      atomicAdd(a.overflow, 1u);
+      slot = -1;
+    }
+    if (lane < kMoeMaxTopk) s_slot[lane] = slot;
+    if (lane < a.topk) {
+      a.slotOf[static_cast<size_t>(t) * a.topk + lane] = slot;
+      if (slot >= 0) *reinterpret_cast<int4*>(a.recvMeta[0] + static_cast<size_t>(slot) * 4) = make_int4(t, expert, lane, 1);
+    }
+    if (lane == 0 && static_cast<int>(seen >> 32) == a.tokens - 1) {
+      a.recvCounts[0][0] = min(static_cast<int>(static_cast<uint32_t>(seen)) + __popc(valid), a.rowsPerSource);
+      *counter = 0;  // ready for the next call
+    }
+  }
+  if (e0 < H && (lane & 7) == 0) s_scale[e0 >> 7] = scale;
+  __syncthreads();
+  if (e0 < H) {
+    char* col = a.recvX[0] + e0;
+#pragma unroll 1
+    for (int k = 0; k < a.topk; k += 4) {
+      const int4 w = *reinterpret_cast<const int4*>(&s_slot[k]);  // -1 beyond top-k
+      if (w.x >= 0) ptx::st_global_v4(col + static_cast<size_t>(w.x) * H, q);
+      if (w.y >= 0) ptx::st_global_v4(col + static_cast<size_t>(w.y) * H, q);
+      if (w.z >= 0) ptx::st_global_v4(col + static_cast<size_t>(w.z) * H, q);
+      if (w.w >= 0) ptx::st_global_v4(col + static_cast<size_t>(w.w) * H, q);
+    }
+  }
+  for (int i = threadIdx.x; i < a.topk * nblk; i += blockDim.x) {
+    const int k = i / nblk, b = i - k * nblk, slot = s_slot[k];
+    if (slot >= 0) a.recvScale[0][static_cast<size_t>(slot) * nblk + b] = s_scale[b];
+  }
+}
+
+// A token per CTA instead of one per warp, measured when one rank ran this kernel too: 4096 tokens x 7168 on 3552 warps were two
+// uneven rounds of long serial chains, 91 us, and 96 tokens kept 12 SMs busy for 27 us; with a token per CTA 55 us and 7 us.
 __global__ void __launch_bounds__(512, 2) moe_dispatch_kernel(const __grid_constant__ MoeArgs a) {
   extern __shared__ __align__(16) uint8_t moe_smem[];
   __shared__ int s_row[kMoeBufs][kMoeMaxTopk];  // destination << 24 | slot of a buffer's row, -1: none
@@ -53,13 +159,7 @@ __global__ void __launch_bounds__(512, 2) moe_dispatch_kernel(const __grid_const
 #pragma unroll
     for (int j = 0; j < 8; ++j) raw[j] = 0;
     if (t >= a.tokens || e0 >= H) return;
-    const char* p = static_cast<const char*>(a.x) + (static_cast<size_t>(t) * H + e0) * 2;
-    if (wide) {
-      ptx::ld_stream_v8(p, raw);
-    } else {
-      const uint4 lo = ptx::ld_stream_v4(p), hi = ptx::ld_stream_v4(p + 16);
-      raw[0] = lo.x, raw[1] = lo.y, raw[2] = lo.z, raw[3] = lo.w, raw[4] = hi.x, raw[5] = hi.y, raw[6] = hi.z, raw[7] = hi.w;
-    }
+    load16(static_cast<const char*>(a.x) + (static_cast<size_t>(t) * H + e0) * 2, wide, raw);
   };
   // Routing runs ahead, so that no token waits for its latencies: the experts of (t, k) are read two tokens
   // early, the atomics that take row slots are issued one token early (lanes with the same destination
@@ -82,8 +182,6 @@ __global__ void __launch_bounds__(512, 2) moe_dispatch_kernel(const __grid_const
     return -1;
   };
 
-  if (n == 1) ptx::launch_dependents();
-  ptx::wait_dependencies();
   int buf = 0;
   load(blockIdx.x);
   if (threadIdx.x < 32) {
@@ -95,24 +193,11 @@ __global__ void __launch_bounds__(512, 2) moe_dispatch_kernel(const __grid_const
     uint8_t* rowBuf = moe_smem + buf * moe_row_smem(H);
     float* scaleBuf = reinterpret_cast<float*>(rowBuf + H);
     // ---- quantise (lanes beyond the row take part in the shuffles with zeros)
-    __nv_bfloat162 m = __habs2(reinterpret_cast<const __nv_bfloat162&>(raw[0]));
-#pragma unroll
-    for (int j = 1; j < 8; ++j) m = __hmax2(m, __habs2(reinterpret_cast<const __nv_bfloat162&>(raw[j])));
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {  // a 128-element block is eight lanes
-      const uint32_t other = __shfl_xor_sync(0xffffffffu, reinterpret_cast<const uint32_t&>(m), o);
-      m = __hmax2(m, reinterpret_cast<const __nv_bfloat162&>(other));
-    }
-    const float2 mf = __bfloat1622float2(m);
-    const float scale = fp8::block_scale(fmaxf(mf.x, mf.y));
-    const fp8::Divisor div(scale);
-    uint32_t q[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)  // the divisor takes its elements negated
-      q[j] = div.quantise4(ptx::unpack_bf16x2(raw[2 * j] ^ 0x80008000u), ptx::unpack_bf16x2(raw[2 * j + 1] ^ 0x80008000u));
+    float scale;
+    const uint4 q = quantise16(raw, scale);
     load(t + gridDim.x);
     if (e0 < H) {
-      *reinterpret_cast<uint4*>(rowBuf + e0) = make_uint4(q[0], q[1], q[2], q[3]);
+      *reinterpret_cast<uint4*>(rowBuf + e0) = q;
       if ((lane & 7) == 0) scaleBuf[e0 >> 7] = scale;
     }
     int place = -1;
@@ -150,31 +235,20 @@ __global__ void __launch_bounds__(512, 2) moe_dispatch_kernel(const __grid_const
     }
     buf = buf + 1 == kMoeBufs ? 0 : buf + 1;
   }
-  // Every bulk copy of this thread has completed (written, not just read) before the CTA reports in, and before a
-  // launch that has come up early may read the rows.
+  // Every bulk copy of this thread has completed (written, not just read) before the CTA reports in.
   if (router) ptx::tma_store_wait<0>();
 
   // ---- completion: the last CTA publishes counts and flags, then waits for every source
   __shared__ int s_last;
   __syncthreads();
   if (threadIdx.x == 0) {
-    if (n > 1) ptx::fence_sys();
-    else __threadfence();  // the slot counter of this CTA's tokens, for the CTA that reads it below
+    ptx::fence_sys();
     const uint32_t prev = atomicAdd(a.ctasDone, 1u);
     s_last = prev == gridDim.x - 1;
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  if (n == 1) {  // nobody to tell and nobody to wait for
-    if (threadIdx.x == 0) {
-      const uint32_t rows = *reinterpret_cast<volatile uint32_t*>(a.sendCount);
-      a.recvCounts[0][0] = static_cast<int32_t>(min(rows, static_cast<uint32_t>(a.rowsPerSource)));
-      *a.sendCount = 0;  // ready for the next call
-      *a.ctasDone = 0;
-    }
-    return;
-  }
   const uint32_t e = *a.epoch + 1;
   if (threadIdx.x < static_cast<unsigned>(n)) {
     const int p = threadIdx.x;
@@ -248,13 +322,15 @@ __global__ void __launch_bounds__(kCombineThreads, TK > 8 ? 3 : TK > 4 ? 5 : 6) 
 
 cudaError_t launchMoeDispatch(const MoeArgs& a, cudaStream_t stream) {
   if (a.hidden % 128 != 0 || a.hidden > 8192 || a.topk < 1 || a.topk > dev::kMoeMaxTopk) return cudaErrorInvalidValue;
-  const int smem = dev::kMoeBufs * dev::moe_row_smem(a.hidden);  // 25 KiB at most
   const int threads = (a.hidden / 16 + 31) / 32 * 32;
-  // as many CTAs as fit at once: 64 registers a thread
-  const int perSm = 1024 / threads;
-  const int ctas = std::max(1, std::min(a.tokens, deviceSmCount() * perSm));
+  const int resident = deviceSmCount() * (1024 / threads);  // at 64 registers a thread
+  if (a.dc.nranks == 1) {
+    auto kern = a.tokens > resident ? dev::moe_dispatch_one_kernel<4> : dev::moe_dispatch_one_kernel<2>;
+    return launchOverlapped(kern, std::max(1, a.tokens), threads, 0, stream, a);
+  }
+  const int smem = dev::kMoeBufs * dev::moe_row_smem(a.hidden);  // 25 KiB at most
+  const int ctas = std::max(1, std::min(a.tokens, resident));
   // ranks that wait for one another keep to the plain launch
-  if (a.dc.nranks == 1) return launchOverlapped(dev::moe_dispatch_kernel, ctas, threads, smem, stream, a);
   dev::moe_dispatch_kernel<<<ctas, threads, smem, stream>>>(a);
   return cudaGetLastError();
 }

@@ -274,7 +274,7 @@ def test_norm_single_rank_shapes(tokens, hidden):
 @pytest.mark.parametrize("tokens,hidden,experts,topk,off", [
     (1, 128, 1, 1, 0), (3, 1152, 4, 3, 8), (700, 1152, 16, 16, 0), (2000, 384, 8, 2, 0), (1300, 7168, 256, 8, 8), (65, 8192, 32, 5, 0)])
 def test_moe_single_rank_shapes(tokens, hidden, experts, topk, off):
-    """Rows of part of a warp up to 512 threads, scales that bulk copies cannot move, several tokens per CTA, unused
+    """Rows of part of a warp up to 512 threads, tokens that fit on the GPU at once and more, unused
     slots, an input on a 16-byte boundary only (`off` elements in front), every top-k class of the combine."""
     import os
 
@@ -314,6 +314,37 @@ def test_moe_single_rank_shapes(tokens, hidden, experts, topk, off):
     # topk fp32 additions in another order, then one rounding to bf16
     assert ((out.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + mag * topk * 2.0 ** -23).all()
     assert disp.overflow() == 0
+    disp.close()
+    comm.destroy()
+
+
+@gpu
+def test_moe_single_rank_capacity_and_no_tokens():
+    """Rows beyond the capacity are counted and left out, a call without tokens receives nothing, and the counter that the
+    tokens share is ready for the next call after each of them, with more tokens than fit on the GPU at once too."""
+    import os
+
+    from unified_ccl_b200 import _C, Communicator
+    from unified_ccl_b200.parallel import MoeDispatcher
+
+    os.environ.setdefault("UCCL_BOOTSTRAP_IFNAME", "lo")
+    comm = Communicator(0, 1)
+    tokens, hidden, topk = 600, 8192, 3
+    disp = MoeDispatcher(comm, tokens, hidden, 8, topk, capacity_factor=0.5)
+    rows = disp.rows_per_source
+    assert rows == tokens * topk // 2
+    x = torch.randn(tokens, hidden, device="cuda").to(torch.bfloat16)
+    idx = torch.randint(0, 8, (tokens, topk), device="cuda", dtype=torch.int32)
+    over = 0
+    for n in (tokens, 0, 7, rows // topk, rows // topk + 1, tokens):
+        _C.moe_dispatch(disp._ctx, x.data_ptr(), idx.data_ptr(), n, comm._stream())  # an empty tensor has no address
+        assert int(disp.recv_counts[0]) == min(n * topk, rows)
+        over += max(0, n * topk - rows)
+        assert disp.overflow() == over
+        meta = disp.recv_meta[0, : min(n * topk, rows)].long()
+        key = meta[:, 0] * topk + meta[:, 2]
+        assert key.unique().numel() == key.numel() and bool((key < max(1, n * topk)).all())
+        assert torch.equal(meta[:, 1], idx.view(-1)[key].long())
     disp.close()
     comm.destroy()
 
