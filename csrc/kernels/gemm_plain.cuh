@@ -258,19 +258,30 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   ptx::wait_dependencies();
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    // ------------------------------------------------------------ TMA producer: one elected lane.  Behind `lane == 0`
+    // a stage took 400 cycles to issue, of them 290 for the wait on a slot that was free: more than the MMAs of a narrow tile, and
+    // the whole main loop of a short K.  Elected, and with the next slot's barrier looked at before this one's loads are
+    // issued, it takes 88, and 29 as long as there are slots that nothing has used yet.  1 x 672 x 736 5.32 -> 4.32 us, 58 x 7608 x
+    // 1680 9.22 -> 8.15, SwiGLU 557 x 1776 x 1680 10.5 -> 8.3, 26 x 32 x 280 4.1 -> 3.1.  Pairs, whose slots are seldom free early,
+    // look when they need to: with the look ahead SwiGLU 4096 x 7168 x 4096 188.0 us, without 181.8, before 183.1.  2 x 12824 x
+    // 4040, bound by memory, loses: 23.9 -> 24.3.
+    if (ptx::elect_one()) {
       const uint32_t lead_full = CG == 2 ? ptx::mapa(ptx::smem_u32(full_bar), static_cast<uint32_t>(crank - half)) : 0;
       const uint32_t bytes = static_cast<uint32_t>(CG * a.stage_bytes);
-      int s = 0;
+      int s = 0, unused = a.stages;
       uint32_t ph = 1;
+      bool there = true;  // slot s is known to be free
       for (int tile = worker; tile < a.num_tiles && !*bail; tile += a.workers) {
         int mt = first_mt, nt = first_nt;
         if (tile != worker) coords<CG == 2 ? 8 : 16>(a, tile, mt, nt);
         const int m0 = (mt * CG + half) * BM;
         const int b0 = nt * (EPI == kEpiSwiGLU ? a.out_bn : a.bn);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!ptx::mbar_wait_bounded(&empty_bar[s], ph, bail)) break;
+          if (!there && !ptx::mbar_wait_bounded(&empty_bar[s], ph, bail)) break;
+          const int next = s + 1 == a.stages ? 0 : s + 1;
+          const uint32_t next_ph = next == 0 ? ph ^ 1 : ph;
+          if (unused > 0) --unused;
+          there = unused > 0 || (CG == 1 && ptx::mbar_test(&empty_bar[next], next_ph));
           uint8_t* sA = smem + s * a.stage_bytes;
           uint8_t* sB = sA + a.a_rows * (BK * 2);
           if (CG == 2) {
@@ -284,7 +295,7 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             ptx::tma_load_2d(sB, &tmB, &full_bar[s], kb * BK, b0);
             if (EPI == kEpiSwiGLU) ptx::tma_load_2d(sB + a.out_bn * (BK * 2), &tmB, &full_bar[s], kb * BK, b0 + a.b_half_rows);
           }
-          if (++s == a.stages) s = 0, ph ^= 1;
+          s = next, ph = next_ph;
         }
       }
     }
