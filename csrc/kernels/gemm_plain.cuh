@@ -11,7 +11,9 @@
 //
 // A tile's stage of the ring holds 64 columns of K: the A rows and bn / CG rows of B.  With fewer than 128
 // rows in all the A part holds just these (a_rows); the tensor core then reads rows of B where the rest of A
-// would be, which only reaches accumulator rows that nobody looks at.
+// would be, which only reaches accumulator rows that nobody looks at.  Up to 64 rows take MMAs of 64 rows: as fast where the
+// tile is wide, 29 cycles and not 43 where it is narrow, and half the energy, which the SM clock gets back under the power
+// cap: MLP of 64 x 4096 x 14336 71.2 -> 68.5 us, 2 x 12824 x 4040 24.4 -> 22.7, 58 x 7608 x 1680 8.1 -> 7.4.
 //
 // Whole tiles give the same bits in every cut; a tile in parts adds K up in another order, so that the bits of a row can
 // depend on how many rows there are.  The parts are the closer of the two to the exact sum: of 71 shapes, none
@@ -44,6 +46,7 @@ struct Args {
   int tma_n;             // a TMA store may start at columns below this one
   int b_half_rows;       // SwiGLU: row offset of the "up" half inside B
   int a_rows;            // rows of A in a stage (128, or fewer when M is)
+  int warp_rows;         // rows of a tile that a warp's TMEM lanes hold, from its first lane on: 32, or 16 of a 64-row tile
   int stages, stage_bytes;
   int split, workers;    // clusters in the grid; one tile each if split > 1
   uint32_t* err;
@@ -84,7 +87,7 @@ __device__ __forceinline__ void store16(const Args& a, int row, int col, const u
   }
 }
 
-// The whole tile of one warp (32 rows from row0): 64 output columns at a time through shared memory and TMA
+// The whole tile of one warp (warp_rows rows from row0): 64 output columns at a time through shared memory and TMA
 // stores, which clip what lies outside C; the columns that are left in units of 16 straight from registers.
 // A TMA store writes whole pieces of 16 bytes: where C ends inside of one, it would overwrite what the caller keeps
 // behind the row's end, so the last columns of such a C take the second way (tma_n).
@@ -122,7 +125,7 @@ __device__ __forceinline__ void store_tile(const Args& a, const CUtensorMap* tmC
     if (EPI == kEpiSwiGLU) ptx::tmem_ld_32x32b_x16(taddr + a.out_bn + c, y);
     ptx::tmem_ld_wait();
     pack16<EPI>(x, y, o);
-    store16(a, row0 + lane, col0 + c, o);
+    store16(a, lane < a.warp_rows ? row0 + lane : a.M, col0 + c, o);
     __syncwarp();
   }
 }
@@ -150,6 +153,7 @@ __device__ __forceinline__ void send_parts(const Args& a, uint32_t ring, uint32_
 #pragma unroll
       for (int h = 0; h < H; ++h) ptx::tmem_ld_32x32b_x16(taddr + h * a.out_bn + dst * w + c, x[h]);
       ptx::tmem_ld_wait();
+      if ((r & 31) >= a.warp_rows) continue;
 #pragma unroll
       for (int h = 0; h < H; ++h)
 #pragma unroll
@@ -343,7 +347,7 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       // 24.6 -> 23.7, 32 x 4096 x 4096 11.2 -> 10.6, 16 x 4096 x 1792 8.1 -> 7.8.  SwiGLU of a few rows with K below 600 loses by
       // it: 8 x 512 x 256 3.09 -> 3.11 us, 32 x 1792 x 256 3.14 -> 3.16.  Pairs, whose MMAs are wider, gain and lose one or two
       // percent by either and keep the plain form.
-      const uint32_t idesc = ptx::umma_idesc_f16(1u, BM, static_cast<uint32_t>(a.bn));
+      const uint32_t idesc = ptx::umma_idesc_f16(1u, static_cast<uint32_t>(4 * a.warp_rows), static_cast<uint32_t>(a.bn));
       const uint32_t act = ptx::elect_one() ? 1u : 0u, ring = ptx::smem_u32(smem), base = __shfl_sync(0xffffffffu, tmem_base, 0);
       int s = 0;
       uint32_t ph = 0, tcount = 0;
@@ -390,7 +394,7 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (a.split > 1) break;  // one tile, finished below
       ptx::tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-      store_tile<EPI>(a, &tmC, taddr, (mt * CG + half) * BM + q * 32, nt * a.out_bn, lane, stage, stage_it);
+      store_tile<EPI>(a, &tmC, taddr, (mt * CG + half) * BM + q * a.warp_rows, nt * a.out_bn, lane, stage, stage_it);
       ptx::tc_fence_before();
       __syncwarp();
       if (lane == 0) {
@@ -406,9 +410,10 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   if (a.split > 1) {
     const int mt = first_mt, nt = first_nt;
-    const int q = warp & 3, r = q * 32 + lane, row = (mt * CG + half) * BM + r;
+    const int q = warp & 3, r = q * 32 + lane, row0 = (mt * CG + half) * BM + q * a.warp_rows;
+    const int row = lane < a.warp_rows ? row0 + lane : a.M;
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-    const bool busy = warp >= 2 && row - lane < a.M;
+    const bool busy = warp >= 2 && row0 < a.M;
     ptx::cluster_sync();  // every part has used up its ring
     ptx::tc_fence_after();
     if (busy) send_parts<EPI>(a, ptx::smem_u32(smem), taddr, part, half, CG, r);

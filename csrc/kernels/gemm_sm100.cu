@@ -270,6 +270,7 @@ ucclResult_t launchPlain(const GemmLaunch& g, const GemmCut* cut, cudaStream_t s
   a.out_bn = swiglu ? p.bn / 2 : p.bn;
   a.b_half_rows = swiglu ? g.N / 2 : 0;
   a.a_rows = p.cg == 1 && g.M < gemm::BM ? (g.M + 7) / 8 * 8 : gemm::BM;
+  a.warp_rows = p.cg == 1 && g.M <= 64 ? 16 : 32;
   a.tiles_m = (g.M + p.cg * gemm::BM - 1) / (p.cg * gemm::BM);
   a.tiles_n = (out_n + a.out_bn - 1) / a.out_bn;
   a.num_tiles = a.tiles_m * a.tiles_n;
@@ -286,7 +287,7 @@ ucclResult_t launchPlain(const GemmLaunch& g, const GemmCut* cut, cudaStream_t s
   a.workers = p.split > 1 ? a.num_tiles : std::min(a.num_tiles, resident);
   CUtensorMap tmA, tmB, tmC = {};
   if (!makeTensorMap(&tmA, g.A, g.M, g.K, g.lda, gemm::BK, a.a_rows) || !makeTensorMap(&tmB, g.B, g.N, g.K, g.ldb, gemm::BK, swiglu || p.cg == 2 ? p.bn / 2 : p.bn) ||
-      (mapped && !makeTensorMap(&tmC, g.C, g.M, out_n, ldc, 64, 32)))
+      (mapped && !makeTensorMap(&tmC, g.C, g.M, out_n, ldc, 64, a.warp_rows)))
     return ucclSystemError;
   cudaError_t e;
   if (swiglu) e = p.cg == 2 ? launchPlainT<gemm::kEpiSwiGLU, 2>(tmA, tmB, tmC, a, stream) : launchPlainT<gemm::kEpiSwiGLU, 1>(tmA, tmB, tmC, a, stream);

@@ -101,6 +101,8 @@ def _cut_lib():
     (4096, 5160, 128, 0, (2, 256, 1)), (2560, 5160, 72, 0, (1, 240, 1)),  # the same with all rows
     (300, 325, 512, 0, (2, 160, 1)), (300, 321, 512, 0, (1, 64, 1)),  # TMA stores that end inside 16 bytes, after five elements and one
     (300, 650, 512, 1, (1, 128, 1)), (300, 386, 512, 1, (2, 256, 1)),
+    (15, 72, 200, 0, (1, 64, 1)), (16, 650, 512, 1, (1, 128, 1)), (17, 321, 512, 0, (1, 64, 1)), (64, 325, 1032, 0, (1, 96, 1)),  # tiles of 64 rows
+    (33, 512, 2048, 0, (1, 64, 2)), (48, 256, 1096, 1, (1, 128, 4)), (63, 100, 4096, 0, (1, 128, 8)), (65, 256, 1096, 1, (1, 128, 4)),
 ])
 def test_gemm_in_cut(M, N, K, epilogue, cut):
     """A given cut, in an output with a border that has to stay as it is; whole K gives the bits of every other cut."""
@@ -131,6 +133,25 @@ def test_gemm_in_cut(M, N, K, epilogue, cut):
     # as in test_gemm_cuts
     bound = ref.abs() * 2.0 ** -8 + K * 2.0 ** -24 * K * 0.013 * (8 if epilogue else 1) + 1e-6
     assert ((out.double() - ref).abs() <= bound).all()
+
+
+@gpu
+@pytest.mark.parametrize("epilogue,cut", [(0, (1, 48, 1)), (0, (1, 128, 4)), (1, (1, 96, 1)), (1, (1, 128, 2))])
+def test_gemm_rows_are_the_same_in_tiles_of_64_and_128_rows(epilogue, cut):
+    """64 rows take MMAs of 64 rows, 65 of 128: the 64 rows that both have are the same bits."""
+    import ctypes
+
+    lib = _cut_lib()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    N, K = 384, 2056
+    a = torch.randn(65, K, device="cuda", generator=g).to(torch.bfloat16)
+    b = (torch.randn(N, K, device="cuda", generator=g) * 0.02).to(torch.bfloat16)
+    out = torch.zeros(2, 65, N, device="cuda", dtype=torch.bfloat16)
+    for o, rows in zip(out, (64, 65)):
+        ptr = [ctypes.c_void_p(t.data_ptr()) for t in (a, b, o)]
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert lib.ucclTestGemmInCut(*ptr, rows, N, K, K, K, N, epilogue, (ctypes.c_int * 3)(*cut), stream) == 0
+    assert torch.equal(out[0, :64], out[1, :64]) and (out[0, 64] == 0).all() and bool(out[1, 64].any())
 
 
 def test_gemm_cut_choice_runs():
