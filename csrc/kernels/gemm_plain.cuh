@@ -32,6 +32,7 @@ namespace plain {
 
 constexpr int MAX_STAGES = 24;
 constexpr int MAX_CLUSTER = 8;
+constexpr int NARROW_PAIR = 192;  // pairs with tiles of up to this many columns issue as single CTAs do
 constexpr int SMEM = PIPE_BYTES + EPI_STAGE_BYTES + 1024 /*align slack*/ + 512 /*barriers*/;
 
 struct Args {
@@ -306,7 +307,7 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer: the warp stays converged (see the
     // pair kernel of gemm_sm100.cuh), one elected lane issues
-    if (CG == 2 && leader) {
+    if (CG == 2 && a.bn > NARROW_PAIR && leader) {
       const uint32_t idesc = ptx::umma_idesc_f16(1u, 2 * BM, static_cast<uint32_t>(a.bn));
       const bool issue = ptx::elect_one();
       int s = 0;
@@ -340,14 +341,15 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         __syncwarp();
       }
     }
-    if (CG == 1) {
-      // Single CTAs run the narrow tiles, whose four MMAs of a stage take about as long as the warp's wait for it, 200 cycles
-      // also where there is nothing to wait for.  So the next stage's barrier is looked at while this one is issued, and no
+    if (CG == 1 || (a.bn <= NARROW_PAIR && leader)) {
+      // Single CTAs and narrow pairs: the four MMAs of a stage take less than the warp's wait for it and the branch to the
+      // issuing lane, 360 cycles also where there is nothing to wait for.  So the next stage's barrier is looked at while this one is issued, and no
       // branch parts the MMAs from the warp.  Device time back to back: 1 x 4096 x 14336 23.5 -> 22.4 us, 64 x 4096 x 14336
       // 24.6 -> 23.7, 32 x 4096 x 4096 11.2 -> 10.6, 16 x 4096 x 1792 8.1 -> 7.8.  SwiGLU of a few rows with K below 600 loses by
-      // it: 8 x 512 x 256 3.09 -> 3.11 us, 32 x 1792 x 256 3.14 -> 3.16.  Pairs, whose MMAs are wider, gain and lose one or two
-      // percent by either and keep the plain form.
-      const uint32_t idesc = ptx::umma_idesc_f16(1u, static_cast<uint32_t>(4 * a.warp_rows), static_cast<uint32_t>(a.bn));
+      // it: 8 x 512 x 256 3.09 -> 3.11 us, 32 x 1792 x 256 3.14 -> 3.16.  Pairs of up to 192 columns: 512 x 4096 x 4096 21.3 ->
+      // 19.4, SwiGLU 405 x 48 x 4896 10.6 -> 9.7.  Wider ones, whose MMAs take longer than the wait, keep the plain form: SwiGLU
+      // 4096 x 7168 x 4096 (224 columns) 179.0 us with it, 180.6 without.
+      const uint32_t idesc = ptx::umma_idesc_f16(1u, static_cast<uint32_t>(CG * 4 * a.warp_rows), static_cast<uint32_t>(a.bn));
       const uint32_t act = ptx::elect_one() ? 1u : 0u, ring = ptx::smem_u32(smem), base = __shfl_sync(0xffffffffu, tmem_base, 0);
       int s = 0;
       uint32_t ph = 0, tcount = 0;
@@ -370,14 +372,18 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t koff = static_cast<uint64_t>((k * UMMA_K * 2) >> 4);
-            ptx::umma_f16_from(act, d_tmem, da + koff, db + koff, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+            const uint32_t accumulate = (kb != kb0 || k != 0) ? 1u : 0u;
+            if (CG == 2) ptx::umma_f16_pair_from(act, d_tmem, da + koff, db + koff, idesc, accumulate);
+            else ptx::umma_f16_from(act, d_tmem, da + koff, db + koff, idesc, accumulate);
           }
-          ptx::umma_commit_from(act, &empty_bar[s]);
+          if (CG == 2) ptx::umma_commit_both_from(act, &empty_bar[s], crank);
+          else ptx::umma_commit_from(act, &empty_bar[s]);
           there = __any_sync(0xffffffffu, seen != 0);
           s = next, ph = next_ph;
         }
         if (!ok) break;
-        ptx::umma_commit_from(act, &tfull_bar[acc]);
+        if (CG == 2) ptx::umma_commit_both_from(act, &tfull_bar[acc], crank);
+        else ptx::umma_commit_from(act, &tfull_bar[acc]);
       }
     }
   } else {

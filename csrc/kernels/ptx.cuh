@@ -489,6 +489,25 @@ __device__ __forceinline__ void umma_commit_both(uint64_t* bar, int leader = 0) 
                : "memory");
 }
 
+// Both from a whole warp of which one lane issues, as umma_f16_from.
+__device__ __forceinline__ void umma_f16_pair_from(uint32_t act, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(act)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_both_from(uint32_t act, uint64_t* bar, int leader) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
+      "h"(static_cast<uint16_t>(3 << leader)), "r"(act)
+      : "memory");
+}
+
 // ---------------------------------------------------------------- packed arithmetic
 // Two elements per instruction.
 __device__ __forceinline__ float2 mul2(float2 x, float2 y) {
