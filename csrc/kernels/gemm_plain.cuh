@@ -50,6 +50,7 @@ struct Args {
   int warp_rows;         // rows of a tile that a warp's TMEM lanes hold, from its first lane on: 32, or 16 of a 64-row tile
   int stages, stage_bytes;
   int split, workers;    // clusters in the grid; one tile each if split > 1
+  int x_rows, x_slot;    // split > 1: rows in a slot of the exchange buffer, bytes of a slot
   uint32_t* err;
 };
 
@@ -73,19 +74,21 @@ __device__ __forceinline__ void pack16(const uint32_t (&x)[16], const uint32_t (
     else o[j] = ptx::pack_bf16x2(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1]));
   }
 }
+__device__ __forceinline__ void store8(const Args& a, int row, int col, const uint4& o) {
+  __nv_bfloat16* p = a.C + static_cast<size_t>(row) * a.ldc + col;
+  if (col + 8 <= a.out_n) {
+    *reinterpret_cast<uint4*>(p) = o;
+  } else {
+    const uint32_t w[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (col + j < a.out_n) reinterpret_cast<uint16_t*>(p)[j] = static_cast<uint16_t>(w[j / 2] >> (16 * (j & 1)));
+  }
+}
 __device__ __forceinline__ void store16(const Args& a, int row, int col, const uint32_t (&o)[8]) {
   if (row >= a.M) return;
-  __nv_bfloat16* p = a.C + static_cast<size_t>(row) * a.ldc + col;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    if (col + h * 8 + 8 <= a.out_n) {
-      *reinterpret_cast<uint4*>(p + h * 8) = make_uint4(o[4 * h], o[4 * h + 1], o[4 * h + 2], o[4 * h + 3]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (col + h * 8 + j < a.out_n) reinterpret_cast<uint16_t*>(p)[h * 8 + j] = static_cast<uint16_t>(o[4 * h + j / 2] >> (16 * (j & 1)));
-    }
-  }
+  store8(a, row, col, make_uint4(o[0], o[1], o[2], o[3]));
+  if (col + 8 < a.out_n) store8(a, row, col + 8, make_uint4(o[4], o[5], o[6], o[7]));
 }
 
 // The whole tile of one warp (warp_rows rows from row0): 64 output columns at a time through shared memory and TMA
@@ -131,75 +134,98 @@ __device__ __forceinline__ void store_tile(const Args& a, const CUtensorMap* tmC
   }
 }
 
-// split > 1, after a cluster barrier that follows everybody's last MMA: part s of the cluster owns output columns
-// [s, s + 1) * out_bn / split.  Every warp hands the other parts their columns of its 32 rows (into the ring, which
-// is idle now: slot of the source, then 16-byte pieces of four columns, 128 rows of each), and after a second
-// barrier adds up what it got in the order of K.
-__device__ __forceinline__ uint32_t part_addr(const Args& a, uint32_t ring, int dst, int src, int halves, int piece, int r) {
-  const int slot = src < dst ? src : src - 1;
-  const int pieces = halves * (a.out_bn / a.split) / 4;
-  return ring + static_cast<uint32_t>(((slot * pieces + piece) * BM + r) * 16);
+// split > 1: part s of the cluster owns output columns [s, s + 1) * out_bn / split.  As soon as a CTA's own MMAs are done it lays
+// its sums out in its ring, which is idle then, a slot for each part, and sends the slots by bulk copies into buffers of the
+// other parts that their rings do not touch.  When its own slots are there, all threads of the CTA add up the parts in the
+// order of K, eight columns at a time.  A slot is pieces of four columns, x_rows rows of 16 bytes in each and 16 bytes
+// more, which spreads a warp's reads over the banks.
+//
+// Stores by the lanes move 10 to 20 bytes per cycle into another CTA, @@
+constexpr int X_END = PIPE_BYTES + EPI_STAGE_BYTES;  // the buffer ends here; the ring of a split launch ends where it begins
+__device__ __forceinline__ uint32_t x_offset(const Args& a, int dst, int src) {
+  return static_cast<uint32_t>(X_END - (a.split - 1 - (src < dst ? src : src - 1)) * a.x_slot);
 }
+// 16 accumulator columns into four pieces
+__device__ __forceinline__ void put_pieces(uint32_t to, int pitch, const uint32_t* x) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) ptx::st_shared_v4(to + j * pitch, make_uint4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]));
+}
+// `to`: this lane's row in the first piece of the first slot; the slots follow one another, and so do their pieces.  Lanes without
+// a row (live false) only take part in the reads.
 template <int EPI>
-__device__ __forceinline__ void send_parts(const Args& a, uint32_t ring, uint32_t taddr, int part, int rank0, int cg, int r) {
-  constexpr int H = EPI == kEpiSwiGLU ? 2 : 1;
-  const int w = a.out_bn / a.split;
+__device__ __forceinline__ void lay_out_parts(const Args& a, uint32_t to, uint32_t taddr, bool live) {
+  const int w = a.out_bn / a.split, pitch = a.x_rows * 16 + 16;
+  int dst = 0, up = 0, c = 0;  // SwiGLU: the slot of a part holds its gate columns, then its up columns
 #pragma unroll 1
-  for (int i = 1; i < a.split; ++i) {
-    const int dst = part + i < a.split ? part + i : part + i - a.split;
-    const uint32_t remote = ptx::mapa(ring, static_cast<uint32_t>(dst * cg + rank0));
-#pragma unroll 1
-    for (int c = 0; c < w; c += 16) {
-      uint32_t x[H][16];
+  for (int c0 = 0; c0 < a.bn; c0 += 64) {
+    uint32_t x[4][16];
+    const bool more = c0 + 32 < a.bn;  // bn is a multiple of 32
 #pragma unroll
-      for (int h = 0; h < H; ++h) ptx::tmem_ld_32x32b_x16(taddr + h * a.out_bn + dst * w + c, x[h]);
-      ptx::tmem_ld_wait();
-      if ((r & 31) >= a.warp_rows) continue;
-#pragma unroll
-      for (int h = 0; h < H; ++h)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          ptx::st_cluster_v4(part_addr(a, remote, dst, part, H, (h * w + c) / 4 + j, r),
-                             make_uint4(x[h][4 * j], x[h][4 * j + 1], x[h][4 * j + 2], x[h][4 * j + 3]));
+    for (int u = 0; u < 4; ++u) {
+      if (u >= 2 && !more) break;
+      if constexpr (EPI == kEpiSwiGLU) {
+        ptx::tmem_ld_32x32b_x16(taddr + up * a.out_bn + dst * w + c, x[u]);
+        if ((c += 16) == w) c = 0, dst += up, up ^= 1;
+      } else {
+        ptx::tmem_ld_32x32b_x16(taddr + c0 + u * 16, x[u]);
+      }
     }
+    ptx::tmem_ld_wait();
+    if (live) {
+      put_pieces(to, pitch, x[0]);
+      put_pieces(to + 4 * pitch, pitch, x[1]);
+      if (more) put_pieces(to + 8 * pitch, pitch, x[2]);
+      if (more) put_pieces(to + 12 * pitch, pitch, x[3]);
+    }
+    to += 16 * pitch;
+    __syncwarp();
   }
 }
+// `rows` rows of the tile, from row m0 of C on.  A thread keeps to its eight columns.
 template <int EPI>
-__device__ __forceinline__ void sum_parts(const Args& a, const uint8_t* ring, uint32_t taddr, int part, int row, int col0, int r) {
+__device__ __forceinline__ void sum_parts(const Args& a, uint32_t smem, int part, int m0, int rows, int col0) {
   constexpr int H = EPI == kEpiSwiGLU ? 2 : 1;
-  const int w = a.out_bn / a.split;
+  const int w = a.out_bn / a.split, groups = w / 8, pitch = a.x_rows * 16 + 16, step = NUM_THREADS / groups;
+  const int first = threadIdx.x / groups, g = threadIdx.x - first * groups, col = col0 + part * w + g * 8;
+  if (first >= step || col >= a.out_n) return;
+  const uint32_t own = smem + static_cast<uint32_t>(part * a.x_slot + 2 * g * pitch), got = smem + x_offset(a, part, part ? 0 : 1) + 2 * g * pitch;
+#pragma unroll 2
+  for (int row = first; row < rows; row += step) {
+    float sum[H][8];
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const uint32_t at = static_cast<uint32_t>(h * (w / 4) * pitch + row * 16);
 #pragma unroll 1
-  for (int c = 0; c < w && col0 + part * w + c < a.out_n; c += 16) {
-    uint32_t own[H][16];
-    float sum[H][16];
+      for (int s0 = 0; s0 < a.split; s0 += 4) {  // the reads of four parts are out before the first is added
+        float4 v[4][2];
 #pragma unroll
-    for (int h = 0; h < H; ++h) ptx::tmem_ld_32x32b_x16(taddr + h * a.out_bn + part * w + c, own[h]);
-    ptx::tmem_ld_wait();
-#pragma unroll 1
-    for (int s = 0; s < a.split; ++s) {
+        for (int s = 0; s < 4; ++s) {
+          if (s0 + s >= a.split) break;
+          const uint32_t from = at + (s0 + s == part ? own : got + (s0 + s - (s0 + s > part ? 1 : 0)) * a.x_slot);
+          v[s][0] = ptx::ld_shared_f4(from);
+          v[s][1] = ptx::ld_shared_f4(from + pitch);
+        }
 #pragma unroll
-      for (int h = 0; h < H; ++h) {
+        for (int s = 0; s < 4; ++s) {
+          if (s0 + s >= a.split) break;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float4 v;
-          if (s == part) v = make_float4(__uint_as_float(own[h][4 * j]), __uint_as_float(own[h][4 * j + 1]), __uint_as_float(own[h][4 * j + 2]), __uint_as_float(own[h][4 * j + 3]));
-          else v = *reinterpret_cast<const float4*>(ring + part_addr(a, 0, part, s, H, (h * w + c) / 4 + j, r));
-          sum[h][4 * j] = s == 0 ? v.x : sum[h][4 * j] + v.x;
-          sum[h][4 * j + 1] = s == 0 ? v.y : sum[h][4 * j + 1] + v.y;
-          sum[h][4 * j + 2] = s == 0 ? v.z : sum[h][4 * j + 2] + v.z;
-          sum[h][4 * j + 3] = s == 0 ? v.w : sum[h][4 * j + 3] + v.w;
+          for (int j = 0; j < 2; ++j) {
+            const bool start = s0 + s == 0;
+            sum[h][4 * j] = start ? v[s][j].x : sum[h][4 * j] + v[s][j].x;
+            sum[h][4 * j + 1] = start ? v[s][j].y : sum[h][4 * j + 1] + v[s][j].y;
+            sum[h][4 * j + 2] = start ? v[s][j].z : sum[h][4 * j + 2] + v[s][j].z;
+            sum[h][4 * j + 3] = start ? v[s][j].w : sum[h][4 * j + 3] + v[s][j].w;
+          }
         }
       }
     }
-    uint32_t x[16], y[16], o[8];
+    uint32_t o[4];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      x[j] = __float_as_uint(sum[0][j]);
-      y[j] = __float_as_uint(sum[H - 1][j]);
+    for (int j = 0; j < 4; ++j) {
+      if (EPI == kEpiSwiGLU) o[j] = swiglu2(make_float2(sum[0][2 * j], sum[0][2 * j + 1]), make_float2(sum[H - 1][2 * j], sum[H - 1][2 * j + 1]));
+      else o[j] = ptx::pack_bf16x2(sum[0][2 * j], sum[0][2 * j + 1]);
     }
-    pack16<EPI>(x, y, o);
-    store16(a, row, col0 + part * w + c, o);
-    __syncwarp();
+    store8(a, m0 + row, col, make_uint4(o[0], o[1], o[2], o[3]));
   }
 }
 
@@ -215,6 +241,7 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint64_t* tempty_bar = tfull_bar + 2;  // CG 2: used in the leader
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile uint32_t* bail = tmem_holder + 1;
+  uint64_t* parts_bar = reinterpret_cast<uint64_t*>(tmem_holder + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int csize = CG * a.split;
@@ -225,6 +252,15 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int kb0 = a.split > 1 ? a.num_kb * part / a.split : 0;
   const int kb1 = a.split > 1 ? a.num_kb * (part + 1) / a.split : a.num_kb;
 
+  // The first tile's place takes divisions: done while the launch before runs, not between its end and the first load.
+  int first_mt, first_nt;
+  coords<CG == 2 ? 8 : 16>(a, worker, first_mt, first_nt);
+  const int tile_rows = min(a.M - (first_mt * CG + half) * BM, 4 * a.warp_rows);  // of the first tile, may be none
+  const int part_cols = a.out_bn / a.split;
+  // whether part p of this tile has something to add up
+  auto has_columns = [&](int p) { return tile_rows > 0 && first_nt * a.out_bn + p * part_cols < a.out_n; };
+  const bool takes_parts = a.split > 1 && has_columns(part);
+
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.stages; ++s) {
       ptx::mbar_init(&full_bar[s], 1);
@@ -233,6 +269,10 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&tfull_bar[i], 1);
       ptx::mbar_init(&tempty_bar[i], 4 * CG);
+    }
+    if (takes_parts) {
+      ptx::mbar_init(parts_bar, 1);
+      ptx::mbar_expect_tx(parts_bar, static_cast<uint32_t>((a.split - 1) * a.x_slot));
     }
     *bail = 0;
     ptx::mbar_fence_init();
@@ -251,12 +291,11 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   }
   ptx::tc_fence_before();
   __syncthreads();
-  if (CG == 2) ptx::cluster_sync();  // both CTAs' barriers and TMEM exist before anybody signals the other
+  // both CTAs' barriers and TMEM exist before anybody signals the other; parts in single CTAs wait for that when they need it
+  if (CG == 2) ptx::cluster_sync();
+  else if (a.split > 1) ptx::cluster_arrive();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  // The first tile's place takes divisions: done while the launch before runs, not between its end and the first load.
-  int first_mt, first_nt;
-  coords<CG == 2 ? 8 : 16>(a, worker, first_mt, first_nt);
   // Everything up to here may run while the launch before is still at work; no operand is read and C not
   // touched before that one has ended.
   ptx::launch_dependents();
@@ -415,21 +454,31 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   ptx::tc_fence_before();
   __syncthreads();
   if (a.split > 1) {
-    const int mt = first_mt, nt = first_nt;
-    const int q = warp & 3, r = q * 32 + lane, row0 = (mt * CG + half) * BM + q * a.warp_rows;
-    const int row = lane < a.warp_rows ? row0 + lane : a.M;
-    const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-    const bool busy = warp >= 2 && row0 < a.M;
-    ptx::cluster_sync();  // every part has used up its ring
+    const int q = warp & 3, row = q * a.warp_rows + lane;
     ptx::tc_fence_after();
-    if (busy) send_parts<EPI>(a, ptx::smem_u32(smem), taddr, part, half, CG, r);
-    __syncwarp();
-    ptx::cluster_sync();
-    if (busy) sum_parts<EPI>(a, smem, taddr, part, row, nt * a.out_bn, r);
+    if (warp >= 2 && row - lane < tile_rows)
+      lay_out_parts<EPI>(a, ptx::smem_u32(smem) + row * 16, tmem_base + (static_cast<uint32_t>(q * 32) << 16), lane < a.warp_rows && row < tile_rows);
+    ptx::fence_proxy_async_smem();
+    if (CG == 1) ptx::cluster_wait();  // the other CTAs' barriers exist
     ptx::tc_fence_before();
     __syncthreads();
+    if (ptx::elect_one()) {
+      for (int p = warp; p < a.split; p += NUM_THREADS / 32)
+        if (p != part && has_columns(p)) {
+          const uint32_t rank = static_cast<uint32_t>(p * CG + half), ring = ptx::smem_u32(smem);
+          ptx::bulk_copy_cluster(ptx::mapa(ring + x_offset(a, p, part), rank), ring + p * a.x_slot, a.x_slot, ptx::mapa(ptx::smem_u32(parts_bar), rank));
+        }
+    }
+    __syncwarp();
+    const bool there = !takes_parts || ptx::mbar_wait_bounded(parts_bar, 0, bail);
+    __syncwarp();
+    ptx::cluster_arrive_relaxed();
+    if (takes_parts && there) sum_parts<EPI>(a, ptx::smem_u32(smem), part, (first_mt * CG + half) * BM, tile_rows, first_nt * a.out_bn);
+    __syncwarp();
+    ptx::cluster_wait();  // nobody leaves before all have got what this CTA sent
+  } else if (CG == 2) {
+    ptx::cluster_sync();  // nobody leaves while the other CTA may still signal it or read its memory
   }
-  if (CG == 2) ptx::cluster_sync();  // nobody leaves while the other CTA may still signal it or read its memory
   if (warp == 1) {
     ptx::tc_fence_after();
     if (CG == 2) ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS);

@@ -36,6 +36,14 @@ int cutStep(int cg, bool swiglu) { return cg == 2 || swiglu ? 32 : 16; }
 
 }  // namespace
 
+namespace {
+// Rows of a tile that the parts exchange, and whether what a CTA sends and what it gets have room side by side.
+int exchangeRows(int M, int cg) { return std::min((M + 7) / 8 * 8, cg == 1 && M <= 64 ? 64 : gemm::BM); }
+bool exchangeFits(const GemmCut& c, int M) {
+  return c.split == 1 || (2 * c.split - 1) * (c.bn / c.split / 4) * (exchangeRows(M, c.cg) * 16 + 16) <= gemm::plain::X_END;
+}
+}  // namespace
+
 bool gemmCutRuns(const GemmCut& c, int K, bool swiglu) {
   if (c.cg != 1 && c.cg != 2) return false;
   if (c.bn < 16 || c.bn > gemm::BN || c.bn % cutStep(c.cg, swiglu) != 0) return false;
@@ -181,7 +189,7 @@ GemmCut choosePlain(int M, int N, int K, bool swiglu) {
       const int kbs = (num_kb + split - 1) / split;
       for (int bn = step; bn <= gemm::BN; bn += step) {
         const int out_bn = swiglu ? bn / 2 : bn;
-        if (!gemmCutRuns({cg, bn, split}, K, swiglu)) continue;
+        if (!gemmCutRuns({cg, bn, split}, K, swiglu) || !exchangeFits({cg, bn, split}, M)) continue;
         const int tiles = tiles_m * ((out_n + out_bn - 1) / out_bn);
         if (split > 1 && tiles > resident) continue;
         const int waves = (tiles + resident - 1) / resident;
@@ -259,7 +267,8 @@ ucclResult_t launchPlain(const GemmLaunch& g, const GemmCut* cut, cudaStream_t s
   const bool swiglu = g.epilogue == gemm::kEpiSwiGLU;
   const int out_n = swiglu ? g.N / 2 : g.N;
   if (cut && !gemmCutRuns(*cut, g.K, swiglu)) return ucclInvalidArgument;
-  const GemmCut p = cut ? *cut : cutFor(g.M, g.N, g.K, swiglu);
+  GemmCut p = cut ? *cut : cutFor(g.M, g.N, g.K, swiglu);
+  while (!exchangeFits(p, g.M)) p.split /= 2;  // of the cuts that may be asked for, 256 columns of 128 rows in four parts or more
   gemm::plain::Args a = {};
   a.C = static_cast<__nv_bfloat16*>(g.C);
   a.ldc = g.ldc;
@@ -275,8 +284,12 @@ ucclResult_t launchPlain(const GemmLaunch& g, const GemmCut* cut, cudaStream_t s
   a.tiles_n = (out_n + a.out_bn - 1) / a.out_bn;
   a.num_tiles = a.tiles_m * a.tiles_n;
   a.stage_bytes = (a.a_rows + p.bn / p.cg) * gemm::BK * 2;
-  a.stages = std::min(gemm::plain::MAX_STAGES, gemm::PIPE_BYTES / a.stage_bytes);
+  // parts: no staging of the output, that room and the ring's end are the exchange buffer
   a.split = p.split;
+  a.x_rows = exchangeRows(g.M, p.cg);
+  a.x_slot = p.bn / p.split / 4 * (a.x_rows * 16 + 16);
+  const int ring = p.split > 1 ? gemm::plain::X_END - (p.split - 1) * a.x_slot : gemm::PIPE_BYTES;
+  a.stages = std::min(gemm::plain::MAX_STAGES, ring / a.stage_bytes);
   a.err = g.err;
   // the stride of a single row means nothing; rows that overlap have no tensor map
   const int ldc = g.M == 1 ? (out_n + 7) / 8 * 8 : g.ldc;
