@@ -140,7 +140,11 @@ __device__ __forceinline__ void store_tile(const Args& a, const CUtensorMap* tmC
 // order of K, eight columns at a time.  A slot is pieces of four columns, x_rows rows of 16 bytes in each and 16 bytes
 // more, which spreads a warp's reads over the banks.
 //
-// Stores by the lanes move 10 to 20 bytes per cycle into another CTA, @@
+// Bound by latencies and by instructions that stand one behind the other.  Before, the lanes stored into the other parts' rings
+// between two cluster barriers (10 to 20 bytes per cycle and CTA) and the warps that hold the rows added up, with an integer
+// division for every 16 columns: 46 x 8 x 4800 in eight parts 6.7 -> 5.2 us, 7 x 2040 x 10816 15.5 -> 12.8, MLP of 2 x 4096 x 3584
+// 24.7 -> 22.6, 64 x 4096 x 14336 in four parts 24.5 -> 24.0, 300 x 4096 x 7168 in two parts of 192 columns 31.3 -> 31.3.  The ring is
+// shorter by what the slots take.
 constexpr int X_END = PIPE_BYTES + EPI_STAGE_BYTES;  // the buffer ends here; the ring of a split launch ends where it begins
 __device__ __forceinline__ uint32_t x_offset(const Args& a, int dst, int src) {
   return static_cast<uint32_t>(X_END - (a.split - 1 - (src < dst ? src : src - 1)) * a.x_slot);
@@ -189,33 +193,22 @@ __device__ __forceinline__ void sum_parts(const Args& a, uint32_t smem, int part
   const int first = threadIdx.x / groups, g = threadIdx.x - first * groups, col = col0 + part * w + g * 8;
   if (first >= step || col >= a.out_n) return;
   const uint32_t own = smem + static_cast<uint32_t>(part * a.x_slot + 2 * g * pitch), got = smem + x_offset(a, part, part ? 0 : 1) + 2 * g * pitch;
-#pragma unroll 2
+#pragma unroll 1
   for (int row = first; row < rows; row += step) {
     float sum[H][8];
 #pragma unroll
     for (int h = 0; h < H; ++h) {
       const uint32_t at = static_cast<uint32_t>(h * (w / 4) * pitch + row * 16);
-#pragma unroll 1
-      for (int s0 = 0; s0 < a.split; s0 += 4) {  // the reads of four parts are out before the first is added
-        float4 v[4][2];
+#pragma unroll 2
+      for (int s = 0; s < a.split; ++s) {
+        const uint32_t from = at + (s == part ? own : got + (s - (s > part ? 1 : 0)) * a.x_slot);
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          if (s0 + s >= a.split) break;
-          const uint32_t from = at + (s0 + s == part ? own : got + (s0 + s - (s0 + s > part ? 1 : 0)) * a.x_slot);
-          v[s][0] = ptx::ld_shared_f4(from);
-          v[s][1] = ptx::ld_shared_f4(from + pitch);
-        }
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          if (s0 + s >= a.split) break;
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const bool start = s0 + s == 0;
-            sum[h][4 * j] = start ? v[s][j].x : sum[h][4 * j] + v[s][j].x;
-            sum[h][4 * j + 1] = start ? v[s][j].y : sum[h][4 * j + 1] + v[s][j].y;
-            sum[h][4 * j + 2] = start ? v[s][j].z : sum[h][4 * j + 2] + v[s][j].z;
-            sum[h][4 * j + 3] = start ? v[s][j].w : sum[h][4 * j + 3] + v[s][j].w;
-          }
+        for (int j = 0; j < 2; ++j) {
+          const float4 v = ptx::ld_shared_f4(from + j * pitch);
+          sum[h][4 * j] = s == 0 ? v.x : sum[h][4 * j] + v.x;
+          sum[h][4 * j + 1] = s == 0 ? v.y : sum[h][4 * j + 1] + v.y;
+          sum[h][4 * j + 2] = s == 0 ? v.z : sum[h][4 * j + 2] + v.z;
+          sum[h][4 * j + 3] = s == 0 ? v.w : sum[h][4 * j + 3] + v.w;
         }
       }
     }
@@ -242,6 +235,7 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile uint32_t* bail = tmem_holder + 1;
   uint64_t* parts_bar = reinterpret_cast<uint64_t*>(tmem_holder + 2);
+  volatile int* tail = reinterpret_cast<volatile int*>(parts_bar + 1);  // what a tile in parts needs after its main loop
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int csize = CG * a.split;
@@ -256,10 +250,7 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   int first_mt, first_nt;
   coords<CG == 2 ? 8 : 16>(a, worker, first_mt, first_nt);
   const int tile_rows = min(a.M - (first_mt * CG + half) * BM, 4 * a.warp_rows);  // of the first tile, may be none
-  const int part_cols = a.out_bn / a.split;
-  // whether part p of this tile has something to add up
-  auto has_columns = [&](int p) { return tile_rows > 0 && first_nt * a.out_bn + p * part_cols < a.out_n; };
-  const bool takes_parts = a.split > 1 && has_columns(part);
+  const bool takes_parts = a.split > 1 && tile_rows > 0 && first_nt * a.out_bn + part * (a.out_bn / a.split) < a.out_n;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.stages; ++s) {
@@ -269,6 +260,11 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&tfull_bar[i], 1);
       ptx::mbar_init(&tempty_bar[i], 4 * CG);
+    }
+    if (a.split > 1) {
+      tail[0] = tile_rows;
+      tail[1] = first_nt * a.out_bn;
+      tail[2] = (first_mt * CG + half) * BM;
     }
     if (takes_parts) {
       ptx::mbar_init(parts_bar, 1);
@@ -447,17 +443,19 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         else ptx::mbar_arrive(&tempty_bar[acc]);
       }
     }
-    if (lane == 0) ptx::tma_store_wait<0>();  // staging buffers stay valid until read
+    if (ptx::elect_one()) ptx::tma_store_wait<0>();  // staging buffers stay valid until read
     __syncwarp();
   }
 
   ptx::tc_fence_before();
   __syncthreads();
   if (a.split > 1) {
+    const int rows = tail[0], col0 = tail[1], m0 = tail[2], part_cols = a.out_bn / a.split;
+    auto has_columns = [&](int p) { return rows > 0 && col0 + p * part_cols < a.out_n; };  // whether part p has something to add up
     const int q = warp & 3, row = q * a.warp_rows + lane;
     ptx::tc_fence_after();
-    if (warp >= 2 && row - lane < tile_rows)
-      lay_out_parts<EPI>(a, ptx::smem_u32(smem) + row * 16, tmem_base + (static_cast<uint32_t>(q * 32) << 16), lane < a.warp_rows && row < tile_rows);
+    if (warp >= 2 && row - lane < rows)
+      lay_out_parts<EPI>(a, ptx::smem_u32(smem) + row * 16, tmem_base + (static_cast<uint32_t>(q * 32) << 16), lane < a.warp_rows && row < rows);
     ptx::fence_proxy_async_smem();
     if (CG == 1) ptx::cluster_wait();  // the other CTAs' barriers exist
     ptx::tc_fence_before();
@@ -470,10 +468,10 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         }
     }
     __syncwarp();
-    const bool there = !takes_parts || ptx::mbar_wait_bounded(parts_bar, 0, bail);
+    const bool takes = has_columns(part), there = !takes || ptx::mbar_wait_bounded(parts_bar, 0, bail);
     __syncwarp();
     ptx::cluster_arrive_relaxed();
-    if (takes_parts && there) sum_parts<EPI>(a, ptx::smem_u32(smem), part, (first_mt * CG + half) * BM, tile_rows, first_nt * a.out_bn);
+    if (takes && there) sum_parts<EPI>(a, ptx::smem_u32(smem), part, m0, rows, col0);
     __syncwarp();
     ptx::cluster_wait();  // nobody leaves before all have got what this CTA sent
   } else if (CG == 2) {

@@ -662,12 +662,14 @@ constexpr int kMostThreads = EPI == kEpiSwiGLU ? SWIGLU_BOUND : COMM == kCommAll
 
 // ------------------------------------------------------------------ epilogue of one tile, one warp
 // 64 columns x 32 rows of bf16 (eight 16-byte pieces per lane) -> 128-byte-swizzled staging buffer
-// -> one TMA store at (col0, row0) of `map`.  One bulk group per stage_take and stage_send.
+// -> one TMA store at (col0, row0) of `map`.  One bulk group per stage_take and stage_send.  The lane is elected, always the same
+// one: behind `lane == 0` the compiler does not take the branch for uniform, and a TMA instruction costs 100 cycles (16384 x
+// 4096 x 128 33.1 -> 32.8 us, SwiGLU 4096 x 28672 x 64 68.0 -> 66.8).
 template <int NBUF>
 __device__ __forceinline__ uint8_t* stage_take(uint8_t* stage, uint32_t& stage_it, int lane) {
   uint8_t* buf = stage + (stage_it % NBUF) * EPI_BUF_BYTES;
   ++stage_it;
-  if (lane == 0) ptx::tma_store_wait_read<NBUF - 1>();  // the store that last used this buffer has read it
+  if (ptx::elect_one()) ptx::tma_store_wait_read<NBUF - 1>();  // the store that last used this buffer has read it
   __syncwarp();
   return buf;
 }
@@ -677,8 +679,10 @@ __device__ __forceinline__ void stage_put(uint8_t* buf, int lane, int k, uint4 v
 __device__ __forceinline__ void stage_send(const CUtensorMap* map, uint8_t* buf, int col0, int row0, bool inside, int lane) {
   ptx::fence_proxy_async_smem();
   __syncwarp();
-  if (lane == 0 && inside) ptx::tma_store_2d(map, buf, col0, row0);
-  if (lane == 0) ptx::tma_store_commit();
+  if (ptx::elect_one()) {
+    if (inside) ptx::tma_store_2d(map, buf, col0, row0);
+    ptx::tma_store_commit();
+  }
 }
 template <int NBUF>
 __device__ __forceinline__ void stage_and_store(const CUtensorMap* map, const uint4 (&v)[8], int col0, int row0, bool inside,
