@@ -155,24 +155,20 @@ bool usePairKernel() {
 // How to cut a GEMM without a collective: the candidate with the fewest cycles by one of two formulas.
 //
 // A tile whole: waves of tiles x the longer of a tile's main loop and of the epilogue that runs beside the next tile's
-// (2150 cycles, and per output column 11, or 49 with silu); at least the time of memory, and at least that of all loads
-// together (9000 bytes per cycle into all SMs).  A stage of the main loop takes what the tensor cores need for it (two
-// cycles per accumulator column, at least a round trip of the ring) or its loads (65 bytes per cycle and SM).  A tile in
-// parts of K: the same without the overlapped epilogue (one tile per cluster), plus the exchange of the parts.
+// (2470 cycles, and per output column 15, or 23 with silu, and 400 if columns are left beside the blocks of 64 that TMA stores
+// take); at least the time of memory, and at least that of all loads together (9000 bytes per cycle into all SMs).  A stage of
+// the main loop takes what the tensor cores need for it (two cycles per accumulator column, at least what a stage takes to
+// issue) or its loads (66 bytes per cycle and SM).  A tile in parts of K: the same without the overlapped epilogue (one tile per
+// cluster), plus the exchange of the parts.  Up to 64 rows are not for pairs: their 256 rows would be at most a quarter full.
 //
-// The constants are fits to measurements with every candidate timed on operands that are not in L2: whole tiles to
-// 658 shapes (1 to 16384 rows, K of 64 to 14336), where the choice takes 1.2% more than the best candidate on average (an
-// earlier formula without the epilogue and the common load rate: 2.4%, and 20% on 4096 x 28672 x 512), the parts to 102
-// of them; with the issuer and the epilogue as they are now, the choice takes 0.6% more than the best candidate on 200
-// other shapes.  Both sides of some of the lines, in us, when they were fitted: 64 x 4096 x 14336 25.3 in four parts of 128 columns, 62 uncut;
-// 4096 x 28672 x 512 111 in pair tiles of 256, 125 of 224; 8192 x 3592 x 4104 207 in pair tiles of 256, 244 of 192;
-// 200 x 28672 x 4096 51.6 in pair tiles of 224, 60.2 in single CTAs of 208; 512 x 4096 x 4096 20 in tiles of 128, 25 of 256.
-//
-// The 49 cycles are those of the division that the epilogue once had.  The silu of today takes about 25 (4096 x 28672 x 64
-// 69 us, 16384 x 4096 x 128 40 us, both bound by it), and the fit has not been made anew.  What that costs, on 40 SwiGLU
-// shapes with K of 64 to 1024: 32 are cut as the best candidate and four more lose up to 2.1%; 2 x 12752 x 72 goes into two
-// parts and takes 6.5 us, 4.1 in whole tiles of 96; 10605 x 320 x 520 12.5 and 11.1, 1 x 1152 x 872 6.0 and 5.5, 9373 x 4208 x
-// 824 66.1 and 61.9.
+// The constants are fits to measurements with every candidate timed on operands that are not in L2: 500 shapes (1 to 16384
+// rows, K of 64 to 14336, with and without SwiGLU, up to 250 us), where the choice takes 1.1% more than the best candidate on average
+// and 7% in the worst twentieth (the constants for the kernel as it was before its producer, its small MMAs and its exchange of
+// parts: 2.4% and 12%).  Both sides of some of the lines, in us: 6 x 5088 x 3552 9.8 in single CTAs in four parts of 192 columns,
+// 13.6 in pairs in two parts of 160; SwiGLU 1 x 1648 x 2728 6.0 and 8.2; 64 x 4096 x 14336 23.0 in four parts of 128, 23.3 in two
+// of 64; 512 x 4096 x 4096 16.7 in pairs of 128 columns, 18.3 in single CTAs of 128; 16384 x 4096 x 128 28.8 in tiles of 192, 31.5
+// of 224; 4096 x 7168 x 4096 SwiGLU 156 in pairs of 224, 174 of 256.  Not told apart: SwiGLU 356 x 720 x 1000 11.0 in tiles of
+// 32 columns, 8.4 in pairs in four parts.
 GemmCut choosePlain(int M, int N, int K, bool swiglu) {
   GemmCut best = {1, 256, 1};
   const bool pairs = usePairKernel();
@@ -180,7 +176,7 @@ GemmCut choosePlain(int M, int N, int K, bool swiglu) {
   const int out_n = swiglu ? N / 2 : N;
   const double bytes = 2.0 * (static_cast<double>(M) * K + static_cast<double>(N) * K + static_cast<double>(M) * out_n);
   double best_t = 1e300;
-  for (int cg = 1; cg <= (pairs ? 2 : 1); ++cg) {
+  for (int cg = 1; cg <= (pairs && M > 64 ? 2 : 1); ++cg) {
     const int tiles_m = (M + cg * gemm::BM - 1) / (cg * gemm::BM);
     const int a_rows = cg == 1 && M < gemm::BM ? (M + 7) / 8 * 8 : gemm::BM;
     const int step = cutStep(cg, swiglu);
@@ -194,17 +190,17 @@ GemmCut choosePlain(int M, int N, int K, bool swiglu) {
         if (split > 1 && tiles > resident) continue;
         const int waves = (tiles + resident - 1) / resident;
         const int ctas = std::min(tiles, resident) * cg * split;
-        const double mma = std::max(2.0 * bn, 329.0) + 54.0, stage_bytes = (a_rows + bn / cg) * 128.0;
+        const double mma = std::max(2.0 * bn, 306.0) + 65.0, stage_bytes = (a_rows + bn / cg) * 128.0;
         double t;
         if (split == 1) {
-          const double stage = std::max(mma, stage_bytes / 65.0), epilogue = 2150.0 + (swiglu ? 49.0 : 11.0) * out_bn;
+          const double stage = std::max(mma, stage_bytes / 66.5), epilogue = 2470.0 + (swiglu ? 23.3 : 15.2) * out_bn + (out_bn > 64 && out_bn % 64 ? 406.0 : 0.0);
           const double memory = bytes / std::min(6100.0, ctas * 41.0);
           const double loads = static_cast<double>(tiles) * cg * num_kb * stage_bytes / 9000.0;
           t = std::max(std::max(memory, loads), waves * std::max(num_kb * stage + 34.0, epilogue)) + 0.1 * epilogue;
         } else {
-          const double stage = std::max(mma, stage_bytes / 78.0);
-          const double memory = bytes / std::min(3500.0, ctas * 83.0);
-          t = std::max(memory, waves * kbs * stage) + waves * 34.0 + 3100.0 + 280.0 * split + 30.0 * bn * std::min(M, cg * gemm::BM) / (cg * gemm::BM);
+          const double stage = std::max(mma, stage_bytes / 72.7);
+          const double memory = bytes / std::min(3500.0, ctas * 98.4);
+          t = std::max(memory, waves * kbs * stage) + waves * 34.0 + 2250.0 + 385.0 * split + 29.8 * bn * std::min(M, cg * gemm::BM) / (cg * gemm::BM);
         }
         if (t < best_t) {
           best_t = t;
