@@ -1052,7 +1052,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
     if (COMM == kCommReduceScatter && tcount > 0) publish_tile<0>(a, prev_mb, lane, &warps_done[(tcount - 1) & 3]);
-    if (COMM != kCommReduceScatter && a.epi_tma && lane == 0) ptx::tma_store_wait<0>();  // staging buffers stay valid until read
+    if (COMM != kCommReduceScatter && a.epi_tma && ptx::elect_one()) ptx::tma_store_wait<0>();  // by the lane of stage_send; staging buffers stay valid until read
   }
 
   ptx::tc_fence_before();
@@ -1271,7 +1271,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
     }
     if (COMM == kCommReduceScatter && tcount > 0) publish_tile<0>(a, prev_mb, lane, &warps_done[(tcount - 1) & 3]);
-    if (COMM != kCommReduceScatter && a.epi_tma && lane == 0) ptx::tma_store_wait<0>();  // staging buffers stay valid until read
+    if (COMM != kCommReduceScatter && a.epi_tma && ptx::elect_one()) ptx::tma_store_wait<0>();  // by the lane of stage_send; staging buffers stay valid until read
   }
 
   ptx::tc_fence_before();
