@@ -255,9 +255,9 @@ __device__ __forceinline__ void cast_share(const CastLocalArgs& a, size_t first)
   }
 }
 // Pieces per thread of a large launch, and CTAs per SM.  A conversion to fp8 takes some eighty instructions a piece, and
-// two pieces on six CTAs put more of them beside other CTAs' loads than four pieces on four: 64 Mi bf16 33.0 -> 31.4 us, 16 Mi
-// 11.4 -> 10.1, 6 Mi fp32 6.7 -> 5.8 (measured with a longer quotient, and five CTAs then slower than six: 64 Mi bf16 31.5 and
-// 31.1 us, 32 Mi fp32 26.4 and 25.3); with the rest, bound by its loads and stores, it is the same.
+// two pieces on six CTAs (40 registers) put more of them beside other CTAs' loads than four pieces on four or two on five: 64 Mi bf16
+// 31.1, 31.8 and 32.0 us, 16 Mi 9.2, 10.2 and 9.4, 32 Mi fp32 25.6, 26.4 and 25.6, 20 Mi fp16 10.9, 11.8 and 11.0.  Seven CTAs spill:
+// 34.2, 10.2, 25.9, 13.1 (6 Mi fp32 alone is faster, 4.58 and 4.73).  With the other types, bound by loads and stores, it is the same.
 template <int OUT>
 constexpr int kCastPieces = OUT == OUT_FP8 ? 2 : 4;
 template <int DT, int OUT, int U>
