@@ -137,8 +137,8 @@ __device__ __forceinline__ void store_tile(const Args& a, const CUtensorMap* tmC
 // split > 1: part s of the cluster owns output columns [s, s + 1) * out_bn / split.  As soon as a CTA's own MMAs are done it lays
 // its sums out in its ring, which is idle then, a slot for each part, and sends the slots by bulk copies into buffers of the
 // other parts that their rings do not touch.  When its own slots are there, all threads of the CTA add up the parts in the
-// order of K, eight columns at a time.  A slot is pieces of four columns, x_rows rows of 16 bytes in each and 16 bytes
-// more, which spreads a warp's reads over the banks.
+// order of K, eight columns at a time.  A slot is pieces of four columns with x_rows rows of 16 bytes in each; the rows of every
+// second pair of pieces change places within eight (row ^ pair), which spreads a warp's reads over the banks.
 //
 // Bound by latencies and by instructions that stand one behind the other.  Before, the lanes stored into the other parts' rings
 // between two cluster barriers (10 to 20 bytes per cycle and CTA) and the warps that hold the rows added up, with an integer
@@ -149,16 +149,19 @@ constexpr int X_END = PIPE_BYTES + EPI_STAGE_BYTES;  // the buffer ends here; th
 __device__ __forceinline__ uint32_t x_offset(const Args& a, int dst, int src) {
   return static_cast<uint32_t>(X_END - (a.split - 1 - (src < dst ? src : src - 1)) * a.x_slot);
 }
-// 16 accumulator columns into four pieces
-__device__ __forceinline__ void put_pieces(uint32_t to, int pitch, const uint32_t* x) {
+// 16 accumulator columns, the U-th of four in a row, into their four pieces; `row16`: the lane's row times 16
+template <int U>
+__device__ __forceinline__ void put_pieces(uint32_t to, int pitch, uint32_t row16, const uint32_t (&x)[16]) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) ptx::st_shared_v4(to + j * pitch, make_uint4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]));
+  for (int j = 0; j < 4; ++j)
+    ptx::st_shared_v4(to + (4 * U + j) * pitch + (row16 ^ ((2 * U + j / 2) << 4)), make_uint4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]));
 }
-// `to`: this lane's row in the first piece of the first slot; the slots follow one another, and so do their pieces.  Lanes without
-// a row (live false) only take part in the reads.
+// `to`: the first slot; the slots follow one another, and so do their pieces.  Lanes without a row (live false) only take part
+// in the reads.
 template <int EPI>
-__device__ __forceinline__ void lay_out_parts(const Args& a, uint32_t to, uint32_t taddr, bool live) {
-  const int w = a.out_bn / a.split, pitch = a.x_rows * 16 + 16;
+__device__ __forceinline__ void lay_out_parts(const Args& a, uint32_t to, uint32_t taddr, int row, bool live) {
+  const int w = a.out_bn / a.split, pitch = a.x_rows * 16;
+  const uint32_t row16 = static_cast<uint32_t>(row) * 16;
   int dst = 0, up = 0, c = 0;  // SwiGLU: the slot of a part holds its gate columns, then its up columns
 #pragma unroll 1
   for (int c0 = 0; c0 < a.bn; c0 += 64) {
@@ -176,10 +179,10 @@ __device__ __forceinline__ void lay_out_parts(const Args& a, uint32_t to, uint32
     }
     ptx::tmem_ld_wait();
     if (live) {
-      put_pieces(to, pitch, x[0]);
-      put_pieces(to + 4 * pitch, pitch, x[1]);
-      if (more) put_pieces(to + 8 * pitch, pitch, x[2]);
-      if (more) put_pieces(to + 12 * pitch, pitch, x[3]);
+      put_pieces<0>(to, pitch, row16, x[0]);
+      put_pieces<1>(to, pitch, row16, x[1]);
+      if (more) put_pieces<2>(to, pitch, row16, x[2]);
+      if (more) put_pieces<3>(to, pitch, row16, x[3]);
     }
     to += 16 * pitch;
     __syncwarp();
@@ -189,7 +192,7 @@ __device__ __forceinline__ void lay_out_parts(const Args& a, uint32_t to, uint32
 template <int EPI>
 __device__ __forceinline__ void sum_parts(const Args& a, uint32_t smem, int part, int m0, int rows, int col0) {
   constexpr int H = EPI == kEpiSwiGLU ? 2 : 1;
-  const int w = a.out_bn / a.split, groups = w / 8, pitch = a.x_rows * 16 + 16, step = NUM_THREADS / groups;
+  const int w = a.out_bn / a.split, groups = w / 8, pitch = a.x_rows * 16, step = NUM_THREADS / groups;
   const int first = threadIdx.x / groups, g = threadIdx.x - first * groups, col = col0 + part * w + g * 8;
   if (first >= step || col >= a.out_n) return;
   const uint32_t own = smem + static_cast<uint32_t>(part * a.x_slot + 2 * g * pitch), got = smem + x_offset(a, part, part ? 0 : 1) + 2 * g * pitch;
@@ -198,7 +201,7 @@ __device__ __forceinline__ void sum_parts(const Args& a, uint32_t smem, int part
     float sum[H][8];
 #pragma unroll
     for (int h = 0; h < H; ++h) {
-      const uint32_t at = static_cast<uint32_t>(h * (w / 4) * pitch + row * 16);
+      const uint32_t at = static_cast<uint32_t>(h * (w / 4) * pitch) + (static_cast<uint32_t>(row * 16) ^ (((part * H + h) * groups + g) & 7) << 4);
 #pragma unroll 2
       for (int s = 0; s < a.split; ++s) {
         const uint32_t from = at + (s == part ? own : got + (s - (s > part ? 1 : 0)) * a.x_slot);
@@ -455,7 +458,7 @@ gemm_plain_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int q = warp & 3, row = q * a.warp_rows + lane;
     ptx::tc_fence_after();
     if (warp >= 2 && row - lane < rows)
-      lay_out_parts<EPI>(a, ptx::smem_u32(smem) + row * 16, tmem_base + (static_cast<uint32_t>(q * 32) << 16), lane < a.warp_rows && row < rows);
+      lay_out_parts<EPI>(a, ptx::smem_u32(smem), tmem_base + (static_cast<uint32_t>(q * 32) << 16), row, lane < a.warp_rows && row < rows);
     ptx::fence_proxy_async_smem();
     if (CG == 1) ptx::cluster_wait();  // the other CTAs' barriers exist
     ptx::tc_fence_before();

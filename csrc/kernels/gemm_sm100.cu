@@ -40,7 +40,7 @@ namespace {
 // Rows of a tile that the parts exchange, and whether what a CTA sends and what it gets have room side by side.
 int exchangeRows(int M, int cg) { return std::min((M + 7) / 8 * 8, cg == 1 && M <= 64 ? 64 : gemm::BM); }
 bool exchangeFits(const GemmCut& c, int M) {
-  return c.split == 1 || (2 * c.split - 1) * (c.bn / c.split / 4) * (exchangeRows(M, c.cg) * 16 + 16) <= gemm::plain::X_END;
+  return c.split == 1 || (2 * c.split - 1) * (c.bn / c.split / 4) * exchangeRows(M, c.cg) * 16 <= gemm::plain::X_END;
 }
 }  // namespace
 
@@ -264,7 +264,7 @@ ucclResult_t launchPlain(const GemmLaunch& g, const GemmCut* cut, cudaStream_t s
   const int out_n = swiglu ? g.N / 2 : g.N;
   if (cut && !gemmCutRuns(*cut, g.K, swiglu)) return ucclInvalidArgument;
   GemmCut p = cut ? *cut : cutFor(g.M, g.N, g.K, swiglu);
-  while (!exchangeFits(p, g.M)) p.split /= 2;  // of the cuts that may be asked for, 256 columns of 128 rows in four parts or more
+  while (!exchangeFits(p, g.M)) p.split /= 2;  // of the cuts that may be asked for, 256 columns of 128 rows in eight parts
   gemm::plain::Args a = {};
   a.C = static_cast<__nv_bfloat16*>(g.C);
   a.ldc = g.ldc;
@@ -283,7 +283,7 @@ ucclResult_t launchPlain(const GemmLaunch& g, const GemmCut* cut, cudaStream_t s
   // parts: no staging of the output, that room and the ring's end are the exchange buffer
   a.split = p.split;
   a.x_rows = exchangeRows(g.M, p.cg);
-  a.x_slot = p.bn / p.split / 4 * (a.x_rows * 16 + 16);
+  a.x_slot = p.bn / p.split / 4 * a.x_rows * 16;
   const int ring = p.split > 1 ? gemm::plain::X_END - (p.split - 1) * a.x_slot : gemm::PIPE_BYTES;
   a.stages = std::min(gemm::plain::MAX_STAGES, ring / a.stage_bytes);
   a.err = g.err;
